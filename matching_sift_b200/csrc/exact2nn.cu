@@ -555,63 +555,60 @@ __device__ __forceinline__ bool lex_less(int ka, int ia, int kb, int ib) {
     return ka < kb || (ka == kb && ia < ib);
 }
 
-// FLOATKEY: the keys are ordered images of float keys (float_key) and the
-// query norms float bit patterns (the general float path); else integers.
-template <bool FLOATKEY>
-__global__ void __launch_bounds__(256) merge2nn_kernel(const int4* __restrict__ partial, const ExactPlan plan,
-                                                       const WorkItem* __restrict__ items, int n_items,
-                                                       const WorkItem single, int group_rows, int total_q,
-                                                       const int32_t* __restrict__ qnorm, int metric, float thr,
-                                                       float dscale,
-                                                       uint32_t* __restrict__ matches, float4* __restrict__ sorted,
-                                                       int32_t* __restrict__ nn_idx, float* __restrict__ nn_dist) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= total_q) return;
-    const long long W = plan.units, G = plan.grid;
-    const WorkItem it =
-        items ? items[find_item(n_items, q, [&](int k) { return static_cast<long long>(items[k].a_off); })] : single;
-    int a1 = INT_MAX, j1 = -1, a2 = INT_MAX, j2 = -1;
-    auto push = [&](int k, int i) {
+// Lexicographic (key, index) top-2 of one query row while its partial lists
+// are merged. Every base row is in exactly one list and (key, index) is a total
+// order, so the result does not depend on the order of the pushes.
+struct MergeTop2 {
+    int k1 = INT_MAX, i1 = -1, k2 = INT_MAX, i2 = -1;
+    __device__ __forceinline__ void push(int k, int i) {
         if (i < 0) return;
-        if (lex_less(k, i, a1, j1) || j1 < 0) {
-            a2 = a1; j2 = j1;
-            a1 = k; j1 = i;
-        } else if (lex_less(k, i, a2, j2) || j2 < 0) {
-            a2 = k; j2 = i;
-        }
-    };
-    // No base rows: no CTA scanned this query and every neighbour is absent.
-    if (W > 0 && it.tiles > 0) {
-        const long long first = it.u_begin + static_cast<long long>((q - it.a_off) / group_rows) * it.tiles;
-        const int c0 = plan_cta_of(first, W, G);
-        const int c1 = plan_cta_of(first + it.tiles - 1, W, G);
-        for (int s = 0; s < (c1 - c0 + 1) * plan.parts; ++s) {
-            const int4 p = partial[static_cast<size_t>(s) * plan.q_pad + q];
-            push(p.x, p.y);
-            push(p.z, p.w);
+        if (lex_less(k, i, k1, i1) || i1 < 0) {
+            k2 = k1; i2 = i1;
+            k1 = k; i1 = i;
+        } else if (lex_less(k, i, k2, i2) || i2 < 0) {
+            k2 = k; i2 = i;
         }
     }
-    // Rows past the problem's base set are padding (they may hold another
-    // problem's rows, but only enter a top-2 when fewer real rows exist).
+    __device__ __forceinline__ void push(const int4& p) {
+        push(p.x, p.y);
+        push(p.z, p.w);
+    }
+};
+
+struct MergeOut {
+    uint32_t* matches;
+    float4* sorted;
+    int32_t* nn_idx;
+    float* nn_dist;
+};
+
+// Distances, ratio test and outputs of query row q. Rows past the problem's
+// base set (index >= n_b) are padding: they may hold another problem's rows,
+// but only enter a top-2 when fewer real rows exist. FLOATKEY: the keys are
+// ordered images of float keys (float_key) and qn is a float bit pattern (the
+// general float path); else integers.
+template <bool FLOATKEY>
+__device__ __forceinline__ void merge_finish(const MergeTop2& t, int q, int n_b, const int32_t* __restrict__ qnorm,
+                                             int metric, float thr, float dscale, const MergeOut& out) {
     bool v1, v2;
     float d1, d2;
     if constexpr (FLOATKEY) {
         // Squared distances |b|^2 - 2 q.b + |q|^2 can round a little below
         // zero for (near-)identical rows: clamped at 0.
-        v1 = j1 >= 0 && j1 < it.n_b;
-        v2 = j2 >= 0 && j2 < it.n_b;
+        v1 = t.i1 >= 0 && t.i1 < n_b;
+        v2 = t.i2 >= 0 && t.i2 < n_b;
         const float qn = metric == kMetricL2 ? __int_as_float(qnorm[q]) : 0.0f;
         const float lo = metric == kMetricL2 ? 0.0f : -FLT_MAX;
-        d1 = v1 ? fmaxf((key_float(a1) + qn) * dscale, lo) : FLT_MAX;
-        d2 = v2 ? fmaxf((key_float(a2) + qn) * dscale, lo) : FLT_MAX;
+        d1 = v1 ? fmaxf((key_float(t.k1) + qn) * dscale, lo) : FLT_MAX;
+        d2 = v2 ? fmaxf((key_float(t.k2) + qn) * dscale, lo) : FLT_MAX;
     } else {
-        v1 = j1 >= 0 && j1 < it.n_b && a1 < kKeyPad;
-        v2 = j2 >= 0 && j2 < it.n_b && a2 < kKeyPad;
+        v1 = t.i1 >= 0 && t.i1 < n_b && t.k1 < kKeyPad;
+        v2 = t.i2 >= 0 && t.i2 < n_b && t.k2 < kKeyPad;
         const int qn = metric == kMetricL2 ? qnorm[q] : 0;
-        d1 = v1 ? static_cast<float>(a1 + qn) * dscale : FLT_MAX;
-        d2 = v2 ? static_cast<float>(a2 + qn) * dscale : FLT_MAX;
+        d1 = v1 ? static_cast<float>(t.k1 + qn) * dscale : FLT_MAX;
+        d2 = v2 ? static_cast<float>(t.k2 + qn) * dscale : FLT_MAX;
     }
-    if (matches) {
+    if (out.matches) {
         bool pass = false;
         if (v1) {
             float f1, f2;
@@ -624,46 +621,114 @@ __global__ void __launch_bounds__(256) merge2nn_kernel(const int4* __restrict__ 
             }
             pass = (f1 / f2) < thr;
         }
-        matches[q] = pass ? static_cast<uint32_t>(j1) : UINT32_MAX;
+        out.matches[q] = pass ? static_cast<uint32_t>(t.i1) : UINT32_MAX;
     }
-    if (sorted)
-        sorted[q] = make_float4(d1, d2, v1 ? static_cast<float>(j1) : FLT_MAX, v2 ? static_cast<float>(j2) : FLT_MAX);
-    if (nn_idx) {
-        nn_idx[2 * q] = v1 ? j1 : -1;
-        nn_idx[2 * q + 1] = v2 ? j2 : -1;
+    if (out.sorted)
+        out.sorted[q] =
+            make_float4(d1, d2, v1 ? static_cast<float>(t.i1) : FLT_MAX, v2 ? static_cast<float>(t.i2) : FLT_MAX);
+    if (out.nn_idx) {
+        out.nn_idx[2 * static_cast<size_t>(q)] = v1 ? t.i1 : -1;
+        out.nn_idx[2 * static_cast<size_t>(q) + 1] = v2 ? t.i2 : -1;
     }
-    if (nn_dist) {
-        nn_dist[2 * q] = d1;
-        nn_dist[2 * q + 1] = d2;
+    if (out.nn_dist) {
+        out.nn_dist[2 * static_cast<size_t>(q)] = d1;
+        out.nn_dist[2 * static_cast<size_t>(q) + 1] = d2;
     }
 }
 
-// Merge of a search split over base chunks (indices already global). A
-// query row has a partial list per (chunk, CTA pair of its group, buffer),
-// ~90 for 10,000 x 1,000,000 in 9 chunks: kMergeLanes threads per row read
-// every kMergeLanes-th list (independent loads instead of one dependent
-// chain), and their top-2s are merged by shuffles. Every row of the base is
-// in exactly one list and (key, index) is a total order, so the top-2 does
-// not depend on the order of the merges.
-constexpr int kMergeLanes = 8;
-__global__ void __launch_bounds__(256) merge2nn_chunks_kernel(const int4* __restrict__ partial, const ChunkSet cs,
-                                                              int q_n, const int32_t* __restrict__ qnorm, int metric,
-                                                              float thr, float dscale, uint32_t* __restrict__ matches,
-                                                              float4* __restrict__ sorted,
-                                                              int32_t* __restrict__ nn_idx,
-                                                              float* __restrict__ nn_dist) {
-    const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int q = static_cast<int>(tid / kMergeLanes), sub = static_cast<int>(tid % kMergeLanes);
-    int a1 = INT_MAX, j1 = -1, a2 = INT_MAX, j2 = -1;
-    auto push = [&](int k, int i) {
-        if (i < 0) return;
-        if (lex_less(k, i, a1, j1) || j1 < 0) {
-            a2 = a1; j2 = j1;
-            a1 = k; j1 = i;
-        } else if (lex_less(k, i, a2, j2) || j2 < 0) {
-            a2 = k; j2 = i;
-        }
+// Merge of the partial lists of one search or a batch. A query row has
+// (workers of its group) x parts lists: 76 at 1,000 x 10,000, ~10 at
+// 10,000 x 1,000,000, 2-4 in a batch. What bounds it is the chain of dependent
+// loads per row, so a block of LANES warps owns 32 query rows: warp w reads
+// every LANES-th list of all 32 rows (512 consecutive bytes per list, four
+// lists in flight), the partial top-2s cross through shared memory so that
+// LANES consecutive threads hold one row's, and shuffles merge them. LANES = 1
+// (a thread per row, 256 rows per block) for the few lists of a batch.
+// launch_merge has the rule. Measured (whole match() call): 1,000 x 10,000
+// 56.5 -> 33.8 us, FP16 2,561 x 500,003 435 -> 427 us against one thread per row.
+constexpr int kMergeRows = 32;
+template <int LANES>
+constexpr int kMergeThreads = LANES == 1 ? 256 : kMergeRows * LANES;
+
+// All LANES threads of the block's row (threadIdx.x / LANES) return its top-2.
+template <int LANES>
+__device__ __forceinline__ MergeTop2 merge_lists_of_rows(const MergeTop2& mine) {
+    __shared__ int4 s_top[LANES][kMergeRows + 1];
+    s_top[threadIdx.x / kMergeRows][threadIdx.x % kMergeRows] = make_int4(mine.k1, mine.i1, mine.k2, mine.i2);
+    __syncthreads();
+    const int4 p = s_top[threadIdx.x % LANES][threadIdx.x / LANES];
+    MergeTop2 t{p.x, p.y, p.z, p.w};
+    #pragma unroll
+    for (int off = 1; off < LANES; off <<= 1) {
+        const int4 o = make_int4(__shfl_xor_sync(0xffffffffu, t.k1, off), __shfl_xor_sync(0xffffffffu, t.i1, off),
+                                 __shfl_xor_sync(0xffffffffu, t.k2, off), __shfl_xor_sync(0xffffffffu, t.i2, off));
+        t.push(o);
+    }
+    return t;
+}
+
+// Lists sub, sub + step, ... < n of a row (list s at p + s * stride).
+__device__ __forceinline__ void merge_lists(MergeTop2& t, const int4* __restrict__ p, size_t stride, int sub, int n,
+                                            int step) {
+    int s = sub;
+    for (; s + 3 * step < n; s += 4 * step) {
+        int4 v[4];
+        #pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = p[static_cast<size_t>(s + k * step) * stride];
+        #pragma unroll
+        for (int k = 0; k < 4; ++k) t.push(v[k]);
+    }
+    for (; s < n; s += step) t.push(p[static_cast<size_t>(s) * stride]);
+}
+
+template <bool FLOATKEY, int LANES>
+__global__ void __launch_bounds__(kMergeThreads<LANES>)
+    merge2nn_kernel(const int4* __restrict__ partial, const ExactPlan plan, const WorkItem* __restrict__ items,
+                    int n_items, const WorkItem single, int group_rows, int total_q, const int32_t* __restrict__ qnorm,
+                    int metric, float thr, float dscale, const MergeOut out) {
+    const int row0 = blockIdx.x * (kMergeThreads<LANES> / LANES);
+    int q = row0 + (LANES == 1 ? threadIdx.x : threadIdx.x % kMergeRows);
+    const long long W = plan.units, G = plan.grid;
+    auto item_of = [&](int row) {
+        return items ? items[find_item(n_items, row, [&](int k) { return static_cast<long long>(items[k].a_off); })]
+                     : single;
     };
+    MergeTop2 t;
+    if (LANES == 1 && q >= total_q) return;
+    int n_b = 0;
+    if (q < total_q) {
+        const WorkItem it = item_of(q);
+        n_b = it.n_b;
+        // No base rows: no CTA scanned this query and every neighbour is absent.
+        if (W > 0 && it.tiles > 0) {
+            const long long first = it.u_begin + static_cast<long long>((q - it.a_off) / group_rows) * it.tiles;
+            const int c0 = plan_cta_of(first, W, G);
+            const int c1 = plan_cta_of(first + it.tiles - 1, W, G);
+            merge_lists(t, partial + q, plan.q_pad, LANES == 1 ? 0 : threadIdx.x / kMergeRows,
+                        (c1 - c0 + 1) * plan.parts, LANES);
+        }
+    }
+    if constexpr (LANES > 1) {
+        t = merge_lists_of_rows<LANES>(t);
+        q = row0 + threadIdx.x / LANES;
+        if (threadIdx.x % LANES != 0 || q >= total_q) return;
+        n_b = item_of(q).n_b;
+    }
+    merge_finish<FLOATKEY>(t, q, n_b, qnorm, metric, thr, dscale, out);
+}
+
+// Merge of a search split over base chunks (indices already global): ~90 lists
+// per query row for 10,000 x 1,000,000 in 9 chunks, read as merge2nn_kernel
+// reads them.
+constexpr int kMergeChunkLanes = 8;
+__global__ void __launch_bounds__(kMergeThreads<kMergeChunkLanes>)
+    merge2nn_chunks_kernel(const int4* __restrict__ partial, const ChunkSet cs, int q_n,
+                           const int32_t* __restrict__ qnorm, int metric, float thr, float dscale,
+                           const MergeOut out) {
+    constexpr int LANES = kMergeChunkLanes;
+    int q = blockIdx.x * kMergeRows + threadIdx.x % kMergeRows;
+    const int sub = threadIdx.x / kMergeRows;
+    MergeTop2 t;
     if (q < q_n) {
         const int g = q / (kQT * kBM);
         int done = 0;  // lists of the earlier chunks
@@ -672,49 +737,16 @@ __global__ void __launch_bounds__(256) merge2nn_chunks_kernel(const int4* __rest
             const long long first = static_cast<long long>(g) * cs.tiles[c];
             const int c0 = plan_cta_of(first, cs.W[c], cs.G[c]);
             const int c1 = plan_cta_of(first + cs.tiles[c] - 1, cs.W[c], cs.G[c]);
-            const int4* pc = partial + c * cs.slot_stride;
             const int n_lists = (c1 - c0 + 1) * cs.parts;
-            for (int s = (sub - done % kMergeLanes + kMergeLanes) % kMergeLanes; s < n_lists; s += kMergeLanes) {
-                const int4 p = pc[static_cast<size_t>(s) * cs.q_pad + q];
-                push(p.x, p.y);
-                push(p.z, p.w);
-            }
+            merge_lists(t, partial + c * cs.slot_stride + q, cs.q_pad, (sub - done % LANES + LANES) % LANES, n_lists,
+                        LANES);
             done += n_lists;
         }
     }
-    // The kMergeLanes threads of a row are consecutive lanes of one warp.
-    #pragma unroll
-    for (int off = 1; off < kMergeLanes; off <<= 1) {
-        const int b1 = __shfl_xor_sync(0xffffffffu, a1, off), i1 = __shfl_xor_sync(0xffffffffu, j1, off);
-        const int b2 = __shfl_xor_sync(0xffffffffu, a2, off), i2 = __shfl_xor_sync(0xffffffffu, j2, off);
-        push(b1, i1);
-        push(b2, i2);
-    }
-    if (q >= q_n || sub != 0) return;
-    const bool v1 = j1 >= 0 && j1 < cs.r_n && a1 < kKeyPad;
-    const bool v2 = j2 >= 0 && j2 < cs.r_n && a2 < kKeyPad;
-    const int qn = metric == kMetricL2 ? qnorm[q] : 0;
-    const float d1 = v1 ? static_cast<float>(a1 + qn) * dscale : FLT_MAX;
-    const float d2 = v2 ? static_cast<float>(a2 + qn) * dscale : FLT_MAX;
-    if (matches) {
-        bool pass = false;
-        if (v1) {
-            const float f1 = metric == kMetricL2 ? sqrtf(d1) : sqrtf(d1 + 2.0f);
-            const float f2 = v2 ? (metric == kMetricL2 ? sqrtf(d2) : sqrtf(d2 + 2.0f)) : INFINITY;
-            pass = (f1 / f2) < thr;
-        }
-        matches[q] = pass ? static_cast<uint32_t>(j1) : UINT32_MAX;
-    }
-    if (sorted)
-        sorted[q] = make_float4(d1, d2, v1 ? static_cast<float>(j1) : FLT_MAX, v2 ? static_cast<float>(j2) : FLT_MAX);
-    if (nn_idx) {
-        nn_idx[2 * q] = v1 ? j1 : -1;
-        nn_idx[2 * q + 1] = v2 ? j2 : -1;
-    }
-    if (nn_dist) {
-        nn_dist[2 * q] = d1;
-        nn_dist[2 * q + 1] = d2;
-    }
+    t = merge_lists_of_rows<LANES>(t);
+    q = blockIdx.x * kMergeRows + threadIdx.x / LANES;
+    if (threadIdx.x % LANES != 0 || q >= q_n) return;
+    merge_finish<false>(t, q, cs.r_n, qnorm, metric, thr, dscale, out);
 }
 
 }  // namespace
@@ -723,9 +755,8 @@ cudaError_t launch_merge2nn_chunks(const int4* partial, const ChunkSet& cs, int 
                                    float threshold, float dist_scale, uint32_t* matches, float4* sorted,
                                    int32_t* nn_idx, float* nn_dist, cudaStream_t stream) {
     if (q_n <= 0) return cudaSuccess;
-    const long long threads = static_cast<long long>(q_n) * kMergeLanes;
-    merge2nn_chunks_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(
-        partial, cs, q_n, qnorm, metric, threshold, dist_scale, matches, sorted, nn_idx, nn_dist);
+    merge2nn_chunks_kernel<<<(q_n + kMergeRows - 1) / kMergeRows, kMergeThreads<kMergeChunkLanes>, 0, stream>>>(
+        partial, cs, q_n, qnorm, metric, threshold, dist_scale, MergeOut{matches, sorted, nn_idx, nn_dist});
     return cudaGetLastError();
 }
 
@@ -808,44 +839,57 @@ cudaError_t launch_exact2nn_u8(const CUtensorMap& qmap, const CUtensorMap& bmap,
     return cudaGetLastError();
 }
 
-cudaError_t launch_merge2nn(const int4* partial, const ExactPlan& plan, const int32_t* qnorm, int metric,
-                            float threshold, float dist_scale, uint32_t* matches, float4* sorted, int32_t* nn_idx,
-                            float* nn_dist, cudaStream_t stream) {
-    if (plan.q_n <= 0) return cudaSuccess;
+// The launch of merge2nn_kernel with as many warps per 32 rows as the longest
+// row has lists to share out, in steps of 1, 8 and 32 (one list per thread up
+// to 32 lists, three at the 76 of 1,000 x 10,000; at 2-4 lists the exchange
+// through shared memory would cost more than the second load it saves).
+template <bool FLOATKEY>
+cudaError_t launch_merge(const int4* partial, const ExactPlan& plan, const WorkItem* items, int n_items,
+                         const WorkItem& single, int group_rows, int total_q, const int32_t* qnorm, int metric,
+                         float threshold, float dist_scale, const MergeOut& out, cudaStream_t stream) {
+    if (total_q <= 0) return cudaSuccess;
+    const int lists = plan.max_splits * plan.parts;
+    const int blocks = (total_q + kMergeRows - 1) / kMergeRows;
+    if (lists <= 4)
+        merge2nn_kernel<FLOATKEY, 1><<<(total_q + 255) / 256, kMergeThreads<1>, 0, stream>>>(
+            partial, plan, items, n_items, single, group_rows, total_q, qnorm, metric, threshold, dist_scale, out);
+    else if (lists <= 32)
+        merge2nn_kernel<FLOATKEY, 8><<<blocks, kMergeThreads<8>, 0, stream>>>(
+            partial, plan, items, n_items, single, group_rows, total_q, qnorm, metric, threshold, dist_scale, out);
+    else
+        merge2nn_kernel<FLOATKEY, 32><<<blocks, kMergeThreads<32>, 0, stream>>>(
+            partial, plan, items, n_items, single, group_rows, total_q, qnorm, metric, threshold, dist_scale, out);
+    return cudaGetLastError();
+}
+
+WorkItem merge_item(const ExactPlan& plan) {
     WorkItem single{};
     single.n_a = plan.q_n;
     single.n_b = plan.r_n;
     single.groups = plan.q_groups;
     single.tiles = plan.base_tiles;
-    merge2nn_kernel<false><<<(plan.q_n + 255) / 256, 256, 0, stream>>>(partial, plan, nullptr, 1, single, kQT * kBM,
-                                                                      plan.q_n, qnorm, metric, threshold, dist_scale,
-                                                                      matches, sorted, nn_idx, nn_dist);
-    return cudaGetLastError();
+    return single;
+}
+
+cudaError_t launch_merge2nn(const int4* partial, const ExactPlan& plan, const int32_t* qnorm, int metric,
+                            float threshold, float dist_scale, uint32_t* matches, float4* sorted, int32_t* nn_idx,
+                            float* nn_dist, cudaStream_t stream) {
+    return launch_merge<false>(partial, plan, nullptr, 1, merge_item(plan), kQT * kBM, plan.q_n, qnorm, metric,
+                               threshold, dist_scale, MergeOut{matches, sorted, nn_idx, nn_dist}, stream);
 }
 
 cudaError_t launch_merge2nn_float(const int4* partial, const ExactPlan& plan, int group_rows, const int32_t* qnorm,
                                   int metric, float threshold, float dist_scale, uint32_t* matches, float4* sorted,
                                   int32_t* nn_idx, float* nn_dist, cudaStream_t stream) {
-    if (plan.q_n <= 0) return cudaSuccess;
-    WorkItem single{};
-    single.n_a = plan.q_n;
-    single.n_b = plan.r_n;
-    single.groups = plan.q_groups;
-    single.tiles = plan.base_tiles;
-    merge2nn_kernel<true><<<(plan.q_n + 255) / 256, 256, 0, stream>>>(partial, plan, nullptr, 1, single, group_rows,
-                                                                     plan.q_n, qnorm, metric, threshold, dist_scale,
-                                                                     matches, sorted, nn_idx, nn_dist);
-    return cudaGetLastError();
+    return launch_merge<true>(partial, plan, nullptr, 1, merge_item(plan), group_rows, plan.q_n, qnorm, metric,
+                              threshold, dist_scale, MergeOut{matches, sorted, nn_idx, nn_dist}, stream);
 }
 
 cudaError_t launch_merge2nn_batch(const int4* partial, const BatchPlan& bp, int total_queries, const int32_t* qnorm,
                                   int metric, float threshold, float dist_scale, uint32_t* matches, float4* sorted,
                                   int32_t* nn_idx, float* nn_dist, cudaStream_t stream) {
-    if (total_queries <= 0) return cudaSuccess;
-    merge2nn_kernel<false><<<(total_queries + 255) / 256, 256, 0, stream>>>(
-        partial, bp.plan, bp.items, bp.n_items, WorkItem{}, bp.group_rows, total_queries, qnorm, metric, threshold,
-        dist_scale, matches, sorted, nn_idx, nn_dist);
-    return cudaGetLastError();
+    return launch_merge<false>(partial, bp.plan, bp.items, bp.n_items, WorkItem{}, bp.group_rows, total_queries, qnorm,
+                               metric, threshold, dist_scale, MergeOut{matches, sorted, nn_idx, nn_dist}, stream);
 }
 
 cudaError_t launch_batch_records(const uint8_t* base, int, const BatchPlan& bp, int metric, int32_t* rec,
