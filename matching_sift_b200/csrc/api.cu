@@ -829,10 +829,8 @@ int lsh_match_float(const LshArgs& a, DeviceCtx& c, cudaStream_t st) {
     const uint32_t* probe_codes = codes_q;
     if (multi) {
         uint32_t* pc = reinterpret_cast<uint32_t*>(A + o_pc);
-        for (int t = 0; t < L_; ++t)
-            SIFT_CUDA(launch_probe_codes(codes_q + static_cast<size_t>(t) * q_n, zq + static_cast<size_t>(t) * q_n * k,
-                                         q_n, k, flip, a.probes, pc + static_cast<size_t>(t) * a.probes * q_n, st));
-        g_launches += L_;
+        SIFT_CUDA(launch_probe_codes(codes_q, zq, q_n, L_, k, flip, a.probes, pc, st));
+        ++g_launches;
         probe_codes = pc;
     }
     int* start = reinterpret_cast<int*>(A + o_start);
@@ -940,10 +938,8 @@ int lsh_match(const LshArgs& a) {
         // Per table: the query's code with the lightest subsets of its
         // lowest-margin bits flipped, [t][probe][query] as the scan reads them.
         uint32_t* pc = reinterpret_cast<uint32_t*>(A + o_pc);
-        for (int t = 0; t < L_; ++t)
-            SIFT_CUDA(launch_probe_codes(codes_q + static_cast<size_t>(t) * q_n, zq + static_cast<size_t>(t) * q_n * k,
-                                         q_n, k, flip, a.probes, pc + static_cast<size_t>(t) * a.probes * q_n, st));
-        g_launches += L_;
+        SIFT_CUDA(launch_probe_codes(codes_q, zq, q_n, L_, k, flip, a.probes, pc, st));
+        ++g_launches;
         probe_codes = pc;
     }
     SIFT_CUDA(launch_lsh_buckets(codes_r, r_n, L_, shift, nbins, hist, start, order, ocode, c.num_sms, st));

@@ -381,10 +381,8 @@ int index_search(const sift_code_index* ix, const uint8_t* q, uint32_t q_n_, int
     const uint32_t* probe_codes = codes_q;
     if (multi) {
         uint32_t* pc = reinterpret_cast<uint32_t*>(A + o_pc);
-        for (int t = 0; t < L_; ++t)
-            SIFT_CUDA(launch_probe_codes(codes_q + static_cast<size_t>(t) * q_n, z + static_cast<size_t>(t) * q_n * k,
-                                         q_n, k, flip, probes, pc + static_cast<size_t>(t) * probes * q_n, st));
-        detail::g_launches += L_;
+        SIFT_CUDA(launch_probe_codes(codes_q, z, q_n, L_, k, flip, probes, pc, st));
+        ++detail::g_launches;
         probe_codes = pc;
     }
     {

@@ -37,11 +37,12 @@ cudaError_t launch_mlp_hash(const CUtensorMap& xmap, int n, const CUtensorMap& w
                             int num_sms, cudaStream_t stream);
 size_t mlp_hash_smem_bytes();
 
-// Query-directed multi-probe: probe p of query i is codes[i] with the bits of
-// the p-th lightest subset of its `flip` smallest-|z| bits flipped (subsets
-// ordered by the sum of their |z|; probe 0 is the code itself). Writes
-// probe_codes[p][n] for p < n_probes (n_probes <= 64, flip <= 6).
-cudaError_t launch_probe_codes(const uint32_t* codes, const float* z, int n, int k, int flip, int n_probes,
+// Query-directed multi-probe over `tables` hash tables (codes[t][n], margins
+// z[t][n][k]): probe p of query i is codes[t][i] with the bits of the p-th
+// lightest subset of its `flip` smallest-|z| bits flipped (subsets ordered by
+// the sum of their |z|; probe 0 is the code itself). Writes
+// probe_codes[t][p][n] for p < n_probes (n_probes <= 64, flip <= 6).
+cudaError_t launch_probe_codes(const uint32_t* codes, const float* z, int n, int tables, int k, int flip, int n_probes,
                                uint32_t* probe_codes, cudaStream_t stream);
 
 // ---- training (learned_train.cu)

@@ -130,7 +130,8 @@ int mlp_match(const uint8_t* q, const uint8_t* r, uint32_t q_n_, uint32_t r_n_, 
     SIFT_TRY(detail::encode_u8_rows(&qmap_h, q, q_n, 128));
     SIFT_CUDA(launch_mlp_hash(qmap_h, q_n, w1map, w2map, m.b1, m.b2, k, U32(o_cq), reinterpret_cast<float*>(A + o_z),
                               c.d_status, c.num_sms, st));
-    SIFT_CUDA(launch_probe_codes(U32(o_cq), reinterpret_cast<float*>(A + o_z), q_n, k, flip, n_probes, U32(o_pc), st));
+    SIFT_CUDA(launch_probe_codes(U32(o_cq), reinterpret_cast<float*>(A + o_z), q_n, 1, k, flip, n_probes, U32(o_pc),
+                                 st));
     SIFT_CUDA(launch_lsh_scan(q, r, q_n, r_n, 1, n_probes, shift, nbins, U32(o_pc), I32(o_start), I32(o_order),
                               U32(o_ocode), threshold, threshold > 0.f ? 1 : 0, 1.0f, matches, counts, nn_idx, dist,
                               st));
