@@ -5,7 +5,7 @@
 //   set_bit_h sign packing                 :265-317     -> fused into lsh_hash_kernel's epilogue
 //   thrust::sort by code + host run-length :565-629     -> bucket histogram / scan / scatter kernels
 //   host merge-join of Q and R buckets     :657-681     -> the query code indexes the bucket table
-//   brute_2nn_h + atomic_min2_update       :441-562     -> lsh_scan_kernel (warp per query)
+//   brute_2nn_h + atomic_min2_update       :441-562     -> lsh_scan_kernel (warp or block per query)
 //
 // Codes. Table t of L uses k hyperplanes; bit j of a point's code is set when
 // its dot product with hyperplane j is negative (set_bit_h, src/lsh_h.cu:302-309).
@@ -20,12 +20,12 @@
 // query's code (the reference scans sorted positions starting at a point id
 // instead, src/lsh_h.cu:599,617 vs :469,482, which is not the bucket).
 //
-// Candidate scan. One warp per query over its L buckets (L x P with P probe
-// codes per table: multi-probe); candidate rows are fetched by groups of 8
-// lanes with coalesced 16-byte loads (4 rows per warp-wide load) and scored
-// as the exact |q - b|^2 (byte-wise absolute differences squared and summed
-// by dp4a); the per-query top-2 is lexicographic in (distance, index) and
-// counts a base point found in several tables once.
+// Candidate scan. One warp or one block per query over its L buckets (L x P
+// with P probe codes per table: multi-probe); candidate rows are fetched by
+// groups of 8 lanes with coalesced 16-byte loads (4 rows per warp-wide load)
+// and scored as the exact |q - b|^2 (dp4a); the per-query top-2 is
+// lexicographic in (distance, index) and counts a base point found in several
+// tables once.
 #include <climits>
 #include <cfloat>
 #include <cstdint>
@@ -309,153 +309,272 @@ __device__ __forceinline__ void push_dedup(int d, int i, int& d1, int& i1, int& 
     }
 }
 
-// One warp per query, its buckets walked 32 positions at a time. The ids and
-// codes of a chunk are one coalesced 128-byte load each (the next chunk's are
-// fetched while the current chunk's rows load); members whose full code
-// matches are compacted through shared memory; then every 8 lanes fetch one
-// candidate row with coalesced 16-byte loads (4 rows per warp-wide load, up
-// to 8 loads = 32 rows in flight per lane before any arithmetic), each lane
-// forms the squared distance of its 16 bytes (byte-wise absolute difference,
-// then dp4a) and 3 shuffles sum them: exact integers, no norms needed. The
-// lane leading each group of 8 keeps a lexicographic (distance, index)
-// top-2; the four lists are merged at the end. A base row found in several
-// tables (or probes) is compared each time but enters a list once.
+// NW warps per query. The query's probed buckets (L x P entries: table and
+// code) are laid out in shared memory as runs of 32 positions ("chunks"), and
+// every warp walks its equal share of the chunks: the ids (and, when a group
+// holds several codes, the codes) of a chunk are one coalesced 128-byte load
+// each, the next chunk's fetched while the current one is used. Members whose
+// full code matches are appended to the warp's queue, and every 32 of them are
+// scored together: 8 lanes fetch one row with coalesced 16-byte loads (8 loads,
+// 32 rows in flight per warp), each lane sums b.b - 2 q.b over its 16 bytes
+// by dp4a (|q - b|^2 = |q|^2 + that, exact integers), and 7 shuffles leave one
+// row's distance in each lane. Every lane keeps a lexicographic (distance,
+// index) top-2 of its rows; the lists are merged at the end, and a base row
+// found in several tables (or probes) is compared each time but enters a list
+// once.
+//
+// What bounds it: the random 128-byte rows of the candidates (L2 and DRAM).
+// Candidates per query vary by a factor of 20 (8,788 to 163,868 at 1M rows, 8
+// tables of 16 bits, 16 probes), so with one warp per query the last warps ran
+// alone (70% of the SM cycles active), and the scoring took ~3x the
+// instructions (byte differences, 3 shuffles per 4 rows, chunks of short
+// buckets scored half empty). scan_warps has the rule for NW. Measured: that
+// search 13.4 -> 3.2 ms (25-30 GB of candidate rows and ids: 8 TB/s, part of it
+// from L2), the learned-hash match of 4,096 queries and 8 probes 4.87 -> 1.26 ms.
 constexpr int kScanThreads = 256;
+constexpr int kScanWarps = kScanThreads / 32;
 
-__global__ void __launch_bounds__(kScanThreads) lsh_scan_kernel(
+struct ScanEntry {
+    int pos, end;   // positions of the bucket in its table's order
+    uint32_t code;
+    int chunk0;     // first chunk of the entry among the query's chunks
+};
+
+__host__ __device__ constexpr size_t scan_smem_bytes(int entries, int nw) {
+    return static_cast<size_t>(kScanWarps / nw) * (entries + 1) * sizeof(ScanEntry);
+}
+
+struct ScanTop2 {
+    int d1 = INT_MAX, i1 = -1, d2 = INT_MAX, i2 = -1;
+    __device__ __forceinline__ void push(int d, int i) { push_dedup(d, i, d1, i1, d2, i2); }
+    __device__ __forceinline__ void merge_xor(int o) {
+        const int od1 = __shfl_xor_sync(0xffffffffu, d1, o), oi1 = __shfl_xor_sync(0xffffffffu, i1, o);
+        const int od2 = __shfl_xor_sync(0xffffffffu, d2, o), oi2 = __shfl_xor_sync(0xffffffffu, i2, o);
+        push(od1, oi1);
+        push(od2, oi2);
+    }
+};
+
+// Scores the first 32 ids of a warp's queue (-1: none) against the query row
+// chunk qv of lane part `lane & 7`, |q|^2 = qn.
+__device__ __forceinline__ void score32(const uint8_t* __restrict__ r, const int* queue, const uint4& qv, int qn,
+                                        int lane, ScanTop2& top) {
+    const int sub = lane >> 3, part = lane & 7;  // rows 8 sub .. 8 sub + 7 of the queue, 16-byte chunk of the row
+    const int4 ida = reinterpret_cast<const int4*>(queue)[2 * sub], idb = reinterpret_cast<const int4*>(queue)[2 * sub + 1];
+    const int ids[8] = {ida.x, ida.y, ida.z, ida.w, idb.x, idb.y, idb.z, idb.w};
+    uint4 v[8];
+    #pragma unroll
+    for (int j = 0; j < 8; ++j)
+        v[j] = __ldg(reinterpret_cast<const uint4*>(r + static_cast<size_t>(max(ids[j], 0)) * 128) + part);
+    int d[8];
+    #pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        uint32_t bb = __dp4a(v[j].x, v[j].x, 0u), qb = __dp4a(qv.x, v[j].x, 0u);
+        bb = __dp4a(v[j].y, v[j].y, bb);
+        qb = __dp4a(qv.y, v[j].y, qb);
+        bb = __dp4a(v[j].z, v[j].z, bb);
+        qb = __dp4a(qv.z, v[j].z, qb);
+        bb = __dp4a(v[j].w, v[j].w, bb);
+        qb = __dp4a(qv.w, v[j].w, qb);
+        d[j] = static_cast<int>(bb) - 2 * static_cast<int>(qb);
+    }
+    // Sum over the 8 lanes of a row, halving the rows a lane holds each time.
+    const bool h1 = part & 1, h2 = part & 2, h4 = part & 4;
+    #pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int give = h1 ? d[j] : d[j + 4], keep = h1 ? d[j + 4] : d[j];
+        d[j] = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+    }
+    #pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int give = h2 ? d[j] : d[j + 2], keep = h2 ? d[j + 2] : d[j];
+        d[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+    }
+    const int give = h4 ? d[0] : d[1], keep = h4 ? d[1] : d[0];
+    const int dist = qn + keep + __shfl_xor_sync(0xffffffffu, give, 4);
+    const int id = queue[8 * sub + (h1 ? 4 : 0) + (h2 ? 2 : 0) + (h4 ? 1 : 0)];
+    if (dist <= top.d2) top.push(dist, id);
+}
+
+template <int NW>
+__global__ void __launch_bounds__(kScanThreads, 3) lsh_scan_kernel(
     const uint8_t* __restrict__ q, const uint8_t* __restrict__ r, int q_n, int r_n, int L, int probes, int shift,
     int nbins, const uint32_t* __restrict__ qcodes, const int* __restrict__ start, const int* __restrict__ order,
     const uint32_t* __restrict__ ocode, float thr, int ratio, float dscale, uint32_t* __restrict__ matches,
     uint32_t* __restrict__ counts, int32_t* __restrict__ nn_idx, float* __restrict__ nn_dist) {
-    __shared__ int s_ids[kScanThreads / 32][32];
-    const int wq = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const int sub = lane >> 3, part = lane & 7;  // row slot of a 4-row load, 16-byte chunk of the row
-    if (wq >= q_n) return;
-    int* ids = s_ids[threadIdx.x >> 5];
-    const uint4 qv = __ldg(reinterpret_cast<const uint4*>(q + static_cast<size_t>(wq) * 128) + part);
+    static_assert(NW == 1 || NW == kScanWarps, "a query is a warp's or a block's");
+    extern __shared__ ScanEntry s_entries[];
+    __shared__ __align__(16) int s_queue[kScanWarps][64];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = NW == 1 ? 0 : warp;  // warp of the query
+    const int wq = NW == 1 ? blockIdx.x * kScanWarps + warp : blockIdx.x;
+    if (NW == 1 && wq >= q_n) return;
+    const int E = L * probes;
+    ScanEntry* ent = s_entries + (NW == 1 ? warp * (E + 1) : 0);
+    int* queue = s_queue[warp];
+    auto sync = [] {
+        if constexpr (NW == 1) __syncwarp();
+        else __syncthreads();
+    };
+    const uint4 qv = __ldg(reinterpret_cast<const uint4*>(q + static_cast<size_t>(wq) * 128) + (lane & 7));
+    int qn = static_cast<int>(__dp4a(qv.x, qv.x, __dp4a(qv.y, qv.y, __dp4a(qv.z, qv.z, __dp4a(qv.w, qv.w, 0u)))));
+    qn += __shfl_xor_sync(0xffffffffu, qn, 1);
+    qn += __shfl_xor_sync(0xffffffffu, qn, 2);
+    qn += __shfl_xor_sync(0xffffffffu, qn, 4);
     const bool whole_bins = shift == 0;  // a group holds exactly one code
-    int d1 = INT_MAX, i1 = -1, d2 = INT_MAX, i2 = -1;
+
+    // The entries: codes and bucket bounds, then their chunks' prefix sum.
+    for (int i = w * 32 + lane; i < E; i += NW * 32) {
+        const int t = i / probes;
+        const uint32_t code = qcodes[static_cast<size_t>(i) * q_n + wq];
+        const int* st = start + static_cast<size_t>(t) * (nbins + 1) + (code >> shift);
+        ent[i].code = code;
+        ent[i].pos = st[0];
+        ent[i].end = st[1];
+    }
+    sync();
+    for (int i = w * 32 + lane; i < E; i += NW * 32) {
+        // A repeated probe code (fewer distinct probes than requested) is skipped.
+        bool repeated = false;
+        for (int j = i - i % probes; j < i; ++j) repeated |= ent[j].code == ent[i].code;
+        ent[i].chunk0 = repeated ? 0 : (ent[i].end - ent[i].pos + 31) >> 5;
+    }
+    sync();
+    if (w == 0) {
+        const int per = (E + 31) / 32;
+        const int e0 = min(lane * per, E), e1 = min(e0 + per, E);
+        int mine = 0;
+        for (int i = e0; i < e1; ++i) mine += ent[i].chunk0;
+        int incl = mine;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        int run = incl - mine;
+        for (int i = e0; i < e1; ++i) {
+            const int n = ent[i].chunk0;
+            ent[i].chunk0 = run;
+            run += n;
+        }
+        if (lane == 31) ent[E].chunk0 = incl;
+    }
+    sync();
+
+    ScanTop2 top;
     uint32_t seen = 0;  // candidates compared (bucket members)
-    for (int t = 0; t < L; ++t) {
-        // The table's probe codes and their bucket bounds, one probe per lane
-        // (probes <= 64: two per lane), fetched in parallel: two round trips per
-        // table instead of two per probe.
-        const int* st = start + static_cast<size_t>(t) * (nbins + 1);
-        const uint32_t* tq = qcodes + static_cast<size_t>(t) * probes * q_n + wq;
-        uint32_t pc0 = 0, pc1 = 0;
-        int ps0 = 0, pe0 = 0, ps1 = 0, pe1 = 0;
-        if (lane < probes) pc0 = tq[static_cast<size_t>(lane) * q_n];
-        if (lane + 32 < probes) pc1 = tq[static_cast<size_t>(lane + 32) * q_n];
-        if (lane < probes) {
-            const int b = static_cast<int>(pc0 >> shift);
-            ps0 = st[b];
-            pe0 = st[b + 1];
-        }
-        if (lane + 32 < probes) {
-            const int b = static_cast<int>(pc1 >> shift);
-            ps1 = st[b];
-            pe1 = st[b + 1];
-        }
-        for (int pi = 0; pi < probes; ++pi) {
-            const bool lo = pi < 32;
-            const uint32_t code = __shfl_sync(0xffffffffu, lo ? pc0 : pc1, pi & 31);
-            // A repeated probe code (fewer distinct probes than requested) is skipped.
-            if (__any_sync(0xffffffffu, (lane < pi && pc0 == code) || (lane + 32 < pi && pc1 == code))) continue;
-            const int s = __shfl_sync(0xffffffffu, lo ? ps0 : ps1, pi & 31);
-            const int e = __shfl_sync(0xffffffffu, lo ? pe0 : pe1, pi & 31);
-            const int* ord = order + static_cast<size_t>(t) * r_n;
-            const uint32_t* oc = ocode + static_cast<size_t>(t) * r_n;
-            int nid = -1;
-            uint32_t ncode = ~code;
-            if (s + lane < e) {
-                nid = ord[s + lane];
-                ncode = whole_bins ? code : oc[s + lane];
+    const long long chunks = ent[E].chunk0;
+    const int c0 = static_cast<int>(chunks * w / NW), c1 = static_cast<int>(chunks * (w + 1) / NW);
+    if (c0 < c1) {
+        int e = 0;  // the entry of chunk c0: the last one that starts at or before it and is not empty
+        for (int lo = 0, hi = E - 1; lo <= hi;) {
+            const int mid = (lo + hi) >> 1;
+            if (ent[mid].chunk0 <= c0) {
+                e = mid;
+                lo = mid + 1;
+            } else {
+                hi = mid - 1;
             }
-            for (int p0 = s; p0 < e; p0 += 32) {
-                const int id = nid;
-                const bool hit = id >= 0 && ncode == code;
-                const int pn = p0 + 32 + lane;
-                nid = -1;
-                ncode = ~code;
-                if (pn < e) {
-                    nid = ord[pn];
-                    ncode = whole_bins ? code : oc[pn];
-                }
-                const uint32_t mask = __ballot_sync(0xffffffffu, hit);
-                const int nm = __popc(mask);
-                if (nm == 0) continue;
-                seen += nm;
-                if (hit) ids[__popc(mask & ((1u << lane) - 1u))] = id;
+        }
+        int nid = -1;
+        uint32_t ncode = 0, ecode = 0;
+        auto fetch = [&](int c) {  // ids and codes of chunk c (chunks come in order)
+            while (c >= ent[e + 1].chunk0) ++e;
+            const ScanEntry& x = ent[e];
+            const int p = x.pos + ((c - x.chunk0) << 5) + lane;
+            const size_t at = static_cast<size_t>(e / probes) * r_n + p;
+            ecode = x.code;
+            nid = -1;
+            if (p < x.end) {
+                nid = order[at];
+                ncode = whole_bins ? ecode : ocode[at];
+            }
+        };
+        fetch(c0);
+        int held = 0;  // ids in the queue
+        for (int c = c0; c < c1; ++c) {
+            const int id = nid;
+            const bool hit = id >= 0 && ncode == ecode;
+            if (c + 1 < c1) fetch(c + 1);
+            const uint32_t mask = __ballot_sync(0xffffffffu, hit);
+            if (hit) queue[held + __popc(mask & ((1u << lane) - 1u))] = id;
+            held += __popc(mask);
+            seen += __popc(mask);
+            __syncwarp();
+            if (held >= 32) {
+                score32(r, queue, qv, qn, lane, top);
+                held -= 32;
+                const int rest = queue[32 + lane];
                 __syncwarp();
-                // The hits in two rounds of 16 (4 rows per lane in flight):
-                // fewer registers than one round of 32, so more queries (warps)
-                // share an SM and hide each other's load latency.
-                #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (16 * h >= nm) break;
-                    uint4 rv[4];
-                    int cid[4];
-                    #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int rank = 16 * h + 4 * j + sub;
-                        cid[j] = rank < nm ? ids[rank] : -1;
-                        if (cid[j] >= 0)
-                            rv[j] = __ldg(reinterpret_cast<const uint4*>(r + static_cast<size_t>(cid[j]) * 128) + part);
-                    }
-                    #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        if (16 * h + 4 * j >= nm) break;
-                        // |q - b|^2 of this lane's 16 bytes: byte-wise |q - b| (SIMD
-                        // absolute difference), then the sum of their squares by dp4a.
-                        uint32_t dist = 0;
-                        if (cid[j] >= 0) {
-                            uint32_t a = __vabsdiffu4(qv.x, rv[j].x);
-                            dist = __dp4a(a, a, dist);
-                            a = __vabsdiffu4(qv.y, rv[j].y);
-                            dist = __dp4a(a, a, dist);
-                            a = __vabsdiffu4(qv.z, rv[j].z);
-                            dist = __dp4a(a, a, dist);
-                            a = __vabsdiffu4(qv.w, rv[j].w);
-                            dist = __dp4a(a, a, dist);
-                        }
-                        dist += __shfl_xor_sync(0xffffffffu, dist, 1);
-                        dist += __shfl_xor_sync(0xffffffffu, dist, 2);
-                        dist += __shfl_xor_sync(0xffffffffu, dist, 4);
-                        if (part == 0 && cid[j] >= 0) push_dedup(static_cast<int>(dist), cid[j], d1, i1, d2, i2);
-                    }
-                }
-                __syncwarp();  // ids is rewritten by the next 32 positions
+                if (lane < held) queue[lane] = rest;
+                __syncwarp();
             }
+        }
+        if (held > 0) {
+            if (lane >= held) queue[lane] = -1;
+            __syncwarp();
+            score32(r, queue, qv, qn, lane, top);
         }
     }
-    // Merge the four group lists (lexicographic, duplicates counted once).
     #pragma unroll
-    for (int o = 8; o < 32; o <<= 1) {
-        const int od1 = __shfl_xor_sync(0xffffffffu, d1, o), oi1 = __shfl_xor_sync(0xffffffffu, i1, o);
-        const int od2 = __shfl_xor_sync(0xffffffffu, d2, o), oi2 = __shfl_xor_sync(0xffffffffu, i2, o);
-        push_dedup(od1, oi1, d1, i1, d2, i2);
-        push_dedup(od2, oi2, d1, i1, d2, i2);
+    for (int o = 1; o < 32; o <<= 1) top.merge_xor(o);
+    if constexpr (NW > 1) {
+        __syncwarp();
+        if (lane == 0) {
+            queue[0] = top.d1;
+            queue[1] = top.i1;
+            queue[2] = top.d2;
+            queue[3] = top.i2;
+            queue[4] = static_cast<int>(seen);
+        }
+        __syncthreads();
+        if (warp > 0) return;
+        top = ScanTop2{};
+        seen = 0;
+        if (lane < NW) {
+            top = ScanTop2{s_queue[lane][0], s_queue[lane][1], s_queue[lane][2], s_queue[lane][3]};
+            seen = static_cast<uint32_t>(s_queue[lane][4]);
+        }
+        #pragma unroll
+        for (int o = 1; o < NW; o <<= 1) {
+            top.merge_xor(o);
+            seen += __shfl_xor_sync(0xffffffffu, seen, o);
+        }
     }
     if (lane == 0) {
         if (counts) counts[wq] = seen;
-        const bool v1 = i1 >= 0, v2 = i2 >= 0;
-        const float f1 = v1 ? static_cast<float>(d1) * dscale : FLT_MAX;
-        const float f2 = v2 ? static_cast<float>(d2) * dscale : FLT_MAX;
+        const bool v1 = top.i1 >= 0, v2 = top.i2 >= 0;
+        const float f1 = v1 ? static_cast<float>(top.d1) * dscale : FLT_MAX;
+        const float f2 = v2 ? static_cast<float>(top.d2) * dscale : FLT_MAX;
         if (matches) {
             bool pass = v1;
             if (v1 && ratio) pass = (sqrtf(f1) / (v2 ? sqrtf(f2) : INFINITY)) < thr;
-            matches[wq] = pass ? static_cast<uint32_t>(i1) : UINT32_MAX;
+            matches[wq] = pass ? static_cast<uint32_t>(top.i1) : UINT32_MAX;
         }
         if (nn_idx) {
-            nn_idx[2 * wq] = i1;
-            nn_idx[2 * wq + 1] = i2;
+            nn_idx[2 * wq] = top.i1;
+            nn_idx[2 * wq + 1] = top.i2;
         }
         if (nn_dist) {
             nn_dist[2 * wq] = f1;
             nn_dist[2 * wq + 1] = f2;
         }
     }
+}
+
+// Warps per query from the average number of candidates that evenly spread
+// codes would give (real codes crowd: 4-30 times that). Measured, scan kernel
+// with 1 | 8 warps, 1M rows, 16 bits: 4,096 queries, 1 table and probe
+// (15 expected) 44 | 52 us, 1 table x 4 probes (61) 116 | 89, 4 x 1 (61)
+// 415 | 211, 4 x 4 (244) 1240 | 578; 20,000 rows, 8 x 4 (10) 69 | 80. With 500
+// queries a warp each leaves the chip idle: 20,000 rows, 1 x 1 (0.3) 8.5 | 12.7,
+// 4 x 4 (5) 29 | 19. More than 64 entries a query take the block as well (up to
+// 2,688 of 16 bytes at 42 tables x 64 probes: 8 queries' would not fit in
+// shared memory).
+int scan_warps(int q_n, int r_n, int L, int probes, int nbins) {
+    const double expected = static_cast<double>(L) * probes * r_n / nbins;
+    const bool block = L * probes > 64 || expected >= 16.0 || (q_n <= 1024 && expected >= 2.0);
+    return block ? kScanWarps : 1;
 }
 
 }  // namespace
@@ -500,10 +619,17 @@ cudaError_t launch_lsh_scan(const uint8_t* q, const uint8_t* r, int q_n, int r_n
                             const uint32_t* ocode, float thr, int ratio, float dist_scale, uint32_t* matches,
                             uint32_t* counts, int32_t* nn_idx, float* nn_dist, cudaStream_t stream) {
     if (q_n <= 0) return cudaSuccess;
-    const long long blocks = (static_cast<long long>(q_n) * 32 + kScanThreads - 1) / kScanThreads;
-    lsh_scan_kernel<<<static_cast<unsigned>(blocks), kScanThreads, 0, stream>>>(
-        q, r, q_n, r_n, L, probes, shift, nbins, qcodes, start, order, ocode, thr, ratio, dist_scale, matches, counts,
-        nn_idx, nn_dist);
+    const int entries = L * probes;
+    const int nw = scan_warps(q_n, r_n, L, probes, nbins);
+    const size_t smem = scan_smem_bytes(entries, nw);
+    if (nw == 1)
+        lsh_scan_kernel<1><<<(q_n + kScanWarps - 1) / kScanWarps, kScanThreads, smem, stream>>>(
+            q, r, q_n, r_n, L, probes, shift, nbins, qcodes, start, order, ocode, thr, ratio, dist_scale, matches,
+            counts, nn_idx, nn_dist);
+    else
+        lsh_scan_kernel<kScanWarps><<<q_n, kScanThreads, smem, stream>>>(
+            q, r, q_n, r_n, L, probes, shift, nbins, qcodes, start, order, ocode, thr, ratio, dist_scale, matches,
+            counts, nn_idx, nn_dist);
     return cudaGetLastError();
 }
 
