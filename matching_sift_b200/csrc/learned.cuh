@@ -49,13 +49,16 @@ cudaError_t launch_probe_codes(const uint32_t* codes, const float* z, int n, int
 // One training step's data: R = 3B gathered rows [queries | their exact
 // nearest neighbours | random base rows].
 struct MlpTrainBufs {
-    float* h;        // [R][256] hidden (BF16-rounded, post-ReLU)
-    float* t;        // [R][32] tanh(z)
-    float* dz;       // [R][32]
-    float* da1;      // [R][256] gradient at the hidden pre-activation
-    float* colsum;   // [32] column sums of t
-    float* loss;     // [4] total, positive, negative, balance
+    float* h;          // [R][256] hidden (BF16-rounded, post-ReLU)
+    float* t;          // [R][32] tanh(z)
+    float* colpart;    // [forward blocks][32] column sums of t
+    float* colp;       // [32][32] column sums of t over rows p, p + 32, ...
+    float* part;       // [chunks][kMlpParamCount] shares of the gradients
+    float* terms;      // [B][2] positive and negative loss terms
 };
+// Scratch of a step of B pairs (256-byte aligned memory), and its arrays.
+size_t mlp_train_bytes(int B);
+MlpTrainBufs mlp_train_bufs_at(char* base, int B);
 struct MlpParams {  // FP32 master copies (+ gradients, Adam moments: same layout)
     float* w1;  // [256][128]
     float* b1;  // [256]
@@ -71,17 +74,22 @@ struct MlpLossWeights {
 };
 
 // Forward, loss and gradients for rows x[R][128] (R = 3B), weights from the
-// FP32 masters rounded to BF16 (w1b, w2b). Gradients are written (not
-// accumulated) into g; deterministic (no atomics on parameters).
-cudaError_t launch_mlp_loss_grad(const uint8_t* x, int B, int k, const MlpParams& p, const __nv_bfloat16* w1b,
-                                 const __nv_bfloat16* w2b, const MlpLossWeights& lw, MlpTrainBufs& tb,
-                                 const MlpParams& g, cudaStream_t stream);
-// Adam step on every parameter; refreshes the BF16 copies. step starts at 1.
-cudaError_t launch_mlp_adam(const MlpParams& p, const MlpParams& g, const MlpParams& m, const MlpParams& v, int k,
-                            int step, float lr, __nv_bfloat16* w1b, __nv_bfloat16* w2b, cudaStream_t stream);
-// FP32 masters -> BF16 copies (W1, W2 rows < k) and, when given, b1 / b2 (k entries).
-cudaError_t launch_mlp_export(const MlpParams& p, int k, __nv_bfloat16* w1b, __nv_bfloat16* w2b, float* b1_out,
-                              float* b2_out, cudaStream_t stream);
+// FP32 masters rounded to BF16 (w1t: W1 transposed, [128][256]; w2b).
+// Gradients are written (not accumulated) into g, loss[4] = total, positive,
+// negative, balance; deterministic (no atomics on parameters).
+cudaError_t launch_mlp_loss_grad(const uint8_t* x, int B, int k, const MlpParams& p, const __nv_bfloat16* w1t,
+                                 const __nv_bfloat16* w2b, const MlpLossWeights& lw, const MlpTrainBufs& tb,
+                                 const MlpParams& g, float* loss, cudaStream_t stream);
+// The same followed by the Adam step on every parameter (step starts at 1),
+// which refreshes w1t and w2b.
+cudaError_t launch_mlp_train_step(const uint8_t* x, int B, int k, const MlpParams& p, const MlpParams& m,
+                                  const MlpParams& v, __nv_bfloat16* w1t, __nv_bfloat16* w2b,
+                                  const MlpLossWeights& lw, const MlpTrainBufs& tb, int step, float lr, float* loss,
+                                  cudaStream_t stream);
+// FP32 masters -> BF16 copies (W1 as it is and / or transposed, W2 rows < k)
+// and, when given, b1 / b2 (k entries).
+cudaError_t launch_mlp_export(const MlpParams& p, int k, __nv_bfloat16* w1b, __nv_bfloat16* w1t, __nv_bfloat16* w2b,
+                              float* b1_out, float* b2_out, cudaStream_t stream);
 // Gathers the training rows of one step: for i < B with seed-derived choices
 // qi in [0, t_n), rows q[qi], base[nn[2 qi]], base[ri] (ri in [0, r_n)).
 cudaError_t launch_mlp_gather(const uint8_t* tq, int t_n, const int32_t* nn, const uint8_t* base, int r_n, int B,

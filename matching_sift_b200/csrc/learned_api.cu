@@ -154,32 +154,24 @@ int mlp_loss_grad(const uint8_t* x, int B, int k, const float* params, float neg
     SIFT_TRY(detail::ensure_ready(cp, dev));
     DeviceCtx& c = *cp;
     detail::ArenaLock lk(c, nullptr);
-    const int R = 3 * B;
     detail::Layout L;
-    const size_t o_w1b = L.take(kMlpHidden * kMlpIn * 2);
+    const size_t o_w1t = L.take(kMlpHidden * kMlpIn * 2);
     const size_t o_w2b = L.take(kMlpOutRows * kMlpHidden * 2);
-    const size_t o_h = L.take(static_cast<size_t>(R) * kMlpHidden * 4);
-    const size_t o_t = L.take(static_cast<size_t>(R) * kMlpOutRows * 4);
-    const size_t o_dz = L.take(static_cast<size_t>(R) * kMlpOutRows * 4);
-    const size_t o_da = L.take(static_cast<size_t>(R) * kMlpHidden * 4);
-    const size_t o_cs = L.take(kMlpOutRows * 4);
+    const size_t o_tb = L.take(mlp_train_bytes(B));
     const size_t o_loss = L.take(16);
     SIFT_TRY(detail::ensure_arena(c, L.off));
     char* A = c.arena;
     cudaStream_t st = nullptr;
     const MlpParams p = mlp_params_at(const_cast<float*>(params));
     const MlpParams g = mlp_params_at(grads);
-    auto* w1b = reinterpret_cast<__nv_bfloat16*>(A + o_w1b);
+    auto* w1t = reinterpret_cast<__nv_bfloat16*>(A + o_w1t);
     auto* w2b = reinterpret_cast<__nv_bfloat16*>(A + o_w2b);
-    SIFT_CUDA(cudaMemsetAsync(w2b, 0, kMlpOutRows * kMlpHidden * 2, st));
-    SIFT_CUDA(launch_mlp_export(p, k, w1b, w2b, nullptr, nullptr, st));
-    MlpTrainBufs tb{reinterpret_cast<float*>(A + o_h), reinterpret_cast<float*>(A + o_t),
-                    reinterpret_cast<float*>(A + o_dz), reinterpret_cast<float*>(A + o_da),
-                    reinterpret_cast<float*>(A + o_cs), reinterpret_cast<float*>(A + o_loss)};
-    SIFT_CUDA(launch_mlp_loss_grad(x, B, k, p, w1b, w2b, MlpLossWeights{neg_w, bal_w}, tb, g, st));
-    SIFT_CUDA(cudaMemcpyAsync(loss_host, tb.loss, 4 * sizeof(float), cudaMemcpyDeviceToHost, st));
-    SIFT_CUDA(cudaStreamSynchronize(st));
-    detail::g_launches += 9;
+    float* loss = reinterpret_cast<float*>(A + o_loss);
+    SIFT_CUDA(launch_mlp_export(p, k, nullptr, w1t, w2b, nullptr, nullptr, st));
+    SIFT_CUDA(launch_mlp_loss_grad(x, B, k, p, w1t, w2b, MlpLossWeights{neg_w, bal_w}, mlp_train_bufs_at(A + o_tb, B),
+                                   g, loss, st));
+    SIFT_CUDA(cudaMemcpyAsync(loss_host, loss, 4 * sizeof(float), cudaMemcpyDeviceToHost, st));
+    detail::g_launches += 4;
     return detail::collect_device_status(c, st);
 }
 
@@ -212,7 +204,6 @@ int mlp_train(const uint8_t* base, uint32_t r_n, const uint8_t* tq, uint32_t t_n
         return rc;
     }
     // Training buffers (one-off allocations: training is not on the search path).
-    const int R = 3 * batch;
     const size_t np = kMlpParamCount;
     std::vector<void*> owned;
     auto alloc = [&](size_t bytes) -> char* {
@@ -224,27 +215,22 @@ int mlp_train(const uint8_t* base, uint32_t r_n, const uint8_t* tq, uint32_t t_n
         owned.push_back(p);
         return static_cast<char*>(p);
     };
-    char* pm = alloc(4 * np * sizeof(float));
-    char* w1b = alloc(kMlpHidden * kMlpIn * 2);
+    char* pm = alloc(3 * np * sizeof(float));
+    char* w1t = alloc(kMlpHidden * kMlpIn * 2);
     char* w2b = alloc(kMlpOutRows * kMlpHidden * 2);
-    char* xb = alloc(static_cast<size_t>(R) * kMlpIn);
-    char* h = alloc(static_cast<size_t>(R) * kMlpHidden * 4);
-    char* t = alloc(static_cast<size_t>(R) * kMlpOutRows * 4);
-    char* dz = alloc(static_cast<size_t>(R) * kMlpOutRows * 4);
-    char* da = alloc(static_cast<size_t>(R) * kMlpHidden * 4);
-    char* cs = alloc(kMlpOutRows * 4);
+    char* xb = alloc(3 * static_cast<size_t>(batch) * kMlpIn);
+    char* tbm = alloc(mlp_train_bytes(batch));
     char* losses = alloc(static_cast<size_t>(steps + 1) * 4 * sizeof(float));
     auto release = [&]() {
         for (void* p : owned) cudaFree(p);
         cudaFree(nn);
     };
-    if (owned.size() != 10) {
+    if (owned.size() != 6) {
         release();
         return SIFT_ERR_ALLOC;
     }
     float* P = reinterpret_cast<float*>(pm);
-    const MlpParams p = mlp_params_at(P), g = mlp_params_at(P + np), mo = mlp_params_at(P + 2 * np),
-                    vo = mlp_params_at(P + 3 * np);
+    const MlpParams p = mlp_params_at(P), mo = mlp_params_at(P + np), vo = mlp_params_at(P + 2 * np);
     // Initial weights: W1 ~ N(0, 1/64) (pre-activations ~ N(0, 1) for inputs
     // of norm 512 / 64), W2 rows < k ~ N(0, 1/128), biases 0.
     std::vector<float> init(np, 0.0f);
@@ -260,26 +246,21 @@ int mlp_train(const uint8_t* base, uint32_t r_n, const uint8_t* tq, uint32_t t_n
         if (rc == SIFT_OK && e != cudaSuccess) rc = detail::map_cuda(e);
     };
     step_rc(cudaMemcpy(P, init.data(), np * sizeof(float), cudaMemcpyHostToDevice));
-    step_rc(cudaMemset(P + np, 0, 3 * np * sizeof(float)));
-    step_rc(cudaMemset(w2b, 0, kMlpOutRows * kMlpHidden * 2));
-    step_rc(launch_mlp_export(p, k, reinterpret_cast<__nv_bfloat16*>(w1b), reinterpret_cast<__nv_bfloat16*>(w2b),
-                              nullptr, nullptr, st));
-    MlpTrainBufs tb{reinterpret_cast<float*>(h), reinterpret_cast<float*>(t), reinterpret_cast<float*>(dz),
-                    reinterpret_cast<float*>(da), reinterpret_cast<float*>(cs), nullptr};
+    step_rc(cudaMemset(P + np, 0, 2 * np * sizeof(float)));
+    auto* w1t_p = reinterpret_cast<__nv_bfloat16*>(w1t);
+    auto* w2b_p = reinterpret_cast<__nv_bfloat16*>(w2b);
+    step_rc(launch_mlp_export(p, k, nullptr, w1t_p, w2b_p, nullptr, nullptr, st));
+    const MlpTrainBufs tb = mlp_train_bufs_at(tbm, batch);
     const MlpLossWeights lw{neg_w, bal_w};
     for (int s = 0; s < steps && rc == SIFT_OK; ++s) {
-        tb.loss = reinterpret_cast<float*>(losses) + 4 * s;
         step_rc(launch_mlp_gather(tq, static_cast<int>(t_n), nn, base, static_cast<int>(r_n), batch, seed, s,
                                   reinterpret_cast<uint8_t*>(xb), st));
-        step_rc(launch_mlp_loss_grad(reinterpret_cast<uint8_t*>(xb), batch, k, p,
-                                     reinterpret_cast<__nv_bfloat16*>(w1b), reinterpret_cast<__nv_bfloat16*>(w2b), lw,
-                                     tb, g, st));
-        step_rc(launch_mlp_adam(p, g, mo, vo, k, s + 1, lr, reinterpret_cast<__nv_bfloat16*>(w1b),
-                                reinterpret_cast<__nv_bfloat16*>(w2b), st));
-        detail::g_launches += 12;
+        step_rc(launch_mlp_train_step(reinterpret_cast<uint8_t*>(xb), batch, k, p, mo, vo, w1t_p, w2b_p, lw, tb, s + 1,
+                                      lr, reinterpret_cast<float*>(losses) + 4 * s, st));
+        detail::g_launches += 4;
     }
-    step_rc(launch_mlp_export(p, k, static_cast<__nv_bfloat16*>(w1_out), static_cast<__nv_bfloat16*>(w2_out), b1_out,
-                              b2_out, st));
+    step_rc(launch_mlp_export(p, k, static_cast<__nv_bfloat16*>(w1_out), nullptr, static_cast<__nv_bfloat16*>(w2_out),
+                              b1_out, b2_out, st));
     if (params_out) step_rc(cudaMemcpyAsync(params_out, P, np * sizeof(float), cudaMemcpyDeviceToDevice, st));
     if (loss_curve && steps > 0) {
         std::vector<float> lv(static_cast<size_t>(steps) * 4);

@@ -10,6 +10,23 @@
 // the data evenly). Gradients pass straight through the BF16 roundings of the
 // weights and of h. Every reduction runs in a fixed order, so a step is
 // deterministic.
+//
+// Three launches per step, FP32 throughout (CUDA cores):
+//   mlp_fwd_kernel   h and t of kFwdRows rows per block, column sums of t
+//   mlp_bwd_kernel   per (64 hidden units, chunk of pairs): dz, the hidden
+//                    gradient and the chunk's share of every weight gradient;
+//                    four more blocks form the pairs' loss terms
+//   mlp_reduce_kernel  the shares of all chunks, the loss, and in training the
+//                    Adam update with the BF16 copies of the next step
+// The step is bound by FP32 issue (0.43 GFMA at a batch of 2,048 pairs, 11 us
+// on 148 SMs) and by the latency of three short launches. Before: eight
+// launches, with the weight gradients in 8 and 32 blocks that walked all rows
+// (dW2 566 us, dW1 515 us) and W1 transposed through 2-byte shared stores in
+// every forward block (115 us). One step at 2,048 pairs, 16 bits (whole
+// mlp_loss_grad call): 865 -> 103 us, at 4,096 pairs 1,671 -> 168 us; 300 training
+// steps of 2,048 pairs with their labels 266 -> 25 ms. The gradients' error
+// against FP64 fell with the shorter sums (2,048 pairs: 1.0e-6 -> 1.4e-7 of the norm).
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -18,131 +35,416 @@
 namespace sift {
 namespace {
 
-constexpr int kFwdRows = 32;
-constexpr size_t kFwdSmem = kMlpIn * kMlpHidden * 2 + kMlpHidden * kMlpOutRows * 4 + kFwdRows * kMlpIn * 4 +
-                            kFwdRows * kMlpHidden * 4;
+// ---------------------------------------------------------------- forward
+// 48 rows per block (128 blocks for 3 x 2,048 rows: one wave). W1 arrives
+// transposed ([in][hidden], 64 KB) so that it is copied as it is; warp w owns
+// rows 6 w .. 6 w + 5 and lane l hidden units 8 l .. 8 l + 7, so one 16-byte
+// load of weights and three broadcast loads of inputs feed 48 FMAs. Sums run
+// over the inputs (hidden units) in order.
+constexpr int kFwdRows = 48;
+constexpr int kFwdThreads = 256;
+constexpr int kFwdWarpRows = kFwdRows / (kFwdThreads / 32);
+constexpr int kFwdHPitch = kMlpHidden + 4;
+constexpr int kFwdW2Pitch = kMlpOutRows + 1;
+constexpr size_t kFwdSmem = kMlpIn * kMlpHidden * 2 + kMlpHidden * kFwdW2Pitch * 4 + kFwdRows * kMlpIn * 4 +
+                            kFwdRows * kFwdHPitch * 4;
 
-// Block of 256 threads per 32 rows. Thread j: hidden unit j of the 32 rows;
-// then 4 (row, output) pairs of layer 2.
-__global__ void __launch_bounds__(256) mlp_fwd_kernel(const uint8_t* __restrict__ x, int R,
-                                                      const __nv_bfloat16* __restrict__ w1b,
-                                                      const float* __restrict__ b1,
-                                                      const __nv_bfloat16* __restrict__ w2b,
-                                                      const float* __restrict__ b2, int k, float* __restrict__ h_out,
-                                                      float* __restrict__ t_out) {
-    extern __shared__ uint8_t smem[];
-    __nv_bfloat16* w1t = reinterpret_cast<__nv_bfloat16*>(smem);                 // [128][256]
-    float* w2t = reinterpret_cast<float*>(smem + kMlpIn * kMlpHidden * 2);          // [256][32]
-    float* xs = w2t + kMlpHidden * kMlpOutRows;                                     // [32][128]
-    float* hs = xs + kFwdRows * kMlpIn;                                             // [32][256]
-    const int tid = threadIdx.x;
-    for (int e = tid; e < kMlpIn * kMlpHidden; e += 256) {
-        const int j = e / kMlpIn, i = e % kMlpIn;
-        w1t[i * kMlpHidden + j] = w1b[e];
-    }
-    for (int e = tid; e < kMlpOutRows * kMlpHidden; e += 256) {
-        const int m = e / kMlpHidden, j = e % kMlpHidden;
-        w2t[j * kMlpOutRows + m] = m < k ? __bfloat162float(w2b[e]) : 0.0f;
-    }
+__global__ void __launch_bounds__(kFwdThreads, 1)
+    mlp_fwd_kernel(const uint8_t* __restrict__ x, int R, const __nv_bfloat16* __restrict__ w1t,
+                   const float* __restrict__ b1, const __nv_bfloat16* __restrict__ w2b, const float* __restrict__ b2,
+                   int k, float* __restrict__ h_out, float* __restrict__ t_out, float* __restrict__ colpart) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    uint8_t* w1s = smem;                                                            // [128][256] bf16
+    float* w2s = reinterpret_cast<float*>(smem + kMlpIn * kMlpHidden * 2);          // [256][33]
+    float* xs = w2s + kMlpHidden * kFwdW2Pitch;                                     // [128][48]
+    float* hs = xs + kFwdRows * kMlpIn;                                             // [48][260]
+    __shared__ float s_col[kFwdThreads / 32][32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = blockIdx.x * kFwdRows;
-    for (int e = tid; e < kFwdRows * kMlpIn; e += 256) {
-        const int r = e / kMlpIn;
-        xs[e] = row0 + r < R ? static_cast<float>(x[static_cast<size_t>(row0) * kMlpIn + e]) * kMlpInScale : 0.0f;
+    #pragma unroll 8
+    for (int e = tid; e < kMlpIn * kMlpHidden / 8; e += kFwdThreads)
+        reinterpret_cast<uint4*>(w1s)[e] = reinterpret_cast<const uint4*>(w1t)[e];
+    for (int e = tid; e < kFwdRows * 8; e += kFwdThreads) {
+        const int r = e % kFwdRows, c = e / kFwdRows;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (row0 + r < R) v = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row0 + r) * kMlpIn)[c];
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        #pragma unroll
+        for (int i = 0; i < 16; ++i)
+            xs[(16 * c + i) * kFwdRows + r] = static_cast<float>((w[i >> 2] >> (8 * (i & 3))) & 0xffu) * kMlpInScale;
+    }
+    for (int e = tid; e < kMlpOutRows * kMlpHidden; e += kFwdThreads) {
+        const int m = e / kMlpHidden, j = e % kMlpHidden;
+        w2s[j * kFwdW2Pitch + m] = m < k ? __bfloat162float(w2b[e]) : 0.0f;
     }
     __syncthreads();
     {
-        const int j = tid;
-        float acc[kFwdRows];
+        float acc[kFwdWarpRows][8];
         #pragma unroll
-        for (int r = 0; r < kFwdRows; ++r) acc[r] = 0.0f;
-        for (int i = 0; i < kMlpIn; ++i) {
-            const float w = __bfloat162float(w1t[i * kMlpHidden + j]);
+        for (int r = 0; r < kFwdWarpRows; ++r)
             #pragma unroll
-            for (int r = 0; r < kFwdRows; ++r) acc[r] = fmaf(xs[r * kMlpIn + i], w, acc[r]);
+            for (int c = 0; c < 8; ++c) acc[r][c] = 0.0f;
+        const uint4* wp = reinterpret_cast<const uint4*>(w1s) + lane;
+        const float* xp = xs + warp * kFwdWarpRows;
+        #pragma unroll 4
+        for (int i = 0; i < kMlpIn; ++i) {
+            const uint4 v = wp[i * (kMlpHidden / 8)];
+            const uint32_t w2[4] = {v.x, v.y, v.z, v.w};
+            float w[8];
+            #pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                w[2 * c] = __uint_as_float(w2[c] << 16);
+                w[2 * c + 1] = __uint_as_float(w2[c] & 0xffff0000u);
+            }
+            #pragma unroll
+            for (int r = 0; r < kFwdWarpRows; r += 2) {
+                const float2 xv = *reinterpret_cast<const float2*>(xp + i * kFwdRows + r);
+                #pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    acc[r][c] = fmaf(xv.x, w[c], acc[r][c]);
+                    acc[r + 1][c] = fmaf(xv.y, w[c], acc[r + 1][c]);
+                }
+            }
         }
-        const float bj = b1[j];
+        float bj[8];
         #pragma unroll
-        for (int r = 0; r < kFwdRows; ++r) {
-            const float hv = __bfloat162float(__float2bfloat16_rn(fmaxf(acc[r] + bj, 0.0f)));
-            hs[r * kMlpHidden + j] = hv;
-            if (row0 + r < R) h_out[static_cast<size_t>(row0 + r) * kMlpHidden + j] = hv;
+        for (int c = 0; c < 8; ++c) bj[c] = b1[8 * lane + c];
+        #pragma unroll
+        for (int r = 0; r < kFwdWarpRows; ++r) {
+            const int lr = warp * kFwdWarpRows + r;
+            float hv[8];
+            #pragma unroll
+            for (int c = 0; c < 8; ++c) hv[c] = __bfloat162float(__float2bfloat16_rn(fmaxf(acc[r][c] + bj[c], 0.0f)));
+            #pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                const float4 o = make_float4(hv[4 * g], hv[4 * g + 1], hv[4 * g + 2], hv[4 * g + 3]);
+                *reinterpret_cast<float4*>(hs + lr * kFwdHPitch + 8 * lane + 4 * g) = o;
+                if (row0 + lr < R)
+                    *reinterpret_cast<float4*>(h_out + static_cast<size_t>(row0 + lr) * kMlpHidden + 8 * lane + 4 * g) =
+                        o;
+            }
         }
     }
+    __syncwarp();  // layer 2 reads the warp's own rows
+    float acc[kFwdWarpRows];
+    #pragma unroll
+    for (int r = 0; r < kFwdWarpRows; ++r) acc[r] = 0.0f;
+    #pragma unroll 2
+    for (int j = 0; j < kMlpHidden; j += 4) {
+        float w[4];
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) w[u] = w2s[(j + u) * kFwdW2Pitch + lane];
+        #pragma unroll
+        for (int r = 0; r < kFwdWarpRows; ++r) {
+            const float4 hv = *reinterpret_cast<const float4*>(hs + (warp * kFwdWarpRows + r) * kFwdHPitch + j);
+            acc[r] = fmaf(hv.x, w[0], acc[r]);
+            acc[r] = fmaf(hv.y, w[1], acc[r]);
+            acc[r] = fmaf(hv.z, w[2], acc[r]);
+            acc[r] = fmaf(hv.w, w[3], acc[r]);
+        }
+    }
+    const float bm = lane < k ? b2[lane] : 0.0f;
+    float col = 0.0f;
+    #pragma unroll
+    for (int r = 0; r < kFwdWarpRows; ++r) {
+        const int row = row0 + warp * kFwdWarpRows + r;
+        if (row < R) {
+            const float t = lane < k ? tanhf(acc[r] + bm) : 0.0f;
+            t_out[static_cast<size_t>(row) * kMlpOutRows + lane] = t;
+            col += t;
+        }
+    }
+    s_col[warp][lane] = col;
     __syncthreads();
-    const int m = tid & 31;
-    for (int r = tid >> 5; r < kFwdRows; r += 8) {
-        float acc = 0.0f;
-        for (int j = 0; j < kMlpHidden; ++j) acc = fmaf(hs[r * kMlpHidden + j], w2t[j * kMlpOutRows + m], acc);
-        if (row0 + r < R)
-            t_out[static_cast<size_t>(row0 + r) * kMlpOutRows + m] = m < k ? tanhf(acc + b2[m]) : 0.0f;
+    if (warp == 0) {
+        float c = 0.0f;
+        #pragma unroll
+        for (int w = 0; w < kFwdThreads / 32; ++w) c += s_col[w][lane];
+        colpart[static_cast<size_t>(blockIdx.x) * 32 + lane] = c;
     }
 }
 
-// colsum[m] = sum over rows of a[row][m] (width 32), one block, fixed order.
-__global__ void __launch_bounds__(1024) colsum32_kernel(const float* __restrict__ a, int R, float* __restrict__ out) {
-    __shared__ float part[32][33];
-    const int m = threadIdx.x & 31, p = threadIdx.x >> 5;
-    float s = 0.0f;
-    for (int r = p; r < R; r += 32) s += a[static_cast<size_t>(r) * kMlpOutRows + m];
-    part[p][m] = s;
-    __syncthreads();
-    if (p == 0) {
-        float t = 0.0f;
-        for (int q = 0; q < 32; ++q) t += part[q][m];
-        out[m] = t;
+// --------------------------------------------------------------- backward
+// Block (a, c): hidden units [64 a, 64 a + 64) and pairs [B c / C, B (c + 1) / C),
+// C = gridDim.y, 32 pairs (96 rows: queries, neighbours, random rows) at a time:
+// dz of the 96 rows, then per 32 rows the hidden gradient
+// da1[row][j] = (sum_m dz[row][m] W2[m][j]) (h[row][j] > 0) and the rank-32
+// updates dW1 += da1^T (x / 64) (4 x 8 outputs per thread, 64 x 128 per block),
+// dW2 += dz^T h, db1, db2. The next 32 rows' x and h load meanwhile. The four
+// blocks of a chunk recompute its dz (a few FMAs per row against the 8,192 of
+// its share of dW1). The chunk's sums go to part[c][kMlpParamCount].
+// Blocks (a, C) are the loss role, which only reads t and runs beside the
+// others: the terms of every pair and 32 strided column sums of t, in one fixed
+// order of additions (a thread per pair over the outputs in order; rows p,
+// p + 32, ... per strided sum) that does not depend on the chunks.
+constexpr int kBwdCols = 64;
+constexpr int kBwdPairs = 32;
+constexpr int kBwdThreads = 256;
+constexpr int kBwdColBlocks = kMlpHidden / kBwdCols;
+constexpr int kBwdMaxChunks = 36;  // + the loss role, x 4 column blocks = one block per SM
+constexpr int kBwdPitch = kBwdCols + 4, kBwdXPitch = kMlpIn + 4;
+constexpr size_t kBwdSmem =
+    (3 * kBwdPairs * 33 + 32 * kBwdPitch * 2 + 32 * kBwdXPitch + kMlpOutRows * kBwdCols + 32 + 8 * 32) * 4;
+
+__device__ __forceinline__ void loss_role(const float* __restrict__ t, int B, int k, int a, float* __restrict__ colp,
+                                          float* __restrict__ terms) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int R = 3 * B;
+    for (int p = a * (kBwdThreads / 32) + warp; p < 32; p += kBwdColBlocks * (kBwdThreads / 32)) {
+        float s = 0.0f;
+        #pragma unroll 16
+        for (int r = p; r < R; r += 32) s += t[static_cast<size_t>(r) * kMlpOutRows + lane];
+        colp[p * 32 + lane] = s;
+    }
+    for (int i = a * kBwdThreads + threadIdx.x; i < B; i += kBwdColBlocks * kBwdThreads) {
+        const float* tq = t + static_cast<size_t>(i) * kMlpOutRows;
+        const float* tp = t + (static_cast<size_t>(B) + i) * kMlpOutRows;
+        const float* tn = t + (2 * static_cast<size_t>(B) + i) * kMlpOutRows;
+        float sqp = 0.0f, sqn = 0.0f;
+        for (int j0 = 0; j0 < k; j0 += 4) {
+            const float4 q = *reinterpret_cast<const float4*>(tq + j0), p = *reinterpret_cast<const float4*>(tp + j0),
+                         n = *reinterpret_cast<const float4*>(tn + j0);
+            const float qv[4] = {q.x, q.y, q.z, q.w}, pv[4] = {p.x, p.y, p.z, p.w}, nv[4] = {n.x, n.y, n.z, n.w};
+            #pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (j0 + j < k) {
+                    sqp = fmaf(qv[j], pv[j], sqp);
+                    sqn = fmaf(qv[j], nv[j], sqn);
+                }
+            }
+        }
+        sqp /= k;
+        sqn /= k;
+        terms[2 * static_cast<size_t>(i)] = 1.0f - sqp;
+        terms[2 * static_cast<size_t>(i) + 1] = sqn * sqn;
     }
 }
 
-// One thread per pair i: dz of rows q_i, p_i, n_i and the pair's loss terms.
-__global__ void mlp_dz_kernel(const float* __restrict__ t, int B, int k, const float* __restrict__ colsum,
-                              MlpLossWeights lw, float* __restrict__ dz, float* __restrict__ terms) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B) return;
-    const float* tq = t + static_cast<size_t>(i) * kMlpOutRows;
-    const float* tp = t + static_cast<size_t>(B + i) * kMlpOutRows;
-    const float* tn = t + static_cast<size_t>(2 * B + i) * kMlpOutRows;
-    float sqp = 0.0f, sqn = 0.0f;
-    for (int j = 0; j < k; ++j) {
-        sqp += tq[j] * tp[j];
-        sqn += tq[j] * tn[j];
+__global__ void __launch_bounds__(kBwdThreads, 1)
+    mlp_bwd_kernel(const uint8_t* __restrict__ x, int B, int k, const float* __restrict__ h,
+                   const float* __restrict__ t, const __nv_bfloat16* __restrict__ w2b, MlpLossWeights lw,
+                   const float* __restrict__ colpart, int n_colpart, float* __restrict__ colp,
+                   float* __restrict__ terms, float* __restrict__ part) {
+    const int c = blockIdx.y, C = gridDim.y - 1;
+    if (c == C) {
+        loss_role(t, B, k, blockIdx.x, colp, terms);
+        return;
     }
-    sqp /= k;
-    sqn /= k;
+    extern __shared__ __align__(16) uint8_t smem[];
+    float* hs = reinterpret_cast<float*>(smem);        // [32][68]
+    float* as = hs + 32 * kBwdPitch;                   // [32][68]
+    float* xs = as + 32 * kBwdPitch;                   // [32][132]
+    float* w2s = xs + 32 * kBwdXPitch;                 // [32][64]
+    float* dzs = w2s + kMlpOutRows * kBwdCols;         // [96][33]
+    float* cs = dzs + 3 * kBwdPairs * 33;              // [32]
+    float* red = cs + 32;                              // [8][32]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int col0 = blockIdx.x * kBwdCols;
+    const int i_begin = static_cast<int>(static_cast<long long>(B) * c / C);
+    const int i_end = static_cast<int>(static_cast<long long>(B) * (c + 1) / C);
     const float rows = 3.0f * B;
-    const float cp = -1.0f / (k * static_cast<float>(B));
-    const float cn = lw.neg * 2.0f * sqn / (k * static_cast<float>(B));
-    float* dq = dz + static_cast<size_t>(i) * kMlpOutRows;
-    float* dp = dz + static_cast<size_t>(B + i) * kMlpOutRows;
-    float* dn = dz + static_cast<size_t>(2 * B + i) * kMlpOutRows;
-    for (int j = 0; j < kMlpOutRows; ++j) {
-        if (j < k) {
-            const float bal = lw.balance * 2.0f * (colsum[j] / rows) / rows;
-            const float gq = cp * tp[j] + cn * tn[j] + bal;
-            const float gp = cp * tq[j] + bal;
-            const float gn = cn * tq[j] + bal;
-            dq[j] = gq * (1.0f - tq[j] * tq[j]);
-            dp[j] = gp * (1.0f - tp[j] * tp[j]);
-            dn[j] = gn * (1.0f - tn[j] * tn[j]);
+
+    {
+        float s = 0.0f;
+        for (int b = warp; b < n_colpart; b += kBwdThreads / 32) s += colpart[static_cast<size_t>(b) * 32 + lane];
+        red[warp * 32 + lane] = s;
+    }
+    for (int e = tid; e < kMlpOutRows * kBwdCols; e += kBwdThreads) {
+        const int m = e / kBwdCols, j = e % kBwdCols;
+        w2s[e] = m < k ? __bfloat162float(w2b[m * kMlpHidden + col0 + j]) : 0.0f;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        float s = 0.0f;
+        #pragma unroll
+        for (int w = 0; w < kBwdThreads / 32; ++w) s += red[w * 32 + lane];
+        cs[lane] = s;
+    }
+    __syncthreads();
+
+    // Outputs of this thread: dW1 rows 4 ty .. + 3 (hidden units), columns
+    // 4 tx .. + 3 and 64 + 4 tx .. + 3; dW2 row m2, columns 8 j2 .. + 7.
+    const int ty = tid >> 4, tx = tid & 15;
+    const int m2 = tid >> 3, j2 = tid & 7;
+    float acc[4][8], acc2[8], b1s[4] = {0.0f, 0.0f, 0.0f, 0.0f}, b2s = 0.0f;
+    #pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        acc2[e] = 0.0f;
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q][e] = 0.0f;
+    }
+
+    // x and h of 32 rows [part p of pairs i0 ..): 16 bytes of x and 32 of h per thread.
+    uint4 nx;
+    float4 nh[2];
+    auto fetch = [&](int p, int i0, int np) {
+        const int r = tid >> 3, q = tid & 7;
+        if (r < np) {
+            const size_t row = static_cast<size_t>(p) * B + i0 + r;
+            nx = reinterpret_cast<const uint4*>(x + row * kMlpIn)[q];
+            nh[0] = *reinterpret_cast<const float4*>(h + row * kMlpHidden + col0 + 8 * q);
+            nh[1] = *reinterpret_cast<const float4*>(h + row * kMlpHidden + col0 + 8 * q + 4);
         } else {
-            dq[j] = dp[j] = dn[j] = 0.0f;
+            nx = make_uint4(0u, 0u, 0u, 0u);
+            nh[0] = nh[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+
+    if (i_begin < i_end) fetch(0, i_begin, min(kBwdPairs, i_end - i_begin));
+    for (int i0 = i_begin; i0 < i_end; i0 += kBwdPairs) {
+        const int np = min(kBwdPairs, i_end - i0);
+        // dz of the 3 np rows: a warp per pair, a lane per output.
+        for (int pi = warp; pi < kBwdPairs; pi += kBwdThreads / 32) {
+            float dq = 0.0f, dp = 0.0f, dn = 0.0f;
+            if (pi < np) {
+                const size_t i = static_cast<size_t>(i0) + pi;
+                const float tq = t[i * kMlpOutRows + lane], tp = t[(B + i) * kMlpOutRows + lane],
+                            tn = t[(2 * static_cast<size_t>(B) + i) * kMlpOutRows + lane];
+                float sqn = tq * tn;  // zero for lanes >= k
+                #pragma unroll
+                for (int o = 16; o > 0; o >>= 1) sqn += __shfl_xor_sync(0xffffffffu, sqn, o);
+                sqn /= k;
+                const float cp = -1.0f / (k * static_cast<float>(B));
+                const float cn = lw.neg * 2.0f * sqn / (k * static_cast<float>(B));
+                if (lane < k) {
+                    const float bal = lw.balance * 2.0f * (cs[lane] / rows) / rows;
+                    dq = (cp * tp + cn * tn + bal) * (1.0f - tq * tq);
+                    dp = (cp * tq + bal) * (1.0f - tp * tp);
+                    dn = (cn * tq + bal) * (1.0f - tn * tn);
+                }
+            }
+            dzs[pi * 33 + lane] = dq;
+            dzs[(kBwdPairs + pi) * 33 + lane] = dp;
+            dzs[(2 * kBwdPairs + pi) * 33 + lane] = dn;
+        }
+        for (int p = 0; p < 3; ++p) {
+            {
+                const int r = tid >> 3, q = tid & 7;
+                const uint32_t w[4] = {nx.x, nx.y, nx.z, nx.w};
+                #pragma unroll
+                for (int g = 0; g < 4; ++g)
+                    *reinterpret_cast<float4*>(xs + r * kBwdXPitch + 16 * q + 4 * g) =
+                        make_float4(static_cast<float>(w[g] & 0xffu) * kMlpInScale,
+                                    static_cast<float>((w[g] >> 8) & 0xffu) * kMlpInScale,
+                                    static_cast<float>((w[g] >> 16) & 0xffu) * kMlpInScale,
+                                    static_cast<float>(w[g] >> 24) * kMlpInScale);
+                *reinterpret_cast<float4*>(hs + r * kBwdPitch + 8 * q) = nh[0];
+                *reinterpret_cast<float4*>(hs + r * kBwdPitch + 8 * q + 4) = nh[1];
+            }
+            if (p < 2)
+                fetch(p + 1, i0, np);
+            else if (i0 + kBwdPairs < i_end)
+                fetch(0, i0 + kBwdPairs, min(kBwdPairs, i_end - i0 - kBwdPairs));
+            __syncthreads();  // dzs, xs, hs
+            const float* dz = dzs + p * kBwdPairs * 33;
+            {
+                const int r = tid >> 3, q = tid & 7;
+                float s[8];
+                #pragma unroll
+                for (int e = 0; e < 8; ++e) s[e] = 0.0f;
+                for (int m = 0; m < k; ++m) {
+                    const float d = dz[r * 33 + m];
+                    const float4 wa = *reinterpret_cast<const float4*>(w2s + m * kBwdCols + 8 * q);
+                    const float4 wb = *reinterpret_cast<const float4*>(w2s + m * kBwdCols + 8 * q + 4);
+                    s[0] = fmaf(d, wa.x, s[0]);
+                    s[1] = fmaf(d, wa.y, s[1]);
+                    s[2] = fmaf(d, wa.z, s[2]);
+                    s[3] = fmaf(d, wa.w, s[3]);
+                    s[4] = fmaf(d, wb.x, s[4]);
+                    s[5] = fmaf(d, wb.y, s[5]);
+                    s[6] = fmaf(d, wb.z, s[6]);
+                    s[7] = fmaf(d, wb.w, s[7]);
+                }
+                const float* hr = hs + r * kBwdPitch + 8 * q;
+                #pragma unroll
+                for (int e = 0; e < 8; ++e) as[r * kBwdPitch + 8 * q + e] = hr[e] > 0.0f ? s[e] : 0.0f;
+            }
+            __syncthreads();  // as
+            #pragma unroll 4
+            for (int r = 0; r < 32; ++r) {
+                const float4 a = *reinterpret_cast<const float4*>(as + r * kBwdPitch + 4 * ty);
+                const float4 u = *reinterpret_cast<const float4*>(xs + r * kBwdXPitch + 4 * tx);
+                const float4 v = *reinterpret_cast<const float4*>(xs + r * kBwdXPitch + 64 + 4 * tx);
+                const float av[4] = {a.x, a.y, a.z, a.w};
+                const float bv[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+                #pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    #pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[q][e] = fmaf(av[q], bv[e], acc[q][e]);
+                    b1s[q] += av[q];
+                }
+            }
+            if (m2 < k) {
+                #pragma unroll 4
+                for (int r = 0; r < 32; ++r) {
+                    const float d = dz[r * 33 + m2];
+                    const float4 u = *reinterpret_cast<const float4*>(hs + r * kBwdPitch + 8 * j2);
+                    const float4 v = *reinterpret_cast<const float4*>(hs + r * kBwdPitch + 8 * j2 + 4);
+                    acc2[0] = fmaf(d, u.x, acc2[0]);
+                    acc2[1] = fmaf(d, u.y, acc2[1]);
+                    acc2[2] = fmaf(d, u.z, acc2[2]);
+                    acc2[3] = fmaf(d, u.w, acc2[3]);
+                    acc2[4] = fmaf(d, v.x, acc2[4]);
+                    acc2[5] = fmaf(d, v.y, acc2[5]);
+                    acc2[6] = fmaf(d, v.z, acc2[6]);
+                    acc2[7] = fmaf(d, v.w, acc2[7]);
+                    b2s += d;
+                }
+            }
+            __syncthreads();  // xs, hs, as and (after the last part) dzs are rewritten
         }
     }
-    terms[2 * i] = 1.0f - sqp;
-    terms[2 * i + 1] = sqn * sqn;
+
+    float* o = part + static_cast<size_t>(c) * kMlpParamCount;
+    float* o1 = o + static_cast<size_t>(col0) * kMlpIn;
+    #pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        float* row = o1 + (4 * ty + q) * kMlpIn + 4 * tx;
+        *reinterpret_cast<float4*>(row) = make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
+        *reinterpret_cast<float4*>(row + 64) = make_float4(acc[q][4], acc[q][5], acc[q][6], acc[q][7]);
+        if (tx == 0) o[kMlpHidden * kMlpIn + col0 + 4 * ty + q] = b1s[q];
+    }
+    float* o2 = o + kMlpHidden * kMlpIn + kMlpHidden;
+    float* row2 = o2 + m2 * kMlpHidden + col0 + 8 * j2;
+    *reinterpret_cast<float4*>(row2) = make_float4(acc2[0], acc2[1], acc2[2], acc2[3]);
+    *reinterpret_cast<float4*>(row2 + 4) = make_float4(acc2[4], acc2[5], acc2[6], acc2[7]);
+    if (blockIdx.x == 0 && j2 == 0) o2[kMlpOutRows * kMlpHidden + m2] = b2s;
 }
 
-// loss[0..3] = total, positive, negative, balance (one block, fixed order).
-__global__ void __launch_bounds__(256) mlp_loss_kernel(const float* __restrict__ terms, int B, int k,
-                                                       const float* __restrict__ colsum, MlpLossWeights lw,
-                                                       float* __restrict__ loss) {
-    __shared__ float sp[256], sn[256];
+// ------------------------------------------------- reduction and Adam step
+// g[i] = sum over chunks of part[c][i] (in order), a thread per parameter; the
+// last block forms loss[0..3] = total, positive, negative, balance from the
+// loss role's sums. ADAM: the update of parameter i and, for weights, the BF16
+// copies the next step reads (W1 transposed, W2 as it is). L2 bound: 4 C bytes
+// per parameter.
+struct AdamState {
+    float* p;
+    float* m;
+    float* v;
+    __nv_bfloat16* w1t;
+    __nv_bfloat16* w2b;
+    float lr, c1, c2;
+};
+
+// loss[0..3] = total, positive, negative, balance (one block of 256 threads, fixed order).
+__device__ __forceinline__ void loss_of_terms(const float* __restrict__ colp, const float* __restrict__ terms, int B,
+                                              int k, MlpLossWeights lw, float* __restrict__ loss) {
+    __shared__ float sp[256], sn[256], colsum[32];
     float a = 0.0f, b = 0.0f;
+    #pragma unroll 8
     for (int i = threadIdx.x; i < B; i += 256) {
-        a += terms[2 * i];
-        b += terms[2 * i + 1];
+        const float2 v = reinterpret_cast<const float2*>(terms)[i];
+        a += v.x;
+        b += v.y;
     }
     sp[threadIdx.x] = a;
     sn[threadIdx.x] = b;
+    if (threadIdx.x < 32) {
+        float t = 0.0f;
+        #pragma unroll
+        for (int q = 0; q < 32; ++q) t += colp[q * 32 + threadIdx.x];
+        colsum[threadIdx.x] = t;
+    }
     __syncthreads();
     for (int s = 128; s > 0; s >>= 1) {
         if (threadIdx.x < s) {
@@ -163,74 +465,48 @@ __global__ void __launch_bounds__(256) mlp_loss_kernel(const float* __restrict__
     }
 }
 
-// da1[row][j] = (sum_m dz[row][m] W2[m][j]) * (h[row][j] > 0); one block per row.
-__global__ void __launch_bounds__(256) mlp_dh_kernel(const float* __restrict__ dz, const float* __restrict__ h,
-                                                     const __nv_bfloat16* __restrict__ w2b, int k,
-                                                     float* __restrict__ da1) {
-    __shared__ float d[kMlpOutRows];
-    const size_t row = blockIdx.x;
-    if (threadIdx.x < kMlpOutRows) d[threadIdx.x] = dz[row * kMlpOutRows + threadIdx.x];
-    __syncthreads();
-    const int j = threadIdx.x;
-    float s = 0.0f;
-    for (int m = 0; m < k; ++m) s = fmaf(d[m], __bfloat162float(w2b[static_cast<size_t>(m) * kMlpHidden + j]), s);
-    da1[row * kMlpHidden + j] = h[row * kMlpHidden + j] > 0.0f ? s : 0.0f;
-}
-
-// out[a][b] = sum over rows of A[row][a] * Bm[row][b] * bscale (A: float
-// [R][wa]; Bm: float or u8 [R][wb]); 32 x 32 output tile per block, rows in
-// chunks of 32, fixed order. Also colA[a] = sum over rows of A[row][a] when
-// colA is given (from the blocks with blockIdx.y == 0).
-template <typename TB>
-__global__ void __launch_bounds__(256) wgrad_kernel(const float* __restrict__ A, int wa, const TB* __restrict__ Bm,
-                                                    int wb, float bscale, int R, float* __restrict__ out,
-                                                    float* __restrict__ colA) {
-    __shared__ float as[32][33], bs[32][33];
-    const int a0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 8 row groups of 4 outputs
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    float csum = 0.0f;
-    for (int r0 = 0; r0 < R; r0 += 32) {
-        for (int e = threadIdx.x; e < 32 * 32; e += 256) {
-            const int rr = e >> 5, cc = e & 31;
-            const int row = r0 + rr;
-            as[rr][cc] = row < R ? A[static_cast<size_t>(row) * wa + a0 + cc] : 0.0f;
-            bs[rr][cc] = row < R ? static_cast<float>(Bm[static_cast<size_t>(row) * wb + b0 + cc]) * bscale : 0.0f;
-        }
-        __syncthreads();
-        #pragma unroll 4
-        for (int rr = 0; rr < 32; ++rr) {
-            const float bv = bs[rr][tx];
-            #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[q] = fmaf(as[rr][ty * 4 + q], bv, acc[q]);
-        }
-        if (colA && blockIdx.y == 0 && threadIdx.x < 32)
-            for (int rr = 0; rr < 32; ++rr) csum += as[rr][threadIdx.x];
-        __syncthreads();
+template <bool ADAM>
+__global__ void __launch_bounds__(256)
+    mlp_reduce_kernel(const float* __restrict__ part, int C, const float* __restrict__ colp,
+                      const float* __restrict__ terms, int B, int k, MlpLossWeights lw, float* __restrict__ g,
+                      float* __restrict__ loss, const AdamState ad) {
+    if (blockIdx.x == gridDim.x - 1) {
+        loss_of_terms(colp, terms, B, k, lw, loss);
+        return;
     }
-    #pragma unroll
-    for (int q = 0; q < 4; ++q) out[static_cast<size_t>(a0 + ty * 4 + q) * wb + b0 + tx] = acc[q];
-    if (colA && blockIdx.y == 0 && threadIdx.x < 32) colA[a0 + threadIdx.x] = csum;
-}
-
-__global__ void mlp_adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                                float* __restrict__ v, int n, float lr, float c1, float c2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = 0.9f * m[i] + 0.1f * gi;
-    const float vi = 0.999f * v[i] + 0.001f * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + 1e-8f);
+    if (i < static_cast<int>(kMlpParamCount)) {
+        float s = 0.0f;
+        #pragma unroll 8
+        for (int c = 0; c < C; ++c) s += part[static_cast<size_t>(c) * kMlpParamCount + i];
+        if constexpr (ADAM) {
+            const float mi = 0.9f * ad.m[i] + 0.1f * s;
+            const float vi = 0.999f * ad.v[i] + 0.001f * s * s;
+            ad.m[i] = mi;
+            ad.v[i] = vi;
+            const float p = ad.p[i] - ad.lr * (mi / ad.c1) / (sqrtf(vi / ad.c2) + 1e-8f);
+            ad.p[i] = p;
+            const int w2 = i - (kMlpHidden * kMlpIn + kMlpHidden);
+            if (i < kMlpHidden * kMlpIn)
+                ad.w1t[(i % kMlpIn) * kMlpHidden + i / kMlpIn] = __float2bfloat16_rn(p);
+            else if (w2 >= 0 && w2 < k * kMlpHidden)
+                ad.w2b[w2] = __float2bfloat16_rn(p);
+        } else {
+            g[i] = s;
+        }
+    }
 }
 
+// FP32 masters -> BF16 weights: W1 as it is (w1b) or transposed (w1t), W2, and biases.
 __global__ void mlp_export_kernel(const float* __restrict__ w1, const float* __restrict__ b1,
                                   const float* __restrict__ w2, const float* __restrict__ b2, int k,
-                                  __nv_bfloat16* __restrict__ w1b, __nv_bfloat16* __restrict__ w2b,
-                                  float* __restrict__ b1o, float* __restrict__ b2o) {
+                                  __nv_bfloat16* __restrict__ w1b, __nv_bfloat16* __restrict__ w1t,
+                                  __nv_bfloat16* __restrict__ w2b, float* __restrict__ b1o, float* __restrict__ b2o) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kMlpHidden * kMlpIn) w1b[i] = __float2bfloat16_rn(w1[i]);
+    if (i < kMlpHidden * kMlpIn) {
+        if (w1b) w1b[i] = __float2bfloat16_rn(w1[i]);
+        if (w1t) w1t[i] = __float2bfloat16_rn(w1[(i % kMlpHidden) * kMlpIn + i / kMlpHidden]);
+    }
     if (i < k * kMlpHidden) w2b[i] = __float2bfloat16_rn(w2[i]);
     if (b1o && i < kMlpHidden) b1o[i] = b1[i];
     if (b2o && i < k) b2o[i] = b2[i];
@@ -277,44 +553,79 @@ MlpParams mlp_params_at(float* base) {
     return p;
 }
 
-cudaError_t launch_mlp_loss_grad(const uint8_t* x, int B, int k, const MlpParams& p, const __nv_bfloat16* w1b,
-                                 const __nv_bfloat16* w2b, const MlpLossWeights& lw, MlpTrainBufs& tb,
-                                 const MlpParams& g, cudaStream_t stream) {
+int mlp_fwd_blocks(int R) { return (R + kFwdRows - 1) / kFwdRows; }
+
+// One block per SM (4 column blocks x (36 chunks and the loss role)), at least 8 pairs per chunk.
+int mlp_bwd_chunks(int B) { return std::max(1, std::min(kBwdMaxChunks, B / 8)); }
+
+size_t mlp_train_bytes(int B) {
+    const size_t R = 3 * static_cast<size_t>(B), C = static_cast<size_t>(mlp_bwd_chunks(B));
+    return 4 * (R * (kMlpHidden + kMlpOutRows) + 32 * static_cast<size_t>(mlp_fwd_blocks(3 * B)) + 32 * 32 +
+                C * kMlpParamCount + 2 * static_cast<size_t>(B));
+}
+
+MlpTrainBufs mlp_train_bufs_at(char* base, int B) {
+    const size_t R = 3 * static_cast<size_t>(B), C = static_cast<size_t>(mlp_bwd_chunks(B));
+    MlpTrainBufs tb;
+    tb.h = reinterpret_cast<float*>(base);  // every array starts on a multiple of 32 floats
+    tb.t = tb.h + R * kMlpHidden;
+    tb.colpart = tb.t + R * kMlpOutRows;
+    tb.colp = tb.colpart + 32 * static_cast<size_t>(mlp_fwd_blocks(3 * B));
+    tb.part = tb.colp + 32 * 32;
+    tb.terms = tb.part + C * kMlpParamCount;
+    return tb;
+}
+
+namespace {
+
+cudaError_t launch_fwd_bwd(const uint8_t* x, int B, int k, const MlpParams& p, const __nv_bfloat16* w1t,
+                           const __nv_bfloat16* w2b, const MlpLossWeights& lw, const MlpTrainBufs& tb,
+                           cudaStream_t stream) {
     if (B <= 0 || k < 1 || k > kMlpMaxBits) return cudaErrorInvalidValue;
-    const int R = 3 * B;
+    const int R = 3 * B, blocks = mlp_fwd_blocks(R);
     cudaError_t e = cudaFuncSetAttribute(mlp_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kFwdSmem));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(mlp_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kBwdSmem));
     if (e != cudaSuccess) return e;
-    mlp_fwd_kernel<<<(R + kFwdRows - 1) / kFwdRows, 256, kFwdSmem, stream>>>(x, R, w1b, p.b1, w2b, p.b2, k, tb.h,
-                                                                             tb.t);
-    colsum32_kernel<<<1, 1024, 0, stream>>>(tb.t, R, tb.colsum);
-    // per-pair loss terms use the first 2B floats of da1 (written later)
-    float* terms = tb.da1;
-    mlp_dz_kernel<<<(B + 127) / 128, 128, 0, stream>>>(tb.t, B, k, tb.colsum, lw, tb.dz, terms);
-    mlp_loss_kernel<<<1, 256, 0, stream>>>(terms, B, k, tb.colsum, lw, tb.loss);
-    mlp_dh_kernel<<<R, 256, 0, stream>>>(tb.dz, tb.h, w2b, k, tb.da1);
-    // dW2 = dz^T h, db2 = colsum(dz); dW1 = da1^T (x / 64), db1 = colsum(da1)
-    wgrad_kernel<float><<<dim3(kMlpOutRows / 32, kMlpHidden / 32), 256, 0, stream>>>(
-        tb.dz, kMlpOutRows, tb.h, kMlpHidden, 1.0f, R, g.w2, g.b2);
-    wgrad_kernel<uint8_t><<<dim3(kMlpHidden / 32, kMlpIn / 32), 256, 0, stream>>>(
-        tb.da1, kMlpHidden, x, kMlpIn, kMlpInScale, R, g.w1, g.b1);
+    mlp_fwd_kernel<<<blocks, kFwdThreads, kFwdSmem, stream>>>(x, R, w1t, p.b1, w2b, p.b2, k, tb.h, tb.t, tb.colpart);
+    mlp_bwd_kernel<<<dim3(kBwdColBlocks, mlp_bwd_chunks(B) + 1), kBwdThreads, kBwdSmem, stream>>>(
+        x, B, k, tb.h, tb.t, w2b, lw, tb.colpart, blocks, tb.colp, tb.terms, tb.part);
     return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_adam(const MlpParams& p, const MlpParams& g, const MlpParams& m, const MlpParams& v, int k,
-                            int step, float lr, __nv_bfloat16* w1b, __nv_bfloat16* w2b, cudaStream_t stream) {
-    const int n = static_cast<int>(kMlpParamCount);
+constexpr int kReduceBlocks = static_cast<int>((kMlpParamCount + 255) / 256) + 1;  // + the loss
+
+}  // namespace
+
+cudaError_t launch_mlp_loss_grad(const uint8_t* x, int B, int k, const MlpParams& p, const __nv_bfloat16* w1t,
+                                 const __nv_bfloat16* w2b, const MlpLossWeights& lw, const MlpTrainBufs& tb,
+                                 const MlpParams& g, float* loss, cudaStream_t stream) {
+    const cudaError_t e = launch_fwd_bwd(x, B, k, p, w1t, w2b, lw, tb, stream);
+    if (e != cudaSuccess) return e;
+    mlp_reduce_kernel<false><<<kReduceBlocks, 256, 0, stream>>>(tb.part, mlp_bwd_chunks(B), tb.colp, tb.terms, B,
+                                                               k, lw, g.w1, loss, AdamState{});
+    return cudaGetLastError();
+}
+
+cudaError_t launch_mlp_train_step(const uint8_t* x, int B, int k, const MlpParams& p, const MlpParams& m,
+                                  const MlpParams& v, __nv_bfloat16* w1t, __nv_bfloat16* w2b,
+                                  const MlpLossWeights& lw, const MlpTrainBufs& tb, int step, float lr, float* loss,
+                                  cudaStream_t stream) {
+    const cudaError_t e = launch_fwd_bwd(x, B, k, p, w1t, w2b, lw, tb, stream);
+    if (e != cudaSuccess) return e;
     const float c1 = 1.0f - powf(0.9f, static_cast<float>(step));
     const float c2 = 1.0f - powf(0.999f, static_cast<float>(step));
-    mlp_adam_kernel<<<(n + 255) / 256, 256, 0, stream>>>(p.w1, g.w1, m.w1, v.w1, n, lr, c1, c2);
-    mlp_export_kernel<<<(kMlpHidden * kMlpIn + 255) / 256, 256, 0, stream>>>(p.w1, p.b1, p.w2, p.b2, k, w1b, w2b,
-                                                                          nullptr, nullptr);
+    mlp_reduce_kernel<true><<<kReduceBlocks, 256, 0, stream>>>(tb.part, mlp_bwd_chunks(B), tb.colp, tb.terms, B,
+                                                              k, lw, nullptr, loss,
+                                                              AdamState{p.w1, m.w1, v.w1, w1t, w2b, lr, c1, c2});
     return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_export(const MlpParams& p, int k, __nv_bfloat16* w1b, __nv_bfloat16* w2b, float* b1_out,
-                              float* b2_out, cudaStream_t stream) {
-    mlp_export_kernel<<<(kMlpHidden * kMlpIn + 255) / 256, 256, 0, stream>>>(p.w1, p.b1, p.w2, p.b2, k, w1b, w2b,
+cudaError_t launch_mlp_export(const MlpParams& p, int k, __nv_bfloat16* w1b, __nv_bfloat16* w1t, __nv_bfloat16* w2b,
+                              float* b1_out, float* b2_out, cudaStream_t stream) {
+    mlp_export_kernel<<<(kMlpHidden * kMlpIn + 255) / 256, 256, 0, stream>>>(p.w1, p.b1, p.w2, p.b2, k, w1b, w1t, w2b,
                                                                           b1_out, b2_out);
     return cudaGetLastError();
 }
