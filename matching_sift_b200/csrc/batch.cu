@@ -5,8 +5,8 @@
 // src/knn_brute.cu:24; its benchmark loops over calls, src/test.cu:194-216);
 // this has no counterpart there.
 //
-// Sequence per batch (one stream): query norms + bounds, base-tile records of
-// every problem, the search kernel over all units, the merge. A plan
+// Sequence per batch (one stream): query norms + bounds and base-tile records
+// of every problem, the search kernel over all units, the merge. A plan
 // (sift_batch_plan) owns its device memory, picks the kernel shape with a
 // small autotuner (times each shape on the batch itself) and captures the
 // sequence in a CUDA graph, so a repeated batch of the same sizes (new
@@ -128,16 +128,15 @@ int enqueue(DeviceCtx& c, const uint8_t* q, const uint8_t* r, uint32_t r_rows, c
             Shape sh, float thr, uint32_t* matches, int32_t* nn_idx, float* nn_dist, cudaStream_t st) {
     if (b.total_q == 0) return SIFT_OK;
     BatchPlan bp{b.plan, m.items, static_cast<int>(b.items.size()), b.total_tiles, b.group_rows};
-    SIFT_CUDA(launch_row_norms_u8(q, b.total_q, b.plan.q_pad, kMetricL2, m.qnorm, nullptr, m.thresh, st));
+    SIFT_CUDA(launch_batch_prep(r, q, b.total_q, bp, m.rec, m.qnorm, m.thresh, st));
     int launches = 2;
     if (b.units > 0) {
-        SIFT_CUDA(launch_batch_records(r, static_cast<int>(r_rows), bp, kMetricL2, m.rec, st));
         CUtensorMap qmap, rmap;
         SIFT_TRY(detail::encode_u8_rows(&qmap, q, static_cast<uint64_t>(b.total_q), kBM));
         SIFT_TRY(detail::encode_u8_rows(&rmap, r, r_rows, kBN / 2));
         SIFT_CUDA(launch_exact2nn_u8_pair_batch(qmap, rmap, m.rec, bp, m.partial, m.thresh, c.d_status, sh.qpt,
                                                 sh.qbuf, st));
-        launches += 2;
+        ++launches;
     }
     SIFT_CUDA(launch_merge2nn_batch(m.partial, bp, b.total_q, m.qnorm, kMetricL2, thr, 1.0f, matches, nullptr, nn_idx,
                                     nn_dist, st));

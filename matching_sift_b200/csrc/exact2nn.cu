@@ -289,41 +289,61 @@ __device__ __forceinline__ int find_item(int n_items, long long v, F key) {
     return lo;
 }
 
-// Base-tile records of a batch: block b fills quarter b % 4 of record b / 4;
-// the record belongs to the problem whose record range holds it, and rows of
-// its base set past n_b are padding (norm kKeyPad).
-__global__ void __launch_bounds__(256) batch_records_kernel(const uint8_t* __restrict__ x,
-                                                            const WorkItem* __restrict__ items, int n_items,
-                                                            int metric, int32_t* __restrict__ rec) {
-    const int T = blockIdx.x >> 2, part = blockIdx.x & 3;
-    const int p = find_item(n_items, T, [&](int k) { return static_cast<long long>(items[k].rec_off); });
-    const WorkItem it = items[p];
-    const int local = (T - it.rec_off) * kBN + part * 32 + (threadIdx.x >> 3);
-    const int sub = threadIdx.x & 7;
-    uint32_t s = 0;
-    if (local < it.n_b) {
-        const uint4 w = reinterpret_cast<const uint4*>(x + static_cast<size_t>(it.b_off + local) * kDim)[sub];
-        s = __dp4a(w.x, w.x, 0u);
-        s = __dp4a(w.y, w.y, s);
-        s = __dp4a(w.z, w.z, s);
-        s = __dp4a(w.w, w.w, s);
+// Norms of a batch in one launch, one block per 128 rows with four 16-byte row
+// loads in flight per thread. Blocks [0, tiles): the base-tile records of the
+// packed epilogue, K[col] = 127 - col - 128 |b|^2 (epilogue.cuh; the record
+// belongs to the problem whose record range holds it, rows of its base set past
+// n_b get 0). The blocks after them: query norms and cleared bounds. HBM-bound:
+// 128 bytes read per row, 4-8 written.
+__global__ void __launch_bounds__(256)
+    batch_prep_kernel(const uint8_t* __restrict__ base, const WorkItem* __restrict__ items, int n_items, int tiles,
+                      int32_t* __restrict__ rec, const uint8_t* __restrict__ q, int q_n, int q_pad,
+                      int32_t* __restrict__ qnorm, int32_t* __restrict__ thresh) {
+    const int sub = threadIdx.x & 7, lrow = threadIdx.x >> 3;
+    const bool is_base = static_cast<int>(blockIdx.x) < tiles;
+    const uint8_t* x = q;
+    int first = (blockIdx.x - tiles) * kBN, n = q_n;  // rows [first, first + 128) of x, valid below n
+    if (is_base) {
+        const int T = blockIdx.x;
+        // 32 probes per step instead of one: the largest p with rec_off <= T.
+        int lo = 0, hi = n_items;  // rec_off[lo] <= T < rec_off[hi]
+        while (hi - lo > 1) {
+            const int step = (hi - lo + 31) / 32;
+            const int at = lo + (threadIdx.x & 31) * step;
+            const bool le = at < hi && items[at].rec_off <= T;
+            const int k = __popc(__ballot_sync(0xffffffffu, le)) - 1;  // rec_off is non-decreasing
+            hi = min(hi, lo + (k + 1) * step);
+            lo += k * step;
+        }
+        const WorkItem& it = items[lo];
+        x = base + static_cast<size_t>(it.b_off) * kDim;
+        first = (T - it.rec_off) * kBN;
+        n = it.n_b;
     }
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 4);
-    const int32_t v = local < it.n_b ? (metric == kMetricL2 ? static_cast<int32_t>(s) : 0) : kKeyPad;
-    __shared__ int32_t nrm[32];
-    int32_t* r = rec + static_cast<size_t>(T) * kRecInts;
-    if (sub == 0) {
-        nrm[threadIdx.x >> 3] = v;
-        r[part * 32 + (threadIdx.x >> 3)] = v;
+    uint4 w[4];
+    #pragma unroll
+    for (int part = 0; part < 4; ++part) {
+        const int row = first + part * 32 + lrow;
+        w[part] = row < n ? load16_u8(x, row, sub, 1.0f) : make_uint4(0u, 0u, 0u, 0u);
     }
-    __syncthreads();
-    if (threadIdx.x < 4) {
-        int m = nrm[8 * threadIdx.x];
-        #pragma unroll
-        for (int i = 1; i < 8; ++i) m = min(m, nrm[8 * threadIdx.x + i]);
-        r[128 + part * 4 + threadIdx.x] = m;
+    #pragma unroll
+    for (int part = 0; part < 4; ++part) {
+        uint32_t s = __dp4a(w[part].x, w[part].x, 0u);
+        s = __dp4a(w[part].y, w[part].y, s);
+        s = __dp4a(w[part].z, w[part].z, s);
+        s = __dp4a(w[part].w, w[part].w, s);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 4);
+        const int col = part * 32 + lrow, row = first + col;
+        if (sub != 0) continue;
+        if (is_base) {
+            rec[static_cast<size_t>(blockIdx.x) * kRecInts + col] =
+                row < n ? 127 - col - 128 * static_cast<int32_t>(s) : 0;
+        } else if (row < q_pad) {
+            qnorm[row] = static_cast<int32_t>(s);
+            thresh[row] = INT_MAX;
+        }
     }
 }
 
@@ -892,10 +912,12 @@ cudaError_t launch_merge2nn_batch(const int4* partial, const BatchPlan& bp, int 
                                metric, threshold, dist_scale, MergeOut{matches, sorted, nn_idx, nn_dist}, stream);
 }
 
-cudaError_t launch_batch_records(const uint8_t* base, int, const BatchPlan& bp, int metric, int32_t* rec,
-                                 cudaStream_t stream) {
-    if (bp.total_tiles <= 0) return cudaSuccess;
-    batch_records_kernel<<<bp.total_tiles * 4, 256, 0, stream>>>(base, bp.items, bp.n_items, metric, rec);
+cudaError_t launch_batch_prep(const uint8_t* base, const uint8_t* q, int q_n, const BatchPlan& bp, int32_t* rec,
+                              int32_t* qnorm, int32_t* thresh, cudaStream_t stream) {
+    const int blocks = bp.total_tiles + bp.plan.q_tiles;
+    if (blocks <= 0) return cudaSuccess;
+    batch_prep_kernel<<<blocks, 256, 0, stream>>>(base, bp.items, bp.n_items, bp.total_tiles, rec, q, q_n,
+                                                  bp.plan.q_pad, qnorm, thresh);
     return cudaGetLastError();
 }
 

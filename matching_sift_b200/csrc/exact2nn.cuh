@@ -205,10 +205,11 @@ cudaError_t launch_merge2nn_chunks(const int4* partial, const ChunkSet& cs, int 
                                    float threshold, float dist_scale, uint32_t* matches, float4* sorted,
                                    int32_t* nn_idx, float* nn_dist, cudaStream_t stream);
 
-// Base-tile records of every problem of a batch (rows of base set p past
-// n_b[p] are padding), total_tiles records.
-cudaError_t launch_batch_records(const uint8_t* base, int base_rows, const BatchPlan& bp, int metric, int32_t* rec,
-                                 cudaStream_t stream);
+// Base-tile records of every problem of a batch for the packed epilogue
+// (bp.total_tiles records, the first 128 ints of each) and the norms and cleared
+// bounds of its q_n query rows.
+cudaError_t launch_batch_prep(const uint8_t* base, const uint8_t* q, int q_n, const BatchPlan& bp, int32_t* rec,
+                              int32_t* qnorm, int32_t* thresh, cudaStream_t stream);
 // Merge for a batch: query row q belongs to the problem whose range holds it;
 // indices are local to the problem's base set.
 cudaError_t launch_merge2nn_batch(const int4* partial, const BatchPlan& bp, int total_queries, const int32_t* qnorm,

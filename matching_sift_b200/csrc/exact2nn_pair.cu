@@ -199,9 +199,10 @@ struct Cursor {
 
 // has_lo (kModeFloat only): the rows carry lo blocks (split float rows); when
 // false they are plain FP16 rows and only the hi.hi products are formed.
-// TWO_PASS: the two-pass epilogue (single searches) or the one-pass scan
-// (batches of small problems).
-template <int MODE, int QPT, int QB, bool TWO_PASS>
+// PACKED (kModeU8, squared distances): the packed top-2 epilogue of batches,
+// whose records hold K (batch_prep_kernel); else the two-pass epilogue of
+// single searches.
+template <int MODE, int QPT, int QB, bool PACKED>
 __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtensorMap& bmap, const CUtensorMap& fmap,
                                           const int32_t* __restrict__ brec, const ExactPlan& plan,
                                           const WorkItem* __restrict__ items, int n_items, const WorkItem& single,
@@ -209,6 +210,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                                           int* __restrict__ err, float dscale, bool has_lo = false) {
     using Cfg = PairCfg<MODE, QPT, QB>;
     constexpr bool F16 = Cfg::F16;
+    static_assert(!PACKED || MODE == kModeU8, "packed keys are integers of u8 rows");
     // K blocks actually loaded per row (split rows without lo parts: the hi blocks only).
     const int kb_load = (MODE == kModeFloat && !has_lo) ? 2 : Cfg::kKBlocks;
     constexpr int kPStages = Cfg::kStages;
@@ -500,7 +502,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                     const int32_t* rec = r_smem + s * kRecInts;
                     constexpr int kKind = MODE == kModeFloat ? kAccFloat : (F16 ? kAccF32Int : kAccS32);
                     const int row0 = cur.it.idx_base + j * kBN;
-                    if constexpr (TWO_PASS) {
+                    if constexpr (!PACKED) {
                         // Two passes over the slot's 128 columns (8 chunks of 16).
                         // The first bounds every 8-row subgroup against the
                         // threshold held at its start, with no vote and no branch,
@@ -547,31 +549,32 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                         __syncwarp();
                         if (lane == 0) ptx::mbar_arrive_cluster_relaxed(lead_tempty);
                     } else {
-                        // One pass (batches: their bounds pass often, so exact
-                        // keys are formed at once from the registers): chunk c + 1
-                        // loads while chunk c is scanned, and the slot is handed
-                        // back as soon as the last chunk is in registers.
+                        // One pass over 8 chunks of 16 columns: chunk c + 1 loads
+                        // while chunk c is scanned, and the slot is handed back
+                        // as soon as the last chunk is in registers. Query rows
+                        // past the problem's set never pass.
                         uint32_t va[16], vb[16];
-                        auto scan = [&](const uint32_t (&v)[16], int c) {
-                            scan16<kKind>(v, row0 + 16 * c, rec + 16 * c, rec + kBN + 2 * c, st, dscale);
-                        };
+                        const int floor = valid ? packed_floor(st.thr) : INT_MAX;
+                        const int nv = cur.it.n_b - j * kBN;  // valid rows of the tile, if fewer than 128
+                        int m1 = floor, m2 = floor;
                         ptx::tmem_ld16(taddr, va);
                         ptx::tmem_ld_wait(va);
                         #pragma unroll
                         for (int c = 1; c < 8; c += 2) {
                             ptx::tmem_ld16(taddr + 16 * c, vb);
-                            scan(va, c - 1);
+                            packed16(va, 16 * (c - 1), nv, rec + 16 * (c - 1), m1, m2);
                             ptx::tmem_ld_wait(vb);
                             if (c + 1 < 8) {
                                 ptx::tmem_ld16(taddr + 16 * (c + 1), va);
-                                scan(vb, c);
+                                packed16(vb, 16 * c, nv, rec + 16 * c, m1, m2);
                                 ptx::tmem_ld_wait(va);
                             }
                         }
                         ptx::tc_fence_before();
                         __syncwarp();
                         if (lane == 0) ptx::mbar_arrive_cluster_relaxed(lead_tempty);
-                        scan(vb, 7);
+                        packed16(vb, 112, nv, rec + 112, m1, m2);
+                        packed_merge(m1, m2, floor, row0, st);
                     }
                     if (valid && st.k2 < published) {
                         atomicMin(thresh + q, st.k2);
@@ -613,7 +616,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CfgU8::kThreads, 1)
     exact2nn_u8_pair_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap bmap,
                             const int32_t* __restrict__ brec, const ExactPlan plan, const WorkItem single,
                             int4* __restrict__ partial, int32_t* __restrict__ thresh, int* __restrict__ err) {
-    pair_body<kModeU8, 2, 1, true>(qmap, bmap, qmap, brec, plan, nullptr, 1, single, partial, thresh, err, 1.0f);
+    pair_body<kModeU8, 2, 1, false>(qmap, bmap, qmap, brec, plan, nullptr, 1, single, partial, thresh, err, 1.0f);
 }
 
 // fmap: the folding digits (fold_records_kernel), a 2-D u8 tensor of
@@ -623,7 +626,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CfgFold::kThreads, 1
                                 const __grid_constant__ CUtensorMap fmap, const int32_t* __restrict__ brec,
                                 const ExactPlan plan, const WorkItem single, int4* __restrict__ partial,
                                 int32_t* __restrict__ thresh, int* __restrict__ err) {
-    pair_body<kModeU8Fold, 2, 1, true>(qmap, bmap, fmap, brec, plan, nullptr, 1, single, partial, thresh, err, 1.0f);
+    pair_body<kModeU8Fold, 2, 1, false>(qmap, bmap, fmap, brec, plan, nullptr, 1, single, partial, thresh, err, 1.0f);
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CfgF16::kThreads, 1)
@@ -631,7 +634,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CfgF16::kThreads, 1)
                              const int32_t* __restrict__ brec, const ExactPlan plan, const WorkItem single,
                              int4* __restrict__ partial, int32_t* __restrict__ thresh, int* __restrict__ err,
                              float dscale) {
-    pair_body<kModeF16Int, 2, 1, true>(qmap, bmap, qmap, brec, plan, nullptr, 1, single, partial, thresh, err,
+    pair_body<kModeF16Int, 2, 1, false>(qmap, bmap, qmap, brec, plan, nullptr, 1, single, partial, thresh, err,
                                        dscale);
 }
 
@@ -640,7 +643,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(CfgFloat::kThreads, 
                                const int32_t* __restrict__ brec, const ExactPlan plan, const WorkItem single,
                                int4* __restrict__ partial, int32_t* __restrict__ thresh, int* __restrict__ err,
                                int has_lo) {
-    pair_body<kModeFloat, 1, 1, true>(qmap, bmap, qmap, brec, plan, nullptr, 1, single, partial, thresh, err, 1.0f,
+    pair_body<kModeFloat, 1, 1, false>(qmap, bmap, qmap, brec, plan, nullptr, 1, single, partial, thresh, err, 1.0f,
                                       has_lo != 0);
 }
 
@@ -650,7 +653,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<kModeU8, QPT
                                   const int32_t* __restrict__ brec, const ExactPlan plan,
                                   const WorkItem* __restrict__ items, int n_items, int4* __restrict__ partial,
                                   int32_t* __restrict__ thresh, int* __restrict__ err) {
-    pair_body<kModeU8, QPT, QB, false>(qmap, bmap, qmap, brec, plan, items, n_items, WorkItem{}, partial, thresh, err,
+    pair_body<kModeU8, QPT, QB, true>(qmap, bmap, qmap, brec, plan, items, n_items, WorkItem{}, partial, thresh, err,
                                        1.0f);
 }
 
