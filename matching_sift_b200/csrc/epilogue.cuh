@@ -115,8 +115,15 @@ enum AccKind : int {
 // from the spread of the norms. At 500-8,000 base rows per problem a warp of 32
 // queries finds something new in more than half of its 16-row chunks, and the
 // scan with 8-row bounds and serial updates took ~4,800 cycles per unit there.
-// Measured: 512 image pairs (plan replay) 2,276 -> 1,216 us, mutual matching of
-// 128 pairs 1,175 -> 621 us.
+// Measured: 512 image pairs (plan replay) 2,276 -> 1,110 us, mutual matching of
+// 128 pairs 1,175 -> 585 us.
+// The first kPackedDenseTiles tiles of a base set (2,048 rows, where 60-100% of
+// the chunks hold something new for some of the 32 queries) run the network with
+// no test at all, so that the chunks overlap freely; later tiles skip a chunk by
+// a vote on its largest w. 512 pairs of 500-8,000 rows: always testing 1,251 us,
+// never 1,168, from tile 8 / 16 / 28 on 1,139 / 1,117 / 1,117; 64 pairs of
+// 7,000-8,000 rows: 863, 962, 848 / 843 / 855.
+constexpr int kPackedDenseTiles = 16;
 constexpr int kPackedMaxKey = 1 << 23;
 constexpr int kPackedNone = INT_MIN;  // w of a padding row: below every floor
 
@@ -138,8 +145,11 @@ __device__ __forceinline__ void top2_join(int& hi, int& lo, int h, int l) {
 
 // Rows [0, 16) of the chunk that starts at tile column c0: accumulators v, K at
 // k (16-byte aligned), nv valid rows in the tile; m1 >= m2: the running two
-// largest w.
-__device__ __forceinline__ void packed16(const uint32_t (&v)[16], int c0, int nv, const int32_t* k, int& m1, int& m2) {
+// largest w. DENSE: the network at once; else only where some lane's largest w
+// passes its second.
+template <bool DENSE>
+__device__ __forceinline__ void packed16(const uint32_t (&v)[16], int c0, int nv, const int32_t* k, int& m1,
+                                         int& m2) {
     int w[16];
     #pragma unroll
     for (int g = 0; g < 4; ++g) {
@@ -154,10 +164,7 @@ __device__ __forceinline__ void packed16(const uint32_t (&v)[16], int c0, int nv
         for (int e = 0; e < 16; ++e)
             if (c0 + e >= nv) w[e] = kPackedNone;
     }
-    int mx = max(w[0], w[1]);
-    #pragma unroll
-    for (int e = 2; e < 16; e += 2) mx = __vimax3_s32(mx, w[e], w[e + 1]);
-    if (__any_sync(0xffffffffu, mx > m2)) {
+    auto network = [&] {
         int hi, lo, h, l;
         top2_of4(w, hi, lo);
         #pragma unroll
@@ -166,6 +173,12 @@ __device__ __forceinline__ void packed16(const uint32_t (&v)[16], int c0, int nv
             top2_join(hi, lo, h, l);
         }
         top2_join(m1, m2, hi, lo);
+    };
+    if constexpr (DENSE) {
+        network();
+    } else {
+        const int mx = max(max8(reinterpret_cast<const uint32_t*>(w)), max8(reinterpret_cast<const uint32_t*>(w) + 8));
+        if (__any_sync(0xffffffffu, mx > m2)) network();
     }
 }
 

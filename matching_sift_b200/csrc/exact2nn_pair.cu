@@ -78,6 +78,7 @@
 //   exact2nn_u8_pair_batch_kernel<QPT, QB>  u8 batches with the shapes the
 //                             batch autotuner chooses from.
 #include <climits>
+#include <type_traits>
 #include "exact2nn.cuh"
 #include "ptx.cuh"
 #include "epilogue.cuh"
@@ -553,27 +554,34 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                         // while chunk c is scanned, and the slot is handed back
                         // as soon as the last chunk is in registers. Query rows
                         // past the problem's set never pass.
-                        uint32_t va[16], vb[16];
                         const int floor = valid ? packed_floor(st.thr) : INT_MAX;
                         const int nv = cur.it.n_b - j * kBN;  // valid rows of the tile, if fewer than 128
                         int m1 = floor, m2 = floor;
-                        ptx::tmem_ld16(taddr, va);
-                        ptx::tmem_ld_wait(va);
-                        #pragma unroll
-                        for (int c = 1; c < 8; c += 2) {
-                            ptx::tmem_ld16(taddr + 16 * c, vb);
-                            packed16(va, 16 * (c - 1), nv, rec + 16 * (c - 1), m1, m2);
-                            ptx::tmem_ld_wait(vb);
-                            if (c + 1 < 8) {
-                                ptx::tmem_ld16(taddr + 16 * (c + 1), va);
-                                packed16(vb, 16 * c, nv, rec + 16 * c, m1, m2);
-                                ptx::tmem_ld_wait(va);
+                        auto tile = [&](auto dense_tag) {
+                            constexpr bool DENSE = decltype(dense_tag)::value;
+                            uint32_t va[16], vb[16];
+                            ptx::tmem_ld16(taddr, va);
+                            ptx::tmem_ld_wait(va);
+                            #pragma unroll
+                            for (int c = 1; c < 8; c += 2) {
+                                ptx::tmem_ld16(taddr + 16 * c, vb);
+                                packed16<DENSE>(va, 16 * (c - 1), nv, rec + 16 * (c - 1), m1, m2);
+                                ptx::tmem_ld_wait(vb);
+                                if (c + 1 < 8) {
+                                    ptx::tmem_ld16(taddr + 16 * (c + 1), va);
+                                    packed16<DENSE>(vb, 16 * c, nv, rec + 16 * c, m1, m2);
+                                    ptx::tmem_ld_wait(va);
+                                }
                             }
-                        }
-                        ptx::tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive_cluster_relaxed(lead_tempty);
-                        packed16(vb, 112, nv, rec + 112, m1, m2);
+                            ptx::tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) ptx::mbar_arrive_cluster_relaxed(lead_tempty);
+                            packed16<DENSE>(vb, 112, nv, rec + 112, m1, m2);
+                        };
+                        if (j < kPackedDenseTiles)
+                            tile(std::true_type{});
+                        else
+                            tile(std::false_type{});
                         packed_merge(m1, m2, floor, row0, st);
                     }
                     if (valid && st.k2 < published) {

@@ -45,7 +45,7 @@ def test_extreme_keys_and_ties(cuda_device, shape):
 @pytest.mark.parametrize("shape", [0, 2])
 def test_base_set_ends(cuda_device, shape):
     rng = np.random.default_rng(7)
-    sizes = [1, 2, 15, 16, 17, 31, 33, 112, 113, 127, 128, 129, 255, 257, 640, 1025]
+    sizes = [1, 2, 15, 16, 17, 31, 33, 112, 113, 127, 128, 129, 255, 257, 640, 1025, 2047, 2049, 2190]
     sets_r = [rng.integers(0, 6, (n, 128)).astype(np.uint8) for n in sizes]
     # Queries equal rows of the NEXT base set: what lies past a set's end must not be found.
     sets_q = [np.concatenate([sets_r[(k + 1) % len(sizes)][:3], sets_r[k][-1:], rng.integers(0, 6, (1 + 60 * k, 128))]).astype(np.uint8)
