@@ -37,9 +37,15 @@
 // the issuing thread on the order of a hundred cycles, against 64 cycles per
 // 256 x 128 x 32 MMA, and one thread issuing every unit (8 MMAs, two barrier
 // tests, a commit) left the tensor pipe idle half of the time. Two issuer
-// threads, each owning one accumulator buffer (unit parity), share the work;
-// each tests its next unit's barriers behind its queued MMAs and commits once
-// per unit.
+// warps, each owning one accumulator buffer (unit parity), share the work.
+// Each runs its loop with all 32 lanes over its own units only, lane 0 issuing,
+// and waits for a tile's slot right before that tile's MMAs (try_wait blocks, so
+// testing the second slot first would hold the first back). A slot's turn is
+// epilogue 670 + release to issue 300 + issue 520 + commit to visible 300 cycles
+// (u8, norms folded); with both parities walked unit by unit by a single lane the
+// issuer spent ~840 cycles per own unit between its tests, on every slot's path.
+// 10,000 x 1,000,000 u8 1,344 -> 1,184 us per call, FP16 2,561 x 500,003
+// 427 -> 412, general float 2,053 x 131,077 345 -> 335, 512 pairs 1,118 -> 1,092.
 //
 // Barriers and who signals them (L = only the leader's copy is used):
 //   full[s]    (L) both CTAs' base halves of stage s landed        TMA tx
@@ -178,7 +184,11 @@ struct Cursor {
         g = it.tiles > 0 ? static_cast<int>(r / it.tiles) : 0;
         j = static_cast<int>(r - static_cast<long long>(g) * it.tiles);
     }
-    __device__ __forceinline__ bool last_of_group() const { return j + 1 == it.tiles; }
+    // `units` (at most to the end of the query group) units forward.
+    __device__ __forceinline__ void advance(int units) {
+        j += units - 1;
+        next();
+    }
     // One unit forward; true when the next unit opens a query group.
     __device__ __forceinline__ bool next() {
         if (++j < it.tiles) return false;
@@ -362,90 +372,88 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
         }
         __syncwarp();
     } else if (warp == 1 || warp == Cfg::kMma2Warp) {
-        if (lane == 0 && leader) {
+        if (leader) {
             // ------------------------------------------------- MMA issuers
-            // Thread mt issues the units n with n % 2 == mt (accumulator
-            // buffer mt); both walk every unit to follow the query groups.
+            // Warp mt issues the units n with n % 2 == mt (accumulator buffer
+            // mt). The whole warp walks its units, so that descriptors and
+            // barrier addresses stay in uniform registers; lane 0 issues.
             const int mt = warp == 1 ? 0 : 1;
+            const bool elect = lane == 0;
             constexpr uint32_t idesc = Cfg::kIdesc;
             constexpr int kMaxProd = MODE == kModeFloat ? 6 : Cfg::kKBlocks;
             const int n_prod = MODE == kModeFloat ? (has_lo ? 6 : 2) : Cfg::kKBlocks;
             const uint64_t b_desc0 = ptx::sdesc_sw128(b_s);
-            int ngroups = 0;
-            bool new_group = true;
-            uint64_t a_desc0 = ptx::sdesc_sw128(q_s);
-            int qb = 0;
-            bool pre_full = ptx::mbar_test_wait(bar_full + 8 * (mt % kPStages), 0);
-            bool pre_tempty = ptx::mbar_test_wait(bar_tempty + 8 * mt, 1);
-            for (int n = 0; n < n_units; ++n) {
-                if (new_group) {
-                    qb = ngroups % QB;
-                    if (!ptx::mbar_wait_cluster(bar_qfull + 8 * qb, (ngroups / QB) & 1, abort_flag, err, kErrWaitQuery))
-                        break;
-                    a_desc0 = ptx::sdesc_sw128(q_s + qb * Cfg::kQBufBytes);
-                    ++ngroups;
-                }
-                if ((n & 1) == mt) {
-                    const int s = n % kPStages;
-                    if (!pre_full &&
-                        !ptx::mbar_wait_cluster(bar_full + 8 * s, (n / kPStages) & 1, abort_flag, err, kErrWaitMmaFull))
-                        break;
-                    const uint32_t tpar_free = ((n >> 1) & 1) ^ 1;
+            int n = 0, ngroups = 0;
+            int s = mt;                    // base stage of the next own unit and its phase
+            uint32_t ph = 0, tfree = 1;    // ..., parity of its slots' free barriers
+            bool ok = true;
+            while (ok && n < n_units) {
+                // Units n .. n + seg - 1 share one query group.
+                const int seg = min(cur.it.tiles - cur.j, n_units - n);
+                const int qb = ngroups % QB;
+                ok = ptx::mbar_wait_cluster(bar_qfull + 8 * qb, (ngroups / QB) & 1, abort_flag, err, kErrWaitQuery);
+                ++ngroups;
+                const uint64_t a_desc0 = ptx::sdesc_sw128(q_s + qb * Cfg::kQBufBytes);
+                for (int m = n + ((n ^ mt) & 1); ok && m < n + seg; m += 2) {
+                    ok = ptx::mbar_wait_cluster(bar_full + 8 * s, ph, abort_flag, err, kErrWaitMmaFull);
                     const uint64_t b_desc = b_desc0 + static_cast<uint64_t>((s * kPBHalfBytes) >> 4);
-                    bool ok = true;
                     #pragma unroll
                     for (int t = 0; t < QPT; ++t) {
                         // Each tile's slot is handed back on its own: the tile's MMAs
                         // start as soon as its epilogue warps release it.
-                        if (!(t == 0 && pre_tempty) &&
-                            !ptx::mbar_wait_cluster(bar_tempty + 8 * (t * 2 + mt), tpar_free, abort_flag, err,
-                                                    kErrWaitMmaTmem)) {
-                            ok = false;
-                            break;
-                        }
+                        ok = ok && ptx::mbar_wait_cluster(bar_tempty + 8 * (t * 2 + mt), tfree, abort_flag, err,
+                                                          kErrWaitMmaTmem);
+                        if (!ok) break;
                         ptx::tc_fence_after();
                         const uint32_t d = tmem + (t * 2 + mt) * kBN;
-                        // K-block products: (kb, kb) for every block of the row;
-                        // split float rows: hi.hi for both K halves, then (with lo
-                        // parts) hi.lo' and lo.hi'.
-                        #pragma unroll
-                        for (int p = 0; p < kMaxProd; ++p) {
-                            if (p >= n_prod) break;
-                            const int ab = MODE == kModeFloat ? (p < 4 ? (p & 1) : 2 + (p & 1)) : p;
-                            const int bb = MODE == kModeFloat ? (p < 2 ? p : (p < 4 ? 2 + (p & 1) : (p & 1))) : p;
-                            const uint64_t a_desc =
-                                a_desc0 + static_cast<uint64_t>((t * kPQTileBytes + ab * Cfg::kQKBlock) >> 4);
-                            const uint64_t b_kb = b_desc + static_cast<uint64_t>((bb * Cfg::kBKBlock) >> 4);
+                        if (elect) {
+                            // K-block products: (kb, kb) for every block of the row;
+                            // split float rows: hi.hi for both K halves, then (with lo
+                            // parts) hi.lo' and lo.hi'.
                             #pragma unroll
-                            for (int kk = 0; kk < 4; ++kk) {
-                                const uint32_t acc = (p > 0 || kk > 0) ? 1u : 0u;
-                                if constexpr (F16)
-                                    ptx::mma_f16_pair(d, a_desc + 2 * kk, b_kb + 2 * kk, idesc, acc);
-                                else
-                                    ptx::mma_i8_pair(d, a_desc + 2 * kk, b_kb + 2 * kk, idesc, acc);
+                            for (int p = 0; p < kMaxProd; ++p) {
+                                if (p >= n_prod) break;
+                                const int ab = MODE == kModeFloat ? (p < 4 ? (p & 1) : 2 + (p & 1)) : p;
+                                const int bb = MODE == kModeFloat ? (p < 2 ? p : (p < 4 ? 2 + (p & 1) : (p & 1))) : p;
+                                const uint64_t a_desc =
+                                    a_desc0 + static_cast<uint64_t>((t * kPQTileBytes + ab * Cfg::kQKBlock) >> 4);
+                                const uint64_t b_kb = b_desc + static_cast<uint64_t>((bb * Cfg::kBKBlock) >> 4);
+                                #pragma unroll
+                                for (int kk = 0; kk < 4; ++kk) {
+                                    const uint32_t acc = (p > 0 || kk > 0) ? 1u : 0u;
+                                    if constexpr (F16)
+                                        ptx::mma_f16_pair(d, a_desc + 2 * kk, b_kb + 2 * kk, idesc, acc);
+                                    else
+                                        ptx::mma_i8_pair(d, a_desc + 2 * kk, b_kb + 2 * kk, idesc, acc);
+                                }
                             }
+                            if constexpr (Cfg::kFold)
+                                ptx::mma_i8_pair(d, ptx::sdesc_kmajor_noswz(a_s, 128, 256),
+                                                 ptx::sdesc_kmajor_noswz(f_s + s * Cfg::kFoldStage, 128, 256),
+                                                 ptx::idesc_make(2 /*S32*/, 0 /*u8*/, 1 /*s8*/, 2 * kBM, kBN), 1u);
+                            ptx::tc_commit_pair_mc(bar_tfull + 8 * (t * 2 + mt), kPairMask);
                         }
-                        if constexpr (Cfg::kFold)
-                            ptx::mma_i8_pair(d, ptx::sdesc_kmajor_noswz(a_s, 128, 256),
-                                             ptx::sdesc_kmajor_noswz(f_s + s * Cfg::kFoldStage, 128, 256),
-                                             ptx::idesc_make(2 /*S32*/, 0 /*u8*/, 1 /*s8*/, 2 * kBM, kBN), 1u);
-                        ptx::tc_commit_pair_mc(bar_tfull + 8 * (t * 2 + mt), kPairMask);
                     }
-                    if (!ok) break;
-                    // Test the barriers of this issuer's next unit (n + 2) behind its queued MMAs.
-                    if (n + 2 < n_units) {
-                        pre_full = ptx::mbar_test_wait(bar_full + 8 * ((n + 2) % kPStages), ((n + 2) / kPStages) & 1);
-                        pre_tempty = ptx::mbar_test_wait(bar_tempty + 8 * mt, (((n + 2) >> 1) & 1) ^ 1);  // tile 0
+                    s += 2;
+                    if (s >= kPStages) {
+                        s -= kPStages;
+                        ph ^= 1u;
                     }
+                    tfree ^= 1u;
                 }
+                if (!ok) break;
                 // Both issuers release the query buffer at the end of a group
                 // (each commit covers that issuer's own MMAs).
-                if (n + 1 == n_units || cur.last_of_group()) ptx::tc_commit_pair_mc(bar_qempty + 8 * qb, kPairMask);
-                new_group = cur.next();
+                if (elect) ptx::tc_commit_pair_mc(bar_qempty + 8 * qb, kPairMask);
+                n += seg;
+                cur.advance(seg);
             }
             // Drain: all issued MMAs complete before TMEM is released.
-            ptx::tc_commit_pair(bar_drain);
-            ptx::mbar_wait(bar_drain, 0, never, err, kErrWaitDrain);
+            __syncwarp();
+            if (elect) {
+                ptx::tc_commit_pair(bar_drain);
+                ptx::mbar_wait(bar_drain, 0, never, err, kErrWaitDrain);
+            }
         }
         __syncwarp();
     } else {
