@@ -429,7 +429,7 @@ int exact_match_chunked(const MatchArgs& a, DeviceCtx& c, cudaStream_t st, bool 
     const size_t o_r = L.take(static_cast<size_t>(r_n) * kDim + 16);
     const size_t o_brec = L.take(static_cast<size_t>(whole.base_tiles) * kRecInts * 4 + 16);
     const size_t o_qnorm = L.take(static_cast<size_t>(whole.q_pad) * 4);
-    const size_t o_thr = L.take(static_cast<size_t>(whole.q_pad) * 4);
+    const size_t o_thr = L.take(static_cast<size_t>(whole.q_pad) * 8);
     const size_t o_part = L.take(static_cast<size_t>(n_chunks) * cs.slot_stride * sizeof(int4));
     const size_t o_fold = fold ? L.take(static_cast<size_t>(whole.base_tiles) * 2 * kFoldHalfBytes) : 0;
     const size_t o_m = (a.matches && !m_dev) ? L.take(static_cast<size_t>(q_n) * 4) : 0;
@@ -540,7 +540,7 @@ int exact_match_float(const MatchArgs& a, DeviceCtx& c, cudaStream_t st) {
     const size_t o_rs = has_lo ? L.take(static_cast<size_t>(r_n) * 512 + 16) : 0;
     const size_t o_brec = L.take(static_cast<size_t>(plan.base_tiles) * kRecInts * 4 + 16);
     const size_t o_qnorm = L.take(static_cast<size_t>(plan.q_pad) * 4);
-    const size_t o_thr = L.take(static_cast<size_t>(plan.q_pad) * 4);
+    const size_t o_thr = L.take(static_cast<size_t>(plan.q_pad) * 8);
     const size_t o_part = L.take(static_cast<size_t>(plan.max_splits) * plan.parts * plan.q_pad * sizeof(int4));
     const size_t o_m = (a.matches && !m_dev) ? L.take(static_cast<size_t>(q_n) * 4) : 0;
     const size_t o_s = (a.sorted && !s_dev) ? L.take(static_cast<size_t>(q_n) * 16) : 0;
@@ -662,7 +662,7 @@ int exact_match(const MatchArgs& a) {
     SIFT_TRY(plan_inputs(a.q, a.r, use_f16 ? -1 : a.type, q_n, r_n, L, ip));
     const size_t o_brec = L.take(static_cast<size_t>(plan.base_tiles) * kRecInts * 4 + 16);
     const size_t o_qnorm = L.take(static_cast<size_t>(plan.q_pad) * 4);
-    const size_t o_thr = L.take(static_cast<size_t>(plan.q_pad) * 4);
+    const size_t o_thr = L.take(static_cast<size_t>(plan.q_pad) * 8);
     const size_t o_part = L.take(static_cast<size_t>(plan.max_splits) * plan.parts * plan.q_pad * sizeof(int4));
     const size_t o_m = (a.matches && !m_dev) ? L.take(static_cast<size_t>(q_n) * 4) : 0;
     const size_t o_s = (a.sorted && !s_dev) ? L.take(static_cast<size_t>(q_n) * 16) : 0;

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) row_norms_kernel(const T* __restrict__ x,
         nrm[threadIdx.x >> 3] = v;
         if (norm) norm[row] = v;
         if (r) r[part * 32 + (threadIdx.x >> 3)] = v;
-        if (thresh) thresh[row] = INT_MAX;
+        if (thresh) thresh[row] = thresh[n_pad + row] = INT_MAX;
     }
     __syncthreads();
     if (threadIdx.x < 4 && r) {
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(256) row_norms_float_kernel(const T* __restric
         nrm[threadIdx.x >> 3] = v;
         if (norm) norm[row] = __float_as_int(v);
         if (r) r[part * 32 + (threadIdx.x >> 3)] = __float_as_int(v);
-        if (thresh) thresh[row] = INT_MAX;
+        if (thresh) thresh[row] = thresh[n_pad + row] = INT_MAX;
     }
     __syncthreads();
     if (threadIdx.x < 4 && r) {
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(256)
                 row < n ? 127 - col - 128 * static_cast<int32_t>(s) : 0;
         } else if (row < q_pad) {
             qnorm[row] = static_cast<int32_t>(s);
-            thresh[row] = INT_MAX;
+            thresh[row] = thresh[q_pad + row] = INT_MAX;
         }
     }
 }

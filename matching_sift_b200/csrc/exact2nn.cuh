@@ -137,8 +137,10 @@ cudaError_t launch_merge2nn_float(const int4* partial, const ExactPlan& plan, in
 //   norm[n_pad]                       plain per-row norms
 //   rec[n_pad / kBN][kRecInts]        per base tile of kBN rows: the 128 norms
 //                                     and the 16 minima over 8-row groups
-//   thresh[n_pad]                     set to INT_MAX (the per-query shared
-//                                     pruning bound of the search kernel)
+//   thresh[2 n_pad]                   set to INT_MAX (the per-query shared
+//                                     pruning bounds of the search kernels: an
+//                                     upper bound of the final second-best key,
+//                                     then, n_pad further, the best key so far)
 cudaError_t launch_row_norms_u8(const uint8_t* x, int n, int n_pad, int metric, int32_t* norm, int32_t* rec,
                                 int32_t* thresh, cudaStream_t stream);
 // Records of the fold variant: residuals |b|^2 - 2 c (c = the folded
@@ -153,8 +155,8 @@ cudaError_t launch_row_norms_f16(const void* x, int n, int n_pad, float mul, int
 
 // The fused GEMM + top-2 kernel. partial: [max_splits][parts][q_pad] int4
 // {key1, idx1, key2, idx2} with key = norm(b) - 2 q.b. brec: base records
-// (see launch_row_norms_u8). thresh: [q_pad] per-query upper bounds of the
-// second-best key shared by the CTAs that split one query group.
+// (see launch_row_norms_u8). thresh: [2 q_pad] per-query bounds shared by the
+// CTAs that split one query group.
 cudaError_t launch_exact2nn_u8(const CUtensorMap& qmap, const CUtensorMap& bmap, const int32_t* brec,
                                const ExactPlan& plan, int4* partial, int32_t* thresh, int* err, cudaStream_t stream);
 

@@ -470,11 +470,21 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
         int split = 0, q = 0;
         bool active = false, valid = false, open = false;
         bool new_group = true;
-        // The query's shared bound is read one unit of this warp ahead: the
-        // value used for unit n was loaded while unit n - 2 was scanned, so
-        // the L2 round trip never waits in front of the first chunk. An older
-        // value is still a valid bound (bounds only decrease).
-        int next_thr = INT_MAX;
+        // The query's shared bounds are read one unit of this warp ahead: the
+        // values used for unit n were loaded while unit n - 2 was scanned, so
+        // the L2 round trip never waits in front of the first chunk. Older
+        // values are still valid (they only decrease). Two per query: an upper
+        // bound of the final second-best key, and (single searches) the best key
+        // of any list, thresh + q_pad. A list whose own best is not that one
+        // knows that two rows are at least as near as its best, so its best (not
+        // only its second) bounds the final second: over the 10-76 lists of a
+        // query the bound converges to the final second itself instead of to the
+        // smallest second of any list. FP16 2,561 x 500,003 412 -> 392 us, general
+        // float 2,053 x 131,077 335 -> 330, u8 10,000 x 1,000,000 1,183 -> 1,168;
+        // the 2-4 lists of a batch's query gain less than the second bound costs
+        // (512 pairs 1,092 -> 1,118), so batches keep one.
+        int32_t* const best_key = thresh + plan.q_pad;
+        int next_thr = INT_MAX, next_best = INT_MAX, published_best = INT_MAX;
 
         for (int n = 0; n < n_units; ++n) {
             if (new_group) {
@@ -482,7 +492,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                     partial[(static_cast<size_t>(split) * 2 + buf) * plan.q_pad + q] =
                         make_int4(st.k1, st.i1, st.k2, st.i2);
                 st = Top2{INT_MAX, -1, INT_MAX, -1, INT_MAX};
-                published = INT_MAX;
+                published = published_best = INT_MAX;
                 open = true;
                 const int q_local = ((cur.g * QPT + t) * 2 + static_cast<int>(rank)) * kBM + quarter * 32 + lane;
                 valid = q_local < cur.it.n_a;
@@ -490,11 +500,13 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                 split = pair - plan_cta_of(cur.group_first_unit(), W, G);
                 q = cur.it.a_off + q_local;
                 next_thr = valid ? __ldcg(thresh + q) : INT_MAX;
+                next_best = !PACKED && valid ? __ldcg(best_key + q) : INT_MAX;
             }
             const int j = cur.j;
             if ((n & 1) == buf) {
-                const int shared_thr = next_thr;
+                const int shared_thr = next_thr, shared_best = next_best;
                 next_thr = valid ? __ldcg(thresh + q) : INT_MAX;
+                next_best = !PACKED && valid ? __ldcg(best_key + q) : INT_MAX;
                 const int s = n % kPStages;
                 const uint32_t rpar = (n / kPStages) & 1, tpar = (static_cast<uint32_t>(n) >> 1) & 1;
                 // Both tests are issued back to back so their latencies overlap.
@@ -507,7 +519,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                 if (!__all_sync(0xffffffffu, waited)) break;
                 ptx::tc_fence_after();
                 if (active) {
-                    st.thr = min(st.thr, shared_thr);
+                    st.thr = min(st.thr, shared_best < st.k1 ? min(st.k1, shared_thr) : shared_thr);
                     const int32_t* rec = r_smem + s * kRecInts;
                     constexpr int kKind = MODE == kModeFloat ? kAccFloat : (F16 ? kAccF32Int : kAccS32);
                     const int row0 = cur.it.idx_base + j * kBN;
@@ -592,9 +604,16 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                             tile(std::false_type{});
                         packed_merge(m1, m2, floor, row0, st);
                     }
-                    if (valid && st.k2 < published) {
-                        atomicMin(thresh + q, st.k2);
-                        published = st.k2;
+                    if (valid) {
+                        const int second = shared_best < st.k1 ? st.k1 : st.k2;
+                        if (second < published) {
+                            atomicMin(thresh + q, second);
+                            published = second;
+                        }
+                        if (!PACKED && st.k1 < published_best) {
+                            atomicMin(best_key + q, st.k1);
+                            published_best = st.k1;
+                        }
                     }
                 } else {
                     ptx::tc_fence_before();

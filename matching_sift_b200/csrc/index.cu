@@ -95,7 +95,7 @@ void fallback_layout(detail::Layout& L, int q_n, int r_n, int num_workers, bool 
     fs.o_fd = L.take(static_cast<size_t>(q_n) * 8);
     fs.o_brec = own_brec ? L.take(static_cast<size_t>(worst.base_tiles) * kRecInts * 4 + 16) : 0;
     fs.o_fqn = L.take(static_cast<size_t>(worst.q_pad) * 4);
-    fs.o_fthr = L.take(static_cast<size_t>(worst.q_pad) * 4);
+    fs.o_fthr = L.take(static_cast<size_t>(worst.q_pad) * 8);
     fs.o_fpart = L.take(fs.fb_part);
     fs.own_brec = own_brec;
 }

@@ -160,7 +160,7 @@ extern "C" SIFT_API int sift2nn_match_noalloc(const uint8_t* q, const uint8_t* r
     const size_t o_qnorm = off;
     off = align256(off + static_cast<size_t>(plan.q_pad) * 4);
     const size_t o_thr = off;
-    off = align256(off + static_cast<size_t>(plan.q_pad) * 4);
+    off = align256(off + static_cast<size_t>(plan.q_pad) * 8);
     const size_t o_part = off;
     off = align256(off + static_cast<size_t>(plan.max_splits) * plan.parts * plan.q_pad * sizeof(int4));
     if (off > kNoAllocScratchBytes) return SIFT_ERR_INVALID_ARG;
