@@ -212,20 +212,31 @@ int collect_device_status(DeviceCtx& c, cudaStream_t st) {
 
 using namespace detail;
 
-// Largest power-of-two shift needed to make every q and r value (float or
-// half, device-readable) an integer, checked to keep them in [0, 255].
-int common_shift(DeviceCtx& c, const void* q, const void* r, bool half, int q_n, int r_n, cudaStream_t st,
-                 int& shift) {
+// What the survey of float / half inputs found (pack.cuh), read after one
+// synchronisation.
+struct ValueInfo {
+    uint32_t flags = 0;
+    int shift = 0;      // smallest s >= 0 that makes every value * 2^s an integer
+    float max_abs = 0;  // largest |value|
+    bool finite() const { return !(flags & kValueNotFinite); }
+    bool plain_u8() const { return !(flags & kValueNotU8); }
+    // Integers in [0, 255] times one power of two 2^-shift.
+    bool scaled_u8() const {
+        return !(flags & (kValueNotFixed | kValueNotFinite)) && shift <= kMaxShift && ldexpf(max_abs, shift) <= 255.0f;
+    }
+};
+
+int begin_survey(DeviceCtx& c, cudaStream_t st) {
     SIFT_CUDA(cudaMemsetAsync(c.d_status + 1, 0, 3 * sizeof(int), st));
-    SIFT_CUDA(launch_value_stats(q, half, q_n, c.d_status + 1, c.num_sms, st));
-    SIFT_CUDA(launch_value_stats(r, half, r_n, c.d_status + 1, c.num_sms, st));
+    return SIFT_OK;
+}
+
+int end_survey(DeviceCtx& c, cudaStream_t st, ValueInfo& info) {
     SIFT_CUDA(cudaMemcpyAsync(c.h_status + 1, c.d_status + 1, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
     SIFT_CUDA(cudaStreamSynchronize(st));
-    const int bad = c.h_status[1], s = c.h_status[2];
-    float mx = 0.0f;
-    std::memcpy(&mx, &c.h_status[3], sizeof(float));
-    if (bad || s > kMaxShift || ldexpf(mx, s) > 255.0f) return SIFT_ERR_NOT_INTEGER;
-    shift = s;
+    info.flags = static_cast<uint32_t>(c.h_status[1]);
+    info.shift = value_shift(static_cast<uint32_t>(c.h_status[2]));
+    std::memcpy(&info.max_abs, &c.h_status[3], sizeof(float));
     return SIFT_OK;
 }
 
@@ -292,9 +303,11 @@ int plan_inputs(const void* q, const void* r, int type, int q_n, int r_n, Layout
 
 // Produces 16-byte aligned device u8 rows for both sides (arena A laid out by plan_inputs).
 // shift: the inputs were integers times 2^-shift (0 for integer inputs); the
-// u8 rows hold the integers, so distances scale by 2^(-2 shift).
+// u8 rows hold the integers, so distances scale by 2^(-2 shift). Float / half
+// inputs that are no such integers return SIFT_ERR_NOT_INTEGER; `info` then
+// tells what the survey found.
 int stage_inputs(DeviceCtx& c, char* A, const InputPlan& ip, int type, const void* q, const void* r, int q_n,
-                 int r_n, cudaStream_t st, const uint8_t*& qd, const uint8_t*& rd, int& shift) {
+                 int r_n, cudaStream_t st, const uint8_t*& qd, const uint8_t*& rd, int& shift, ValueInfo& info) {
     shift = 0;
     if (type == SIFT_U8_DEVICE && !ip.stage_u8) {
         qd = static_cast<const uint8_t*>(q);
@@ -318,31 +331,20 @@ int stage_inputs(DeviceCtx& c, char* A, const InputPlan& ip, int type, const voi
         q_src = A + ip.o_qf;
         r_src = A + ip.o_rf;
     }
-    SIFT_CUDA(cudaMemsetAsync(c.d_status + 1, 0, sizeof(int), st));
     uint8_t* qo = reinterpret_cast<uint8_t*>(A + ip.o_qu8);
     uint8_t* ro = reinterpret_cast<uint8_t*>(A + ip.o_ru8);
-    g_launches += r_n > 0 ? 2 : 1;
     const bool half = type == SIFT_HALF_DEVICE;
-    auto pack = [&](float mul) -> int {
-        SIFT_CUDA(cudaMemsetAsync(c.d_status + 1, 0, sizeof(int), st));
-        if (half) {
-            SIFT_CUDA(launch_pack_f16_u8(q_src, q_n, mul, qo, c.d_status + 1, c.num_sms, st));
-            SIFT_CUDA(launch_pack_f16_u8(r_src, r_n, mul, ro, c.d_status + 1, c.num_sms, st));
-        } else {
-            SIFT_CUDA(launch_pack_f32_u8(static_cast<const float*>(q_src), q_n, mul, qo, c.d_status + 1, c.num_sms, st));
-            SIFT_CUDA(launch_pack_f32_u8(static_cast<const float*>(r_src), r_n, mul, ro, c.d_status + 1, c.num_sms, st));
-        }
-        SIFT_CUDA(cudaMemcpyAsync(c.h_status + 1, c.d_status + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-        SIFT_CUDA(cudaStreamSynchronize(st));
-        return c.h_status[1] != 0 ? SIFT_ERR_NOT_INTEGER : SIFT_OK;
-    };
-    if (pack(1.0f) != SIFT_OK) {
-        // Not plain integers: look for one power-of-two scale of all values.
-        int s = 0;
-        SIFT_TRY(common_shift(c, q_src, r_src, half, q_n, r_n, st, s));
-        g_launches += 2;
-        SIFT_TRY(pack(ldexpf(1.0f, s)));
-        shift = s;
+    // One pass surveys the values and packs them as they are; integers times a
+    // power of two are packed again with their scale.
+    SIFT_TRY(begin_survey(c, st));
+    SIFT_CUDA(launch_survey(q_src, q_n, r_src, r_n, half, qo, ro, c.d_status + 1, c.num_sms, st));
+    ++g_launches;
+    SIFT_TRY(end_survey(c, st, info));
+    if (!info.plain_u8()) {
+        if (!info.scaled_u8()) return SIFT_ERR_NOT_INTEGER;
+        SIFT_CUDA(launch_pack_u8(q_src, q_n, r_src, r_n, half, ldexpf(1.0f, info.shift), qo, ro, c.num_sms, st));
+        ++g_launches;
+        shift = info.shift;
     }
     qd = qo;
     rd = ro;
@@ -516,9 +518,9 @@ int exact_match_chunked(const MatchArgs& a, DeviceCtx& c, cudaStream_t st, bool 
 // of two 2^e that puts the largest |value| in [2^14, 2^15), and the dot
 // product is hi.hi' + hi.lo' + lo.hi' (22 significant bits per value, the
 // f32 accumulation of the tensor cores). Norms are f32 sums of the scaled
-// values. Distances come back in the caller's units (x 2^-2e). Caller holds
-// the arena lock.
-int exact_match_float(const MatchArgs& a, DeviceCtx& c, cudaStream_t st) {
+// values. Distances come back in the caller's units (x 2^-2e). `info`: the
+// survey of the inputs. Caller holds the arena lock.
+int exact_match_float(const MatchArgs& a, DeviceCtx& c, cudaStream_t st, const ValueInfo& info) {
     const int q_n = static_cast<int>(a.q_n), r_n = static_cast<int>(a.r_n);
     const bool half = a.type == SIFT_HALF_DEVICE;
     const bool host_in = a.type == SIFT_FLOAT_HOST;
@@ -558,39 +560,32 @@ int exact_match_float(const MatchArgs& a, DeviceCtx& c, cudaStream_t st) {
         q_src = A + o_qf;
         r_src = A + o_rf;
     }
-    // Largest |value| of both sets (and a finiteness check) for the scale.
-    SIFT_CUDA(cudaMemsetAsync(c.d_status + 1, 0, 2 * sizeof(int), st));
-    SIFT_CUDA(launch_abs_stats(q_src, half, q_n, c.d_status + 1, c.num_sms, st));
-    SIFT_CUDA(launch_abs_stats(r_src, half, r_n, c.d_status + 1, c.num_sms, st));
-    SIFT_CUDA(cudaMemcpyAsync(c.h_status + 1, c.d_status + 1, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    SIFT_CUDA(cudaStreamSynchronize(st));
-    if (c.h_status[1] != 0) return SIFT_ERR_INVALID_ARG;  // infinite or NaN values
-    float mx = 0.0f;
-    std::memcpy(&mx, &c.h_status[2], sizeof(float));
+    if (!info.finite()) return SIFT_ERR_INVALID_ARG;  // infinite or NaN values
     int e = 0;
-    if (has_lo && mx > 0.0f) {
+    if (has_lo && info.max_abs > 0.0f) {
         int ex = 0;
-        std::frexp(mx, &ex);  // mx in [2^(ex-1), 2^ex)
-        e = 15 - ex;          // mx * 2^e in [2^14, 2^15)
+        std::frexp(info.max_abs, &ex);  // largest |value| in [2^(ex-1), 2^ex)
+        e = 15 - ex;                    // times 2^e in [2^14, 2^15)
     }
     const float mul = ldexpf(1.0f, e);
-    g_launches += (r_n > 0 ? 2 : 1);
 
     const void* q_rows = q_src;
     const void* r_rows = r_src;
-    if (has_lo) {
-        SIFT_CUDA(launch_pack_split_f16(static_cast<const float*>(q_src), q_n, mul, A + o_qs, c.num_sms, st));
-        SIFT_CUDA(launch_pack_split_f16(static_cast<const float*>(r_src), r_n, mul, A + o_rs, c.num_sms, st));
-        q_rows = A + o_qs;
-        r_rows = A + o_rs;
-        g_launches += (r_n > 0 ? 2 : 1);
-    }
     int32_t* brec = reinterpret_cast<int32_t*>(A + o_brec);
     int32_t* qnorm = reinterpret_cast<int32_t*>(A + o_qnorm);
     int32_t* thresh = reinterpret_cast<int32_t*>(A + o_thr);
-    SIFT_CUDA(launch_row_norms_float(r_src, half, r_n, plan.r_pad, mul, a.metric, nullptr, brec, nullptr, st));
-    SIFT_CUDA(launch_row_norms_float(q_src, half, q_n, plan.q_pad, mul, kMetricL2, qnorm, nullptr, thresh, st));
-    g_launches += (plan.r_pad > 0 ? 1 : 0) + 1;
+    if (has_lo) {
+        SIFT_CUDA(launch_split_norms_f32(static_cast<const float*>(r_src), r_n, plan.r_pad, a.metric, A + o_rs, brec,
+                                         static_cast<const float*>(q_src), q_n, plan.q_pad, A + o_qs, qnorm, thresh,
+                                         mul, st));
+        q_rows = A + o_qs;
+        r_rows = A + o_rs;
+        ++g_launches;
+    } else {
+        SIFT_CUDA(launch_row_norms_float(r_src, r_n, plan.r_pad, a.metric, nullptr, brec, nullptr, st));
+        SIFT_CUDA(launch_row_norms_float(q_src, q_n, plan.q_pad, kMetricL2, qnorm, nullptr, thresh, st));
+        g_launches += (plan.r_pad > 0 ? 1 : 0) + 1;
+    }
     int4* partial = reinterpret_cast<int4*>(A + o_part);
     if (r_n > 0) {
         const uint64_t width = has_lo ? 2 * kDim : kDim;
@@ -679,35 +674,36 @@ int exact_match(const MatchArgs& a) {
     int shift = 0;
     // Values that are not integers times one power of two take the general
     // float path (float keys on the FP16 tensor cores).
+    int32_t* brec = reinterpret_cast<int32_t*>(A + o_brec);
+    int32_t* qnorm = reinterpret_cast<int32_t*>(A + o_qnorm);
+    int32_t* thresh = reinterpret_cast<int32_t*>(A + o_thr);
+    ValueInfo info;
     if (use_f16) {
-        const int rc = common_shift(c, a.q, a.r, true, q_n, r_n, st, shift);
-        g_launches += r_n > 0 ? 2 : 1;
-        if (rc == SIFT_ERR_NOT_INTEGER) return exact_match_float(a, c, st);
-        SIFT_TRY(rc);
+        // Survey, norms and records in one pass over the rows.
+        SIFT_TRY(begin_survey(c, st));
+        SIFT_CUDA(launch_survey_norms_f16(a.r, r_n, plan.base_tiles, a.metric, brec, a.q, q_n, plan.q_pad, qnorm, thresh,
+                                          c.d_status + 1, st));
+        ++g_launches;
+        SIFT_TRY(end_survey(c, st, info));
+        if (!info.scaled_u8()) return exact_match_float(a, c, st, info);
+        shift = info.shift;
     } else {
-        const int rc = stage_inputs(c, A, ip, a.type, a.q, a.r, q_n, r_n, st, qd, rd, shift);
+        const int rc = stage_inputs(c, A, ip, a.type, a.q, a.r, q_n, r_n, st, qd, rd, shift, info);
         if (rc == SIFT_ERR_NOT_INTEGER && a.type != SIFT_U8_DEVICE && a.type != SIFT_U8_HOST)
-            return exact_match_float(a, c, st);
+            return exact_match_float(a, c, st, info);
         SIFT_TRY(rc);
     }
 
     // ---- norms
-    int32_t* brec = reinterpret_cast<int32_t*>(A + o_brec);
-    int32_t* qnorm = reinterpret_cast<int32_t*>(A + o_qnorm);
-    int32_t* thresh = reinterpret_cast<int32_t*>(A + o_thr);
-    if (use_f16) {
-        const float mul = ldexpf(1.0f, shift);
-        SIFT_CUDA(launch_row_norms_f16(a.r, r_n, plan.r_pad, mul, a.metric, nullptr, brec, nullptr, st));
-        SIFT_CUDA(launch_row_norms_f16(a.q, q_n, plan.q_pad, mul, kMetricL2, qnorm, nullptr, thresh, st));
-    } else {
+    if (!use_f16) {
         if (use_fold)
             SIFT_CUDA(launch_fold_records_u8(rd, r_n, plan.r_pad, a.metric, brec,
                                              reinterpret_cast<uint32_t*>(A + o_fold), st));
         else
             SIFT_CUDA(launch_row_norms_u8(rd, r_n, plan.r_pad, a.metric, nullptr, brec, nullptr, st));
         SIFT_CUDA(launch_row_norms_u8(qd, q_n, plan.q_pad, kMetricL2, qnorm, nullptr, thresh, st));
+        g_launches += (plan.r_pad > 0 ? 1 : 0) + 1;
     }
-    g_launches += (plan.r_pad > 0 ? 1 : 0) + 1;
 
     // ---- fused GEMM + top-2
     int4* partial = reinterpret_cast<int4*>(A + o_part);
@@ -743,7 +739,7 @@ int exact_match(const MatchArgs& a) {
     int32_t* i_out = (a.nn_idx && !i_dev) ? reinterpret_cast<int32_t*>(A + o_i) : a.nn_idx;
     float* d_out = (a.nn_dist && !d_dev) ? reinterpret_cast<float*>(A + o_d) : a.nn_dist;
     SIFT_CUDA(launch_merge2nn(partial, plan, qnorm, a.metric, a.threshold, ldexpf(1.0f, -2 * shift), m_out, s_out,
-                              i_out, d_out, st));
+                              i_out, d_out, st, use_f16 ? ldexpf(1.0f, 2 * shift) : 0.0f));
     ++g_launches;
     if (a.matches && !m_dev)
         SIFT_CUDA(cudaMemcpyAsync(a.matches, m_out, static_cast<size_t>(q_n) * 4, cudaMemcpyDeviceToHost, st));
@@ -771,7 +767,7 @@ int encode_i8_rows(CUtensorMap* m, const void* base, uint64_t rows, uint32_t box
 // power of two): FP32 hash and scan on the CUDA cores over the caller's rows
 // (host float rows are copied to the device first); the bucketing is the u8
 // path's. Caller holds the arena lock and has checked the arguments.
-int lsh_match_float(const LshArgs& a, DeviceCtx& c, cudaStream_t st) {
+int lsh_match_float(const LshArgs& a, DeviceCtx& c, cudaStream_t st, const ValueInfo& info) {
     const int q_n = static_cast<int>(a.q_n), r_n = static_cast<int>(a.r_n);
     const int L_ = a.L, k = a.k;
     const int top = k < kLshMaxTopBits ? k : kLshMaxTopBits;
@@ -812,13 +808,7 @@ int lsh_match_float(const LshArgs& a, DeviceCtx& c, cudaStream_t st) {
         q_src = A + o_qf;
         r_src = A + o_rf;
     }
-    // Finite values only (the same check as the exact float path).
-    SIFT_CUDA(cudaMemsetAsync(c.d_status + 1, 0, 2 * sizeof(int), st));
-    SIFT_CUDA(launch_abs_stats(q_src, half, q_n, c.d_status + 1, c.num_sms, st));
-    SIFT_CUDA(launch_abs_stats(r_src, half, r_n, c.d_status + 1, c.num_sms, st));
-    SIFT_CUDA(cudaMemcpyAsync(c.h_status + 1, c.d_status + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    SIFT_CUDA(cudaStreamSynchronize(st));
-    if (c.h_status[1] != 0) return SIFT_ERR_INVALID_ARG;
+    if (!info.finite()) return SIFT_ERR_INVALID_ARG;  // as the exact float path
     int8_t* pl = reinterpret_cast<int8_t*>(A + o_pl);
     SIFT_CUDA(cudaMemcpyAsync(pl, a.planes, static_cast<size_t>(L_) * k * kDim, cudaMemcpyDefault, st));
     uint32_t* codes_r = reinterpret_cast<uint32_t*>(A + o_cr);
@@ -905,10 +895,11 @@ int lsh_match(const LshArgs& a) {
     const uint8_t* rd = nullptr;
     int vshift = 0;  // inputs were integers times 2^-vshift
     {
-        const int rc = stage_inputs(c, A, ip, a.type, a.q, a.r, q_n, r_n, st, qd, rd, vshift);
+        ValueInfo info;
+        const int rc = stage_inputs(c, A, ip, a.type, a.q, a.r, q_n, r_n, st, qd, rd, vshift, info);
         // General float values: the same hash and scan in FP32 on the caller's rows.
         if (rc == SIFT_ERR_NOT_INTEGER && a.type != SIFT_U8_DEVICE && a.type != SIFT_U8_HOST)
-            return lsh_match_float(a, c, st);
+            return lsh_match_float(a, c, st, info);
         SIFT_TRY(rc);
     }
     const int8_t* pl = a.planes;

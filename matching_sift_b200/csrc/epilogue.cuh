@@ -15,12 +15,6 @@ __device__ __forceinline__ int max8(const uint32_t* v) {
     return max(m, static_cast<int>(v[7]));
 }
 
-// An f32 accumulator holding an integer multiple of 1/dscale (dscale a power
-// of two; exact, see the FP16 kernel) -> the integer dot product.
-__device__ __forceinline__ int f32_dot(uint32_t bits, float dscale) {
-    return __float2int_rn(__uint_as_float(bits) * dscale);
-}
-
 // Per-thread running top-2 of one query row over base rows visited in
 // increasing index order (strict '<' keeps the lower index on ties).
 struct Top2 {
@@ -41,12 +35,7 @@ __device__ __forceinline__ void top2_update(Top2& s, int key, int idx) {
 }
 
 // One group of 32 consecutive base rows [row0, row0 + 32) for this thread's
-// query row; v[c] = q.b(row0 + c) as s32, or (F32) as the f32 accumulator of
-// the FP16 kernel, q.b / dscale. Those are never negative (inputs are
-// integers in [0, 255] times 2^-s), so their bit patterns, compared as int32,
-// order like the values (-0.0 only below +0.0, and both convert to 0): the
-// max trees run on the raw bits, and only the four subgroup maxima and the
-// values of passing subgroups are converted. nrm points at the group's 32 norms in the
+// query row; v[c] = q.b(row0 + c). nrm points at the group's 32 norms in the
 // shared-memory record, gm8 at its four 8-row minima. Each 8-row subgroup is
 // bounded from below by gm8[k] - 2 max(v[8k..8k+8)) (no key of its rows is
 // smaller), so a subgroup whose bound exceeds the thread's threshold holds no
@@ -54,15 +43,11 @@ __device__ __forceinline__ void top2_update(Top2& s, int key, int idx) {
 // forms its 8 exact keys and updates the top-2 only when their minimum is
 // within the threshold (a key above it cannot reach the final top-2: the
 // threshold never exceeds the final second-best key).
-template <bool F32 = false>
 __device__ __forceinline__ void scan_group(const uint32_t (&v)[32], int row0, const int32_t* nrm, const int32_t* gm8,
-                                           Top2& s, float dscale = 1.0f) {
+                                           Top2& s) {
     int mx[4];
     #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        mx[k] = max8(v + 8 * k);
-        if constexpr (F32) mx[k] = f32_dot(static_cast<uint32_t>(mx[k]), dscale);
-    }
+    for (int k = 0; k < 4; ++k) mx[k] = max8(v + 8 * k);
     const int4 g8 = *reinterpret_cast<const int4*>(gm8);
     const int bnd[4] = {g8.x - 2 * mx[0], g8.y - 2 * mx[1], g8.z - 2 * mx[2], g8.w - 2 * mx[3]};
     const int bmin = min(__vimin3_s32(bnd[0], bnd[1], bnd[2]), bnd[3]);
@@ -78,7 +63,7 @@ __device__ __forceinline__ void scan_group(const uint32_t (&v)[32], int row0, co
                     int key[8];
                     #pragma unroll
                     for (int e = 0; e < 8; ++e)
-                        key[e] = nr[e] - 2 * (F32 ? f32_dot(v[8 * k + e], dscale) : static_cast<int>(v[8 * k + e]));
+                        key[e] = nr[e] - 2 * static_cast<int>(v[8 * k + e]);
                     // Exact keys first; the (rare) updates only when one can enter.
                     int mk = __vimin3_s32(key[0], key[1], key[2]);
                     mk = __vimin3_s32(mk, key[3], key[4]);
@@ -98,7 +83,7 @@ __device__ __forceinline__ void scan_group(const uint32_t (&v)[32], int row0, co
 // Accumulator kinds of bound16 / exact8.
 enum AccKind : int {
     kAccS32 = 0,    // s32 dot products (u8 kernel)
-    kAccF32Int = 1, // f32 accumulators holding integer dot products / dscale (FP16 kernel)
+    kAccF32Int = 1, // f32 accumulators holding integer dot products / dscale (FP16 kernel), float norms
     kAccFloat = 2,  // f32 dot products of general floats (float keys, float norms)
 };
 
@@ -198,26 +183,28 @@ __device__ __forceinline__ void packed_merge(int m1, int m2, int floor, int row0
 // bound16: the pass bits of the chunk's two 8-row subgroups (bit k set when
 // subgroup k's lower bound, the 8-row minimum gm8[k] minus twice the largest
 // q.b of its rows, is within thr; the same bound as scan_group). gm8: the two
-// 8-row minima (8-byte aligned).
+// 8-row minima (8-byte aligned). kAccF32Int: minima and bounds are floats in
+// the units of the accumulators, exact, and thrf is thr in those units.
 template <int KIND>
-__device__ __forceinline__ uint32_t bound16(const uint32_t (&v)[16], const int32_t* gm8, int thr, float dscale) {
+__device__ __forceinline__ uint32_t bound16(const uint32_t (&v)[16], const int32_t* gm8, int thr, float thrf) {
     const int2 g8 = *reinterpret_cast<const int2*>(gm8);
     uint32_t bits = 0;
     #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const int g = k ? g8.y : g8.x;
-        int bnd;
+        bool pass;
         if constexpr (KIND == kAccFloat) {
             float m = __uint_as_float(v[8 * k]);
             #pragma unroll
             for (int e = 1; e < 8; ++e) m = fmaxf(m, __uint_as_float(v[8 * k + e]));
-            bnd = float_key(fmaf(-2.0f, m, __int_as_float(g)));
+            pass = float_key(fmaf(-2.0f, m, __int_as_float(g))) <= thr;
+        } else if constexpr (KIND == kAccF32Int) {
+            const float m = __uint_as_float(static_cast<uint32_t>(max8(v + 8 * k)));
+            pass = fmaf(-2.0f, m, __int_as_float(g)) <= thrf;
         } else {
-            int m = max8(v + 8 * k);
-            if constexpr (KIND == kAccF32Int) m = f32_dot(static_cast<uint32_t>(m), dscale);
-            bnd = g - 2 * m;
+            pass = g - 2 * max8(v + 8 * k) <= thr;
         }
-        bits |= (bnd <= thr ? 1u : 0u) << k;
+        bits |= (pass ? 1u : 0u) << k;
     }
     return bits;
 }
@@ -246,7 +233,7 @@ __device__ __forceinline__ void exact8(const uint32_t (&v)[8], int row0, const i
         if constexpr (KIND == kAccFloat)
             key[e] = float_key(fmaf(-2.0f, __uint_as_float(v[e]), __int_as_float(nr[e])));
         else if constexpr (KIND == kAccF32Int)
-            key[e] = nr[e] - 2 * f32_dot(v[e], dscale);
+            key[e] = __float2int_rn(fmaf(-2.0f, __uint_as_float(v[e]), __int_as_float(nr[e])) * dscale);
         else
             key[e] = nr[e] - 2 * static_cast<int>(v[e]);
     }

@@ -68,31 +68,11 @@ struct __align__(8) SmemCtl {
 constexpr size_t kSmemBytes =
     1024 + kQT * kQTileBytes + kStages * kBTileBytes + kStages * kRecBytes + sizeof(SmemCtl);
 
-// 16 consecutive elements of a row as u8 (FP16: value * mul, exact by contract).
-__device__ __forceinline__ uint4 load16_u8(const uint8_t* x, int row, int sub, float) {
+// 16 consecutive elements of a row.
+__device__ __forceinline__ uint4 load16_u8(const uint8_t* x, int row, int sub) {
     return reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * kDim)[sub];
 }
-__device__ __forceinline__ uint4 load16_u8(const __half* x, int row, int sub, float mul) {
-    const uint4* p = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * kDim) + 2 * sub;
-    uint32_t w[4];
-    #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint4 v = p[h];
-        const __half2* hv = reinterpret_cast<const __half2*>(&v);
-        #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const float2 a = __half22float2(hv[2 * k]), b = __half22float2(hv[2 * k + 1]);
-            w[2 * h + k] = static_cast<uint32_t>(__float2int_rn(a.x * mul)) |
-                           (static_cast<uint32_t>(__float2int_rn(a.y * mul)) << 8) |
-                           (static_cast<uint32_t>(__float2int_rn(b.x * mul)) << 16) |
-                           (static_cast<uint32_t>(__float2int_rn(b.y * mul)) << 24);
-        }
-    }
-    return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) row_norms_kernel(const T* __restrict__ x, int n, int n_pad, float mul,
+__global__ void __launch_bounds__(256) row_norms_kernel(const uint8_t* __restrict__ x, int n, int n_pad,
                                                         int metric, int32_t* __restrict__ norm,
                                                         int32_t* __restrict__ rec,
                                                         int32_t* __restrict__ thresh) {
@@ -101,7 +81,7 @@ __global__ void __launch_bounds__(256) row_norms_kernel(const T* __restrict__ x,
     const int sub = threadIdx.x & 7;
     uint32_t s = 0;
     if (row < n) {
-        const uint4 w = load16_u8(x, row, sub, mul);
+        const uint4 w = load16_u8(x, row, sub);
         s = __dp4a(w.x, w.x, 0u);
         s = __dp4a(w.y, w.y, s);
         s = __dp4a(w.z, w.z, s);
@@ -159,7 +139,7 @@ __global__ void __launch_bounds__(256) fold_records_kernel(const uint8_t* __rest
     #pragma unroll
     for (int part = 0; part < 4; ++part) {
         const int row = t * kBN + part * 32 + lrow;
-        w[part] = row < n ? load16_u8(x, row, sub, 1.0f) : make_uint4(0u, 0u, 0u, 0u);
+        w[part] = row < n ? load16_u8(x, row, sub) : make_uint4(0u, 0u, 0u, 0u);
     }
     __shared__ int32_t res[kBN];
     int32_t* r = rec + static_cast<size_t>(t) * kRecInts;
@@ -209,19 +189,8 @@ __global__ void __launch_bounds__(256) fold_records_kernel(const uint8_t* __rest
     }
 }
 
-// 16 consecutive elements of a row, times mul, as floats.
-__device__ __forceinline__ void load16_f32(const float* x, int row, int sub, float mul, float (&f)[16]) {
-    const float4* p = reinterpret_cast<const float4*>(x + static_cast<size_t>(row) * kDim) + 4 * sub;
-    #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        const float4 v = p[h];
-        f[4 * h] = v.x * mul;
-        f[4 * h + 1] = v.y * mul;
-        f[4 * h + 2] = v.z * mul;
-        f[4 * h + 3] = v.w * mul;
-    }
-}
-__device__ __forceinline__ void load16_f32(const __half* x, int row, int sub, float mul, float (&f)[16]) {
+// 16 consecutive elements of a row as floats.
+__device__ __forceinline__ void load16_f32(const __half* x, int row, int sub, float (&f)[16]) {
     const uint4* p = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * kDim) + 2 * sub;
     #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -230,18 +199,16 @@ __device__ __forceinline__ void load16_f32(const __half* x, int row, int sub, fl
         #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const float2 a = __half22float2(hv[k]);
-            f[8 * h + 2 * k] = a.x * mul;
-            f[8 * h + 2 * k + 1] = a.y * mul;
+            f[8 * h + 2 * k] = a.x;
+            f[8 * h + 2 * k + 1] = a.y;
         }
     }
 }
 
-// Squared norms of general (non-integer) float / half rows times mul, in FP32,
-// stored as float bit patterns in the int32 slots of the integer path (norm,
+// Squared norms of general (non-integer) half rows, in FP32, stored as float bit patterns in the int32 slots of the integer path (norm,
 // record norms and 8-row minima); padding rows get kFloatKeyPad. thresh is set
 // to INT_MAX (the largest ordered key, see float_key).
-template <typename T>
-__global__ void __launch_bounds__(256) row_norms_float_kernel(const T* __restrict__ x, int n, int n_pad, float mul,
+__global__ void __launch_bounds__(256) row_norms_float_kernel(const __half* __restrict__ x, int n, int n_pad,
                                                               int metric, int32_t* __restrict__ norm,
                                                               int32_t* __restrict__ rec,
                                                               int32_t* __restrict__ thresh) {
@@ -250,7 +217,7 @@ __global__ void __launch_bounds__(256) row_norms_float_kernel(const T* __restric
     float s = 0.0f;
     if (row < n) {
         float f[16];
-        load16_f32(x, row, sub, mul, f);
+        load16_f32(x, row, sub, f);
         #pragma unroll
         for (int i = 0; i < 16; ++i) s = fmaf(f[i], f[i], s);
     }
@@ -324,7 +291,7 @@ __global__ void __launch_bounds__(256)
     #pragma unroll
     for (int part = 0; part < 4; ++part) {
         const int row = first + part * 32 + lrow;
-        w[part] = row < n ? load16_u8(x, row, sub, 1.0f) : make_uint4(0u, 0u, 0u, 0u);
+        w[part] = row < n ? load16_u8(x, row, sub) : make_uint4(0u, 0u, 0u, 0u);
     }
     #pragma unroll
     for (int part = 0; part < 4; ++part) {
@@ -600,6 +567,7 @@ struct MergeOut {
     float4* sorted;
     int32_t* nn_idx;
     float* nn_dist;
+    float qmul = 0.0f;
 };
 
 // Distances, ratio test and outputs of query row q. Rows past the problem's
@@ -610,6 +578,7 @@ struct MergeOut {
 template <bool FLOATKEY>
 __device__ __forceinline__ void merge_finish(const MergeTop2& t, int q, int n_b, const int32_t* __restrict__ qnorm,
                                              int metric, float thr, float dscale, const MergeOut& out) {
+    // out.qmul (FP16 rows holding integers): query norms are floats, the integers divided by it.
     bool v1, v2;
     float d1, d2;
     if constexpr (FLOATKEY) {
@@ -624,7 +593,8 @@ __device__ __forceinline__ void merge_finish(const MergeTop2& t, int q, int n_b,
     } else {
         v1 = t.i1 >= 0 && t.i1 < n_b && t.k1 < kKeyPad;
         v2 = t.i2 >= 0 && t.i2 < n_b && t.k2 < kKeyPad;
-        const int qn = metric == kMetricL2 ? qnorm[q] : 0;
+        int qn = metric == kMetricL2 ? qnorm[q] : 0;
+        if (out.qmul > 0.0f) qn = __float2int_rn(__int_as_float(qn) * out.qmul);
         d1 = v1 ? static_cast<float>(t.k1 + qn) * dscale : FLT_MAX;
         d2 = v2 ? static_cast<float>(t.k2 + qn) * dscale : FLT_MAX;
     }
@@ -810,7 +780,7 @@ size_t exact2nn_smem_bytes() { return kSmemBytes; }
 cudaError_t launch_row_norms_u8(const uint8_t* x, int n, int n_pad, int metric, int32_t* norm, int32_t* rec,
                                 int32_t* thresh, cudaStream_t stream) {
     if (n_pad <= 0) return cudaSuccess;
-    row_norms_kernel<uint8_t><<<n_pad / 32, 256, 0, stream>>>(x, n, n_pad, 1.0f, metric, norm, rec, thresh);
+    row_norms_kernel<<<n_pad / 32, 256, 0, stream>>>(x, n, n_pad, metric, norm, rec, thresh);
     return cudaGetLastError();
 }
 
@@ -821,23 +791,11 @@ cudaError_t launch_fold_records_u8(const uint8_t* x, int n, int n_pad, int metri
     return cudaGetLastError();
 }
 
-cudaError_t launch_row_norms_f16(const void* x, int n, int n_pad, float mul, int metric, int32_t* norm, int32_t* rec,
-                                 int32_t* thresh, cudaStream_t stream) {
+cudaError_t launch_row_norms_float(const void* x, int n, int n_pad, int metric, int32_t* norm, int32_t* rec,
+                                   int32_t* thresh, cudaStream_t stream) {
     if (n_pad <= 0) return cudaSuccess;
-    row_norms_kernel<__half><<<n_pad / 32, 256, 0, stream>>>(static_cast<const __half*>(x), n, n_pad, mul, metric,
-                                                             norm, rec, thresh);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_row_norms_float(const void* x, bool half, int n, int n_pad, float mul, int metric, int32_t* norm,
-                                   int32_t* rec, int32_t* thresh, cudaStream_t stream) {
-    if (n_pad <= 0) return cudaSuccess;
-    if (half)
-        row_norms_float_kernel<__half><<<n_pad / 32, 256, 0, stream>>>(static_cast<const __half*>(x), n, n_pad, mul,
-                                                                       metric, norm, rec, thresh);
-    else
-        row_norms_float_kernel<float><<<n_pad / 32, 256, 0, stream>>>(static_cast<const float*>(x), n, n_pad, mul,
-                                                                      metric, norm, rec, thresh);
+    row_norms_float_kernel<<<n_pad / 32, 256, 0, stream>>>(static_cast<const __half*>(x), n, n_pad, metric, norm, rec,
+                                                           thresh);
     return cudaGetLastError();
 }
 
@@ -893,9 +851,9 @@ WorkItem merge_item(const ExactPlan& plan) {
 
 cudaError_t launch_merge2nn(const int4* partial, const ExactPlan& plan, const int32_t* qnorm, int metric,
                             float threshold, float dist_scale, uint32_t* matches, float4* sorted, int32_t* nn_idx,
-                            float* nn_dist, cudaStream_t stream) {
+                            float* nn_dist, cudaStream_t stream, float qnorm_mul) {
     return launch_merge<false>(partial, plan, nullptr, 1, merge_item(plan), kQT * kBM, plan.q_n, qnorm, metric,
-                               threshold, dist_scale, MergeOut{matches, sorted, nn_idx, nn_dist}, stream);
+                               threshold, dist_scale, MergeOut{matches, sorted, nn_idx, nn_dist, qnorm_mul}, stream);
 }
 
 cudaError_t launch_merge2nn_float(const int4* partial, const ExactPlan& plan, int group_rows, const int32_t* qnorm,

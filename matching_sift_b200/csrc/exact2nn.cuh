@@ -115,10 +115,10 @@ __device__ __forceinline__ int32_t float_key(float x) {
 __device__ __forceinline__ float key_float(int32_t k) { return __int_as_float(k >= 0 ? k : (k ^ 0x7fffffff)); }
 constexpr float kFloatKeyPad = 3.0e38f;  // norm of padding rows (never a real key)
 
-// Squared norms (float bit patterns) of n float or half rows times mul, laid
-// out as launch_row_norms_u8's outputs (norm / rec / thresh, each optional).
-cudaError_t launch_row_norms_float(const void* x, bool half, int n, int n_pad, float mul, int metric, int32_t* norm,
-                                   int32_t* rec, int32_t* thresh, cudaStream_t stream);
+// Squared norms (float bit patterns) of n half rows, laid out as
+// launch_row_norms_u8's outputs (norm / rec / thresh, each optional).
+cudaError_t launch_row_norms_float(const void* x, int n, int n_pad, int metric, int32_t* norm, int32_t* rec,
+                                   int32_t* thresh, cudaStream_t stream);
 // The CTA-pair search on FP16 rows with float keys: query and base rows are
 // [hi | lo] split rows of 256 halves (qmap / bmap_half: dims {256, rows}, box
 // {64, 128 / 64}) when has_lo, else plain FP16 rows of 128 halves (the lo
@@ -148,11 +148,6 @@ cudaError_t launch_row_norms_u8(const uint8_t* x, int n, int n_pad, int metric, 
 // folding digits of every row, n_pad / kBN tiles x 2 x kFoldHalfBytes bytes.
 cudaError_t launch_fold_records_u8(const uint8_t* x, int n, int n_pad, int metric, int32_t* rec, uint32_t* fold,
                                    cudaStream_t stream);
-// The same for FP16 rows whose values times mul (a power of two) are
-// integers in [0, 255].
-cudaError_t launch_row_norms_f16(const void* x, int n, int n_pad, float mul, int metric, int32_t* norm, int32_t* rec,
-                                 int32_t* thresh, cudaStream_t stream);
-
 // The fused GEMM + top-2 kernel. partial: [max_splits][parts][q_pad] int4
 // {key1, idx1, key2, idx2} with key = norm(b) - 2 q.b. brec: base records
 // (see launch_row_norms_u8). thresh: [2 q_pad] per-query bounds shared by the
@@ -219,7 +214,7 @@ cudaError_t launch_merge2nn_batch(const int4* partial, const BatchPlan& bp, int 
                                   int32_t* nn_idx, float* nn_dist, cudaStream_t stream);
 // FP16 rows (bmap_half / qmap: half tensor maps with boxes of 64 elements):
 // values are integers times 2^-s and dscale = 2^(2s) turns the f32 dot
-// products back into integers (brec built from the same integers).
+// products and norms (launch_survey_norms_f16) back into integers.
 cudaError_t launch_exact2nn_f16_pair(const CUtensorMap& qmap, const CUtensorMap& bmap_half, const int32_t* brec,
                                      const ExactPlan& plan, int4* partial, int32_t* thresh, int* err, float dscale,
                                      cudaStream_t stream);
@@ -232,10 +227,11 @@ size_t exact2nn_pair_smem_bytes();
 //   nn_idx[2q..] int32 indices (-1 where absent)
 //   nn_dist[2q..] float distances (FLT_MAX where absent)
 // dist_scale multiplies every distance (2^-2s for inputs that were integers
-// times 2^-s; 1 otherwise) before the ratio test and the outputs.
+// times 2^-s; 1 otherwise) before the ratio test and the outputs. qnorm_mul
+// (FP16 rows): qnorm holds floats, integers when multiplied by it.
 cudaError_t launch_merge2nn(const int4* partial, const ExactPlan& plan, const int32_t* qnorm, int metric,
                             float threshold, float dist_scale, uint32_t* matches, float4* sorted, int32_t* nn_idx,
-                            float* nn_dist, cudaStream_t stream);
+                            float* nn_dist, cudaStream_t stream, float qnorm_mul = 0.0f);
 
 size_t exact2nn_smem_bytes();
 

@@ -75,12 +75,12 @@
 //                             are integers times 2^-s (|integer| <= 255), so
 //                             every product and partial sum is an integer
 //                             multiple of 2^-2s below 2^24 * 2^-2s and the f32
-//                             accumulators are exact. The epilogue prunes on
-//                             the raw f32 bits (non-negative values order like
-//                             int32) and converts to the u8 kernel's integer
-//                             dot products (times dscale = 2^2s, rounded) only
-//                             the subgroup maxima and the values of passing
-//                             subgroups; the rest is shared.
+//                             accumulators are exact. The epilogue's max trees
+//                             run on the raw f32 bits (non-negative values order
+//                             like int32), its bounds in float (records hold
+//                             float norms), and only the values of passing
+//                             subgroups are converted to the u8 kernel's integer
+//                             keys (times dscale = 2^2s); the rest is shared.
 //   exact2nn_u8_pair_batch_kernel<QPT, QB>  u8 batches with the shapes the
 //                             batch autotuner chooses from.
 #include <climits>
@@ -221,6 +221,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                                           int* __restrict__ err, float dscale, bool has_lo = false) {
     using Cfg = PairCfg<MODE, QPT, QB>;
     constexpr bool F16 = Cfg::F16;
+    [[maybe_unused]] const float inv_dscale = 1.0f / dscale;
     static_assert(!PACKED || MODE == kModeU8, "packed keys are integers of u8 rows");
     // K blocks actually loaded per row (split rows without lo parts: the hi blocks only).
     const int kb_load = (MODE == kModeFloat && !has_lo) ? 2 : Cfg::kKBlocks;
@@ -534,11 +535,14 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                         uint32_t va[16], vb[16];
                         const int thr0 = st.thr;
                         const int vt = -((thr0 >> 1) + (thr0 & 1));  // fold variant: -floor((thr0 + 1) / 2)
+                        // FP16 variant: thr0 in the accumulators' units (|thr0| < 2^24 or
+                        // INT_MAX, dscale a power of two: exact, INT_MAX rounds up).
+                        const float thrf = static_cast<float>(thr0) * inv_dscale;
                         auto bits = [&](const uint32_t (&v)[16], int c) -> uint32_t {
                             if constexpr (Cfg::kFold)
                                 return fold_bits16(v, vt);
                             else
-                                return bound16<kKind>(v, rec + kBN + 2 * c, thr0, dscale);
+                                return bound16<kKind>(v, rec + kBN + 2 * c, thr0, thrf);
                         };
                         uint32_t pass = 0;  // bit 2 c + k: subgroup k of chunk c may hold a candidate
                         ptx::tmem_ld16(taddr, va);

@@ -4,264 +4,318 @@
 // [0, 255], or such integers times one common power of two (the reference's
 // own benchmark divides SIFT1M's integer components by 512, src/test.cu:99-103),
 // are packed once to u8, the format the tensor-core kernel consumes.
+#include <algorithm>
+#include <climits>
 #include <cuda_fp16.h>
+#include "exact2nn.cuh"
 #include "pack.cuh"
 
 namespace sift {
 namespace {
 
-// v * mul (mul a power of two, so the product is exact) as u8; bad when it is
-// not an integer in [0, 255].
-__device__ __forceinline__ uint32_t to_u8(float v, float mul, bool& bad) {
-    v *= mul;
-    const float r = rintf(v);
-    bad |= !(v >= 0.0f && v <= 255.0f && r == v);
-    return static_cast<uint32_t>(fminf(fmaxf(r, 0.0f), 255.0f));
+// v * mul (mul a power of two, so the product is exact) as u8, clamped.
+__device__ __forceinline__ uint32_t to_u8(float v, float mul) {
+    return static_cast<uint32_t>(fminf(fmaxf(rintf(v * mul), 0.0f), 255.0f));
+}
+__device__ __forceinline__ bool is_u8(float v) { return v >= 0.0f && v <= 255.0f && rintf(v) == v; }
+
+__device__ __forceinline__ uint32_t pack4(float4 v, float mul) {
+    return to_u8(v.x, mul) | (to_u8(v.y, mul) << 8) | (to_u8(v.z, mul) << 16) | (to_u8(v.w, mul) << 24);
+}
+__device__ __forceinline__ uint2 pack8(const uint4& v, float mul) {
+    const __half2* h = reinterpret_cast<const __half2*>(&v);
+    const float2 a = __half22float2(h[0]), b = __half22float2(h[1]), c = __half22float2(h[2]), d = __half22float2(h[3]);
+    return make_uint2(pack4(make_float4(a.x, a.y, b.x, b.y), mul), pack4(make_float4(c.x, c.y, d.x, d.y), mul));
 }
 
-// n4: number of 4-element groups (n_elems / 4; n_elems is a multiple of 128).
-__global__ void pack_f32_u8_kernel(const float4* __restrict__ x, size_t n4, float mul, uchar4* __restrict__ out,
-                                   int* __restrict__ flag) {
-    bool bad = false;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n4;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const float4 v = x[i];
-        uchar4 o;
-        o.x = static_cast<unsigned char>(to_u8(v.x, mul, bad));
-        o.y = static_cast<unsigned char>(to_u8(v.y, mul, bad));
-        o.z = static_cast<unsigned char>(to_u8(v.z, mul, bad));
-        o.w = static_cast<unsigned char>(to_u8(v.w, mul, bad));
-        out[i] = o;
-    }
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flag, 1);
+// ---- survey of one value (value_stats in pack.cuh)
+__device__ __forceinline__ void survey_one(float v, uint32_t& flags, uint32_t& bits, float& mx) {
+    const float a = fabsf(v), t = v * 16777216.0f;
+    if (!(a <= 3.0e38f)) flags |= kValueNotFinite;
+    mx = fmaxf(mx, a);
+    // v in [0, 256): t < 2^32, exact; an integer t fits a uint32.
+    const uint32_t u = __float2uint_rz(t);
+    if (!(v >= 0.0f && v < 256.0f && __uint2float_rn(u) == t)) flags |= kValueNotFixed;
+    bits |= u;
+    if (!is_u8(v)) flags |= kValueNotU8;
 }
-
-// n8: number of 8-element groups.
-__global__ void pack_f16_u8_kernel(const uint4* __restrict__ x, size_t n8, float mul, uint2* __restrict__ out,
-                                   int* __restrict__ flag) {
-    bool bad = false;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n8;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const uint4 v = x[i];
-        const __half2* h = reinterpret_cast<const __half2*>(&v);
-        uint32_t b[8];
-        #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float2 f = __half22float2(h[k]);
-            b[2 * k] = to_u8(f.x, mul, bad);
-            b[2 * k + 1] = to_u8(f.y, mul, bad);
-        }
-        out[i] = make_uint2(b[0] | (b[1] << 8) | (b[2] << 16) | (b[3] << 24),
-                            b[4] | (b[5] << 8) | (b[6] << 16) | (b[7] << 24));
-    }
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flag, 1);
+// Two halves at once: every finite half is a multiple of 2^-24, and the largest
+// magnitude tells infinities and NaN.
+__device__ __forceinline__ void survey_half(uint32_t h, uint32_t& flags, uint32_t& bits) {
+    if (h == 0x8000u) h = 0;  // -0
+    const uint32_t e = h >> 10;
+    if (e > 22u) flags |= kValueNotFixed;  // negative, or 256 and above
+    bits |= ((h & 0x3ffu) | (e ? 0x400u : 0u)) << (e > 1u ? min(e, 22u) - 1u : 0u);
 }
-
-// Smallest s >= 0 with v * 2^s an integer, for finite v >= 0 (0 for v = 0).
-__device__ __forceinline__ int int_shift(float v) {
-    const uint32_t b = __float_as_uint(v);
-    const int e = static_cast<int>((b >> 23) & 0xff);
-    uint32_t m = b & 0x7fffffu;
-    if (m == 0 && e == 0) return 0;
-    int ex = e == 0 ? -149 : e - 150;  // v = m * 2^ex
-    if (e != 0) m |= 0x800000u;
-    ex += __ffs(static_cast<int>(m)) - 1;  // strip trailing zero bits of m
-    return ex < 0 ? -ex : 0;
+__device__ __forceinline__ void survey_half2(uint32_t w, uint32_t& flags, uint32_t& bits, uint32_t& mx2) {
+    mx2 = __vmaxu2(mx2, w & 0x7fff7fffu);
+    survey_half(w & 0xffffu, flags, bits);
+    survey_half(w >> 16, flags, bits);
 }
-
-__device__ __forceinline__ void stat_one(float v, bool& bad, int& sh, float& mx) {
-    bad |= !(v >= 0.0f && v <= 3.0e38f);
-    if (v >= 0.0f && v <= 3.0e38f) {
-        sh = max(sh, int_shift(v));
-        mx = fmaxf(mx, v);
-    }
-}
-
-// stats[0] |= 1 if any value is negative or not finite; stats[1] = max over
-// values of int_shift; stats[2] = bit pattern of the largest value (the bit
-// patterns of non-negative floats order like the values).
-__device__ __forceinline__ void stats_flush(bool bad, int sh, float mx, int* stats) {
-    const unsigned full = 0xffffffffu;
-    #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sh = max(sh, __shfl_xor_sync(full, sh, o));
-        mx = fmaxf(mx, __shfl_xor_sync(full, mx, o));
-    }
-    bad = __any_sync(full, bad);
+__device__ __forceinline__ void survey_flush(uint32_t flags, uint32_t bits, float mx, int* stats) {
+    flags = __reduce_or_sync(0xffffffffu, flags);
+    bits = __reduce_or_sync(0xffffffffu, bits);
+    const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));  // mx >= 0: bits order like values
     if ((threadIdx.x & 31) == 0) {
-        if (bad) atomicOr(stats, 1);
-        atomicMax(stats + 1, sh);
-        atomicMax(stats + 2, __float_as_int(mx));
+        if (flags) atomicOr(stats, static_cast<int>(flags));
+        if (bits) atomicOr(stats + 1, static_cast<int>(bits));
+        atomicMax(stats + 2, static_cast<int>(m));
     }
 }
-
-__global__ void stats_f32_kernel(const float4* __restrict__ x, size_t n4, int* __restrict__ stats) {
-    bool bad = false;
-    int sh = 0;
-    float mx = 0.0f;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n4;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const float4 v = x[i];
-        stat_one(v.x, bad, sh, mx);
-        stat_one(v.y, bad, sh, mx);
-        stat_one(v.z, bad, sh, mx);
-        stat_one(v.w, bad, sh, mx);
-    }
-    stats_flush(bad, sh, mx, stats);
+__device__ __forceinline__ float half_max(uint32_t mx2, uint32_t& flags) {
+    const uint32_t m = max(mx2 & 0xffffu, mx2 >> 16);
+    if (m >= 0x7c00u) flags |= kValueNotFinite;
+    return m >= 0x7c00u ? 0.0f : __half2float(__ushort_as_half(static_cast<unsigned short>(m)));
 }
 
-__global__ void stats_f16_kernel(const uint4* __restrict__ x, size_t n8, int* __restrict__ stats) {
-    bool bad = false;
-    int sh = 0;
+// One pass over the query and the base rows (n_q and n_r groups of 16 bytes):
+// the survey of all values and, with out pointers, their u8 form (mul = 1),
+// final when every value is an integer in [0, 255]. Four loads in flight per
+// thread; HBM-bound (512 or 256 bytes read per row, 128 written).
+// One launch for both sets instead of separate pack, scale and range passes, and
+// one synchronisation for the caller instead of up to three: cublas_2nn_sift
+// on 1,000 x 10,000 rows of integers / 512 132 -> 82 us,
+// general float match() of 2,053 x 131,077 rows 339 -> 257 us (with the fused split).
+template <bool HALF, bool SURVEY>
+__global__ void __launch_bounds__(256)
+    convert_kernel(const uint4* __restrict__ q, size_t n_q, const uint4* __restrict__ r, size_t n_r, float mul,
+                   uint8_t* __restrict__ q_out, uint8_t* __restrict__ r_out, int* __restrict__ stats) {
+    uint32_t flags = 0, bits = 0, mx2 = 0;
     float mx = 0.0f;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n8;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const uint4 v = x[i];
-        const __half2* h = reinterpret_cast<const __half2*>(&v);
+    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x, n = n_q + n_r;
+    for (size_t i0 = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i0 < n; i0 += 4 * stride) {
+        uint4 v[4];
         #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const float2 f = __half22float2(h[k]);
-            stat_one(f.x, bad, sh, mx);
-            stat_one(f.y, bad, sh, mx);
+            const size_t i = i0 + k * stride;
+            v[k] = i < n ? (i < n_q ? q[i] : r[i - n_q]) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        #pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const size_t i = i0 + k * stride;
+            if (i >= n) break;
+            const bool in_q = i < n_q;
+            const size_t at = in_q ? i : i - n_q;
+            uint8_t* out = in_q ? q_out : r_out;
+            if constexpr (HALF) {
+                if constexpr (SURVEY) {
+                    survey_half2(v[k].x, flags, bits, mx2);
+                    survey_half2(v[k].y, flags, bits, mx2);
+                    survey_half2(v[k].z, flags, bits, mx2);
+                    survey_half2(v[k].w, flags, bits, mx2);
+                }
+                if (out) reinterpret_cast<uint2*>(out)[at] = pack8(v[k], mul);
+            } else {
+                const float4 f = *reinterpret_cast<const float4*>(&v[k]);
+                if constexpr (SURVEY) {
+                    survey_one(f.x, flags, bits, mx);
+                    survey_one(f.y, flags, bits, mx);
+                    survey_one(f.z, flags, bits, mx);
+                    survey_one(f.w, flags, bits, mx);
+                }
+                if (out) reinterpret_cast<uint32_t*>(out)[at] = pack4(f, mul);
+            }
         }
     }
-    stats_flush(bad, sh, mx, stats);
+    if constexpr (SURVEY) {
+        if constexpr (HALF) {
+            mx = half_max(mx2, flags);
+            // An integer multiple of 1 up to 255: no bit below 2^24 and in range.
+            if ((bits & 0xffffffu) || (flags & kValueNotFixed)) flags |= kValueNotU8;
+        }
+        survey_flush(flags, bits, mx, stats);
+    }
 }
 
-// General (non-integer) descriptors: stats[0] |= 1 if a value is not finite,
-// stats[1] = bit pattern of the largest |value|.
-__device__ __forceinline__ void abs_one(float v, bool& bad, float& mx) {
-    const float a = fabsf(v);
-    bad |= !(a <= 3.0e38f);
-    if (a <= 3.0e38f) mx = fmaxf(mx, a);
+template <bool SURVEY>
+cudaError_t launch_convert(const void* q, size_t q_rows, const void* r, size_t r_rows, bool half, float mul,
+                           uint8_t* q_out, uint8_t* r_out, int* stats, int num_sms, cudaStream_t stream) {
+    const size_t per_row = half ? 16 : 32, n_q = q_rows * per_row, n_r = r_rows * per_row;
+    if (n_q + n_r == 0) return cudaSuccess;
+    const size_t blocks = std::min<size_t>((n_q + n_r + 1023) / 1024, static_cast<size_t>(num_sms) * 8);
+    const auto* qp = static_cast<const uint4*>(q);
+    const auto* rp = static_cast<const uint4*>(r);
+    if (half)
+        convert_kernel<true, SURVEY><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(qp, n_q, rp, n_r, mul, q_out,
+                                                                                       r_out, stats);
+    else
+        convert_kernel<false, SURVEY><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(qp, n_q, rp, n_r, mul, q_out,
+                                                                                        r_out, stats);
+    return cudaGetLastError();
 }
 
-__device__ __forceinline__ void abs_flush(bool bad, float mx, int* stats) {
+// ---- FP16 rows: survey, norms and records in one pass
+// One block per 128 rows (8 threads per row, four 32-byte loads in flight per
+// thread): the survey of its values and the rows' squared norms, FP32 sums of
+// the squares as they are. For integers times 2^-s every partial sum is an
+// integer below 2^23 times 2^-2s, exact at any scale, so the norms need not
+// wait for s. Blocks [0, base_tiles) write records (norms, 8-row minima), the
+// others query norms and clear the shared bounds. HBM-bound: 256 bytes per row.
+// FP16 2,561 x 500,003: survey 77 + norms 25 us in two passes before, the whole
+// call 407 -> 356 us.
+__global__ void __launch_bounds__(256)
+    survey_norms_f16_kernel(const __half* __restrict__ r, int r_n, int base_tiles, int metric, int32_t* __restrict__ rec,
+                            const __half* __restrict__ q, int q_n, int q_pad, int32_t* __restrict__ qnorm,
+                            int32_t* __restrict__ thresh, int* __restrict__ stats) {
+    const int sub = threadIdx.x & 7, lrow = threadIdx.x >> 3;
+    const bool is_base = static_cast<int>(blockIdx.x) < base_tiles;
+    const __half* x = is_base ? r : q;
+    const int n = is_base ? r_n : q_n;
+    const int row0 = (static_cast<int>(blockIdx.x) - (is_base ? 0 : base_tiles)) * kBN;
+    uint4 v[4][2];
     #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    bad = __any_sync(0xffffffffu, bad);
-    if ((threadIdx.x & 31) == 0) {
-        if (bad) atomicOr(stats, 1);
-        atomicMax(stats + 1, __float_as_int(mx));
+    for (int part = 0; part < 4; ++part) {
+        const int row = row0 + part * 32 + lrow;
+        const uint4* p = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * kDim) + 2 * sub;
+        v[part][0] = row < n ? p[0] : make_uint4(0u, 0u, 0u, 0u);
+        v[part][1] = row < n ? p[1] : make_uint4(0u, 0u, 0u, 0u);
     }
-}
-
-__global__ void abs_stats_f32_kernel(const float4* __restrict__ x, size_t n4, int* __restrict__ stats) {
-    bool bad = false;
-    float mx = 0.0f;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n4;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const float4 v = x[i];
-        abs_one(v.x, bad, mx);
-        abs_one(v.y, bad, mx);
-        abs_one(v.z, bad, mx);
-        abs_one(v.w, bad, mx);
-    }
-    abs_flush(bad, mx, stats);
-}
-
-__global__ void abs_stats_f16_kernel(const uint4* __restrict__ x, size_t n8, int* __restrict__ stats) {
-    bool bad = false;
-    float mx = 0.0f;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n8;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const uint4 v = x[i];
-        const __half2* h = reinterpret_cast<const __half2*>(&v);
+    __shared__ float nrm[kBN];
+    uint32_t flags = 0, bits = 0, mx2 = 0;
+    #pragma unroll
+    for (int part = 0; part < 4; ++part) {
+        float s = 0.0f;
         #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float2 f = __half22float2(h[k]);
-            abs_one(f.x, bad, mx);
-            abs_one(f.y, bad, mx);
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t w[4] = {v[part][h].x, v[part][h].y, v[part][h].z, v[part][h].w};
+            #pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                survey_half2(w[k], flags, bits, mx2);
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+                s = fmaf(f.x, f.x, s);
+                s = fmaf(f.y, f.y, s);
+            }
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 4);
+        const int col = part * 32 + lrow, row = row0 + col;
+        if (sub != 0) continue;
+        if (is_base) {
+            nrm[col] = row < n ? (metric == kMetricL2 ? s : 0.0f) : kFloatKeyPad;
+        } else if (row < q_pad) {
+            qnorm[row] = __float_as_int(s);
+            thresh[row] = thresh[q_pad + row] = INT_MAX;
         }
     }
-    abs_flush(bad, mx, stats);
-}
-
-// Float rows -> split FP16 rows [n][256]: halves [0, 128) hold hi = fp16(x * mul)
-// and [128, 256) lo = fp16(x * mul - hi), so hi + lo carries 22 significant
-// bits of x * mul (mul a power of two: exact). Each thread converts 4
-// consecutive elements of one row.
-__global__ void pack_split_f16_kernel(const float4* __restrict__ x, size_t n4, float mul, __half* __restrict__ out) {
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n4;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const float4 v = x[i];
-        const size_t row = i >> 5, col = (i & 31) * 4;
-        const float s[4] = {v.x * mul, v.y * mul, v.z * mul, v.w * mul};
-        __half hi[4], lo[4];
-        #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            hi[k] = __float2half_rn(s[k]);
-            lo[k] = __float2half_rn(s[k] - __half2float(hi[k]));
+    __syncthreads();
+    if (is_base) {
+        int32_t* o = rec + static_cast<size_t>(blockIdx.x) * kRecInts;
+        if (threadIdx.x < kBN) o[threadIdx.x] = __float_as_int(nrm[threadIdx.x]);
+        if (threadIdx.x < 16) {
+            float m = nrm[8 * threadIdx.x];
+            #pragma unroll
+            for (int i = 1; i < 8; ++i) m = fminf(m, nrm[8 * threadIdx.x + i]);
+            o[kBN + threadIdx.x] = __float_as_int(m);
         }
-        __half* o = out + row * 256 + col;
-        *reinterpret_cast<uint2*>(o) = *reinterpret_cast<const uint2*>(hi);
-        *reinterpret_cast<uint2*>(o + 128) = *reinterpret_cast<const uint2*>(lo);
     }
+    const float mx = half_max(mx2, flags);
+    survey_flush(flags, bits, mx, stats);
 }
 
-unsigned grid_for(size_t items, int num_sms) {
-    size_t blocks = (items + 255) / 256;
-    const size_t cap = static_cast<size_t>(num_sms) * 8;
-    if (blocks > cap) blocks = cap;
-    return static_cast<unsigned>(blocks);
+// ---- general float rows: split and norms in one pass
+// Float rows times mul -> split FP16 rows [n][256], halves [0, 128) holding
+// hi = fp16(x * mul) and [128, 256) lo = fp16(x * mul - hi), so hi + lo carries
+// 22 significant bits of x * mul (mul a power of two: exact); and the squared
+// norms of x * mul (FP32, 16 elements in order per thread, then the 8 threads of
+// a row), as row_norms_float_kernel lays them out: base records, then query
+// norms and cleared bounds. One block per 32 rows; HBM-bound, 512 bytes read and
+// 512 written per row instead of 512 read twice.
+__global__ void __launch_bounds__(256)
+    split_norms_f32_kernel(const float* __restrict__ r, int r_n, int r_pad, int metric, __half* __restrict__ r_out,
+                           int32_t* __restrict__ rec, const float* __restrict__ q, int q_n, int q_pad,
+                           __half* __restrict__ q_out, int32_t* __restrict__ qnorm, int32_t* __restrict__ thresh,
+                           float mul) {
+    const int base_blocks = r_pad / 32;
+    const bool is_base = static_cast<int>(blockIdx.x) < base_blocks;
+    const int b = static_cast<int>(blockIdx.x) - (is_base ? 0 : base_blocks);
+    const int lrow = threadIdx.x >> 3, sub = threadIdx.x & 7, row = b * 32 + lrow;
+    const int n = is_base ? r_n : q_n;
+    float s = 0.0f;
+    if (row < n) {
+        const float4* p = reinterpret_cast<const float4*>((is_base ? r : q) + static_cast<size_t>(row) * kDim) + 4 * sub;
+        float f[16];
+        #pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const float4 v = p[h];
+            f[4 * h] = v.x * mul;
+            f[4 * h + 1] = v.y * mul;
+            f[4 * h + 2] = v.z * mul;
+            f[4 * h + 3] = v.w * mul;
+        }
+        __half hi[16], lo[16];
+        #pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            s = fmaf(f[i], f[i], s);
+            hi[i] = __float2half_rn(f[i]);
+            lo[i] = __float2half_rn(f[i] - __half2float(hi[i]));
+        }
+        uint4* o = reinterpret_cast<uint4*>((is_base ? r_out : q_out) + static_cast<size_t>(row) * 256 + 16 * sub);
+        o[0] = reinterpret_cast<const uint4*>(hi)[0];
+        o[1] = reinterpret_cast<const uint4*>(hi)[1];
+        o[16] = reinterpret_cast<const uint4*>(lo)[0];
+        o[17] = reinterpret_cast<const uint4*>(lo)[1];
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    __shared__ float nrm[32];
+    if (is_base) {
+        const float v = row < n ? (metric == kMetricL2 ? s : 0.0f) : kFloatKeyPad;
+        int32_t* o = rec + static_cast<size_t>(b / 4) * kRecInts;
+        const int part = b & 3;
+        if (sub == 0) {
+            nrm[lrow] = v;
+            o[part * 32 + lrow] = __float_as_int(v);
+        }
+        __syncthreads();
+        if (threadIdx.x < 4) {
+            float m = nrm[8 * threadIdx.x];
+            #pragma unroll
+            for (int i = 1; i < 8; ++i) m = fminf(m, nrm[8 * threadIdx.x + i]);
+            o[kBN + part * 4 + threadIdx.x] = __float_as_int(m);
+        }
+    } else if (sub == 0 && row < q_pad) {
+        qnorm[row] = __float_as_int(row < n ? s : kFloatKeyPad);
+        thresh[row] = thresh[q_pad + row] = INT_MAX;
+    }
 }
 
 }  // namespace
 
-cudaError_t launch_value_stats(const void* x, bool half, size_t n_rows, int* stats, int num_sms, cudaStream_t stream) {
-    if (n_rows == 0) return cudaSuccess;
-    if (half) {
-        const size_t n8 = n_rows * 16;
-        stats_f16_kernel<<<grid_for(n8, num_sms), 256, 0, stream>>>(reinterpret_cast<const uint4*>(x), n8, stats);
-    } else {
-        const size_t n4 = n_rows * 32;
-        stats_f32_kernel<<<grid_for(n4, num_sms), 256, 0, stream>>>(reinterpret_cast<const float4*>(x), n4, stats);
-    }
+int value_shift(uint32_t bits) {
+    int low = 0;
+    while (low < 24 && !((bits >> low) & 1u)) ++low;
+    return bits ? 24 - low : 0;
+}
+
+cudaError_t launch_survey(const void* q, size_t q_rows, const void* r, size_t r_rows, bool half, uint8_t* q_out,
+                          uint8_t* r_out, int* stats, int num_sms, cudaStream_t stream) {
+    return launch_convert<true>(q, q_rows, r, r_rows, half, 1.0f, q_out, r_out, stats, num_sms, stream);
+}
+
+cudaError_t launch_pack_u8(const void* q, size_t q_rows, const void* r, size_t r_rows, bool half, float mul,
+                           uint8_t* q_out, uint8_t* r_out, int num_sms, cudaStream_t stream) {
+    return launch_convert<false>(q, q_rows, r, r_rows, half, mul, q_out, r_out, nullptr, num_sms, stream);
+}
+
+cudaError_t launch_survey_norms_f16(const void* r, int r_n, int base_tiles, int metric, int32_t* rec, const void* q,
+                                    int q_n, int q_pad, int32_t* qnorm, int32_t* thresh, int* stats,
+                                    cudaStream_t stream) {
+    const int blocks = base_tiles + q_pad / kBN;
+    if (blocks <= 0) return cudaSuccess;
+    survey_norms_f16_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __half*>(r), r_n, base_tiles, metric, rec,
+                                                        static_cast<const __half*>(q), q_n, q_pad, qnorm, thresh, stats);
     return cudaGetLastError();
 }
 
-cudaError_t launch_abs_stats(const void* x, bool half, size_t n_rows, int* stats, int num_sms, cudaStream_t stream) {
-    if (n_rows == 0) return cudaSuccess;
-    if (half) {
-        const size_t n8 = n_rows * 16;
-        abs_stats_f16_kernel<<<grid_for(n8, num_sms), 256, 0, stream>>>(reinterpret_cast<const uint4*>(x), n8, stats);
-    } else {
-        const size_t n4 = n_rows * 32;
-        abs_stats_f32_kernel<<<grid_for(n4, num_sms), 256, 0, stream>>>(reinterpret_cast<const float4*>(x), n4, stats);
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pack_split_f16(const float* x, size_t n_rows, float mul, void* out, int num_sms,
-                                  cudaStream_t stream) {
-    const size_t n4 = n_rows * 32;
-    if (n4 == 0) return cudaSuccess;
-    pack_split_f16_kernel<<<grid_for(n4, num_sms), 256, 0, stream>>>(reinterpret_cast<const float4*>(x), n4, mul,
-                                                                     static_cast<__half*>(out));
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pack_f32_u8(const float* x, size_t n_rows, float mul, uint8_t* out, int* flag, int num_sms,
-                               cudaStream_t stream) {
-    const size_t n4 = n_rows * 32;
-    if (n4 == 0) return cudaSuccess;
-    size_t blocks = (n4 + 255) / 256;
-    const size_t cap = static_cast<size_t>(num_sms) * 8;
-    if (blocks > cap) blocks = cap;
-    pack_f32_u8_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(reinterpret_cast<const float4*>(x), n4,
-                                                                         mul, reinterpret_cast<uchar4*>(out), flag);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pack_f16_u8(const void* x, size_t n_rows, float mul, uint8_t* out, int* flag, int num_sms,
-                               cudaStream_t stream) {
-    const size_t n8 = n_rows * 16;
-    if (n8 == 0) return cudaSuccess;
-    size_t blocks = (n8 + 255) / 256;
-    const size_t cap = static_cast<size_t>(num_sms) * 8;
-    if (blocks > cap) blocks = cap;
-    pack_f16_u8_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(reinterpret_cast<const uint4*>(x), n8,
-                                                                         mul, reinterpret_cast<uint2*>(out), flag);
+cudaError_t launch_split_norms_f32(const float* r, int r_n, int r_pad, int metric, void* r_out, int32_t* rec,
+                                   const float* q, int q_n, int q_pad, void* q_out, int32_t* qnorm, int32_t* thresh,
+                                   float mul, cudaStream_t stream) {
+    const int blocks = r_pad / 32 + q_pad / 32;
+    if (blocks <= 0) return cudaSuccess;
+    split_norms_f32_kernel<<<blocks, 256, 0, stream>>>(r, r_n, r_pad, metric, static_cast<__half*>(r_out), rec, q, q_n,
+                                                       q_pad, static_cast<__half*>(q_out), qnorm, thresh, mul);
     return cudaGetLastError();
 }
 
