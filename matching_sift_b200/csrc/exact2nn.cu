@@ -263,8 +263,8 @@ __device__ __forceinline__ int find_item(int n_items, long long v, F key) {
 // n_b get 0). The blocks after them: query norms and cleared bounds. HBM-bound:
 // 128 bytes read per row, 4-8 written.
 __global__ void __launch_bounds__(256)
-    batch_prep_kernel(const uint8_t* __restrict__ base, const WorkItem* __restrict__ items, int n_items, int tiles,
-                      int32_t* __restrict__ rec, const uint8_t* __restrict__ q, int q_n, int q_pad,
+    batch_prep_kernel(const uint8_t* __restrict__ base, const WorkItem* __restrict__ items, int n_items,
+                      const WorkItem single, int tiles, int32_t* __restrict__ rec, const uint8_t* __restrict__ q, int q_n, int q_pad,
                       int32_t* __restrict__ qnorm, int32_t* __restrict__ thresh) {
     const int sub = threadIdx.x & 7, lrow = threadIdx.x >> 3;
     const bool is_base = static_cast<int>(blockIdx.x) < tiles;
@@ -273,8 +273,8 @@ __global__ void __launch_bounds__(256)
     if (is_base) {
         const int T = blockIdx.x;
         // 32 probes per step instead of one: the largest p with rec_off <= T.
-        int lo = 0, hi = n_items;  // rec_off[lo] <= T < rec_off[hi]
-        while (hi - lo > 1) {
+        int lo = 0, hi = n_items;  // rec_off[lo] <= T < rec_off[hi]; no list: the single problem
+        while (items && hi - lo > 1) {
             const int step = (hi - lo + 31) / 32;
             const int at = lo + (threadIdx.x & 31) * step;
             const bool le = at < hi && items[at].rec_off <= T;
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(256)
             hi = min(hi, lo + (k + 1) * step);
             lo += k * step;
         }
-        const WorkItem& it = items[lo];
+        const WorkItem it = items ? items[lo] : single;
         x = base + static_cast<size_t>(it.b_off) * kDim;
         first = (T - it.rec_off) * kBN;
         n = it.n_b;
@@ -874,7 +874,9 @@ cudaError_t launch_batch_prep(const uint8_t* base, const uint8_t* q, int q_n, co
                               int32_t* qnorm, int32_t* thresh, cudaStream_t stream) {
     const int blocks = bp.total_tiles + bp.plan.q_tiles;
     if (blocks <= 0) return cudaSuccess;
-    batch_prep_kernel<<<blocks, 256, 0, stream>>>(base, bp.items, bp.n_items, bp.total_tiles, rec, q, q_n,
+    WorkItem single{};
+    single.n_b = bp.plan.r_n;
+    batch_prep_kernel<<<blocks, 256, 0, stream>>>(base, bp.items, bp.n_items, single, bp.total_tiles, rec, q, q_n,
                                                   bp.plan.q_pad, qnorm, thresh);
     return cudaGetLastError();
 }

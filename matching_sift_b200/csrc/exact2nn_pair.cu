@@ -690,10 +690,9 @@ template <int QPT, int QB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<kModeU8, QPT, QB>::kThreads, 1)
     exact2nn_u8_pair_batch_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap bmap,
                                   const int32_t* __restrict__ brec, const ExactPlan plan,
-                                  const WorkItem* __restrict__ items, int n_items, int4* __restrict__ partial,
-                                  int32_t* __restrict__ thresh, int* __restrict__ err) {
-    pair_body<kModeU8, QPT, QB, true>(qmap, bmap, qmap, brec, plan, items, n_items, WorkItem{}, partial, thresh, err,
-                                       1.0f);
+                                  const WorkItem* __restrict__ items, int n_items, const WorkItem single,
+                                  int4* __restrict__ partial, int32_t* __restrict__ thresh, int* __restrict__ err) {
+    pair_body<kModeU8, QPT, QB, true>(qmap, bmap, qmap, brec, plan, items, n_items, single, partial, thresh, err, 1.0f);
 }
 
 template <typename K>
@@ -731,7 +730,7 @@ cudaError_t launch_batch_variant(const CUtensorMap& qmap, const CUtensorMap& bma
     if (e != cudaSuccess) return e;
     if (bp.plan.grid <= 0) return cudaSuccess;
     exact2nn_u8_pair_batch_kernel<QPT, QB><<<2 * bp.plan.grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(
-        qmap, bmap, brec, bp.plan, bp.items, bp.n_items, partial, thresh, err);
+        qmap, bmap, brec, bp.plan, bp.items, bp.n_items, single_item(bp.plan), partial, thresh, err);
     return cudaGetLastError();
 }
 
