@@ -13,23 +13,16 @@
 namespace sift {
 namespace {
 
-// v * mul (mul a power of two, so the product is exact) as u8, clamped.
-__device__ __forceinline__ uint32_t to_u8(float v, float mul) {
-    return static_cast<uint32_t>(fminf(fmaxf(rintf(v * mul), 0.0f), 255.0f));
-}
-__device__ __forceinline__ bool is_u8(float v) { return v >= 0.0f && v <= 255.0f && rintf(v) == v; }
-
+// v * mul (mul a power of two; the product is an integer in [0, 255]) as u8.
+__device__ __forceinline__ uint32_t to_u8(float v, float mul) { return __float2uint_rz(v * mul) & 0xffu; }
 __device__ __forceinline__ uint32_t pack4(float4 v, float mul) {
     return to_u8(v.x, mul) | (to_u8(v.y, mul) << 8) | (to_u8(v.z, mul) << 16) | (to_u8(v.w, mul) << 24);
 }
-__device__ __forceinline__ uint2 pack8(const uint4& v, float mul) {
-    const __half2* h = reinterpret_cast<const __half2*>(&v);
-    const float2 a = __half22float2(h[0]), b = __half22float2(h[1]), c = __half22float2(h[2]), d = __half22float2(h[3]);
-    return make_uint2(pack4(make_float4(a.x, a.y, b.x, b.y), mul), pack4(make_float4(c.x, c.y, d.x, d.y), mul));
-}
 
-// ---- survey of one value (value_stats in pack.cuh)
-__device__ __forceinline__ void survey_one(float v, uint32_t& flags, uint32_t& bits, float& mx) {
+// ---- survey of one value (launch_survey in pack.cuh)
+// Returns v * 2^24 as an unsigned integer (exact unless kValueNotFixed), whose
+// top byte is v itself when v is an integer in [0, 255].
+__device__ __forceinline__ uint32_t survey_one(float v, uint32_t& flags, uint32_t& bits, float& mx) {
     const float a = fabsf(v), t = v * 16777216.0f;
     if (!(a <= 3.0e38f)) flags |= kValueNotFinite;
     mx = fmaxf(mx, a);
@@ -37,35 +30,54 @@ __device__ __forceinline__ void survey_one(float v, uint32_t& flags, uint32_t& b
     const uint32_t u = __float2uint_rz(t);
     if (!(v >= 0.0f && v < 256.0f && __uint2float_rn(u) == t)) flags |= kValueNotFixed;
     bits |= u;
-    if (!is_u8(v)) flags |= kValueNotU8;
+    return u;
 }
-// Two halves at once: every finite half is a multiple of 2^-24, and the largest
-// magnitude tells infinities and NaN.
-__device__ __forceinline__ void survey_half(uint32_t h, uint32_t& flags, uint32_t& bits) {
-    if (h == 0x8000u) h = 0;  // -0
-    const uint32_t e = h >> 10;
-    if (e > 22u) flags |= kValueNotFixed;  // negative, or 256 and above
-    bits |= ((h & 0x3ffu) | (e ? 0x400u : 0u)) << (e > 1u ? min(e, 22u) - 1u : 0u);
-}
-__device__ __forceinline__ void survey_half2(uint32_t w, uint32_t& flags, uint32_t& bits, uint32_t& mx2) {
+// Two halves at once (w, as floats f): every finite half is a multiple of 2^-24,
+// so f * 2^24 is an integer, below 2^32 for values in [0, 256); range, sign and
+// finiteness follow from the largest magnitude and the OR of all words (a set
+// sign bit is looked at again: it may be a negative zero).
+__device__ __forceinline__ void survey_half2(uint32_t w, float2 f, uint32_t& bits, uint32_t& mx2, uint32_t& words) {
     mx2 = __vmaxu2(mx2, w & 0x7fff7fffu);
-    survey_half(w & 0xffffu, flags, bits);
-    survey_half(w >> 16, flags, bits);
+    words |= w;
+    bits |= __float2uint_rz(f.x * 16777216.0f) | __float2uint_rz(f.y * 16777216.0f);
 }
-__device__ __forceinline__ void survey_flush(uint32_t flags, uint32_t bits, float mx, int* stats) {
-    flags = __reduce_or_sync(0xffffffffu, flags);
-    bits = __reduce_or_sync(0xffffffffu, bits);
-    const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));  // mx >= 0: bits order like values
-    if ((threadIdx.x & 31) == 0) {
-        if (flags) atomicOr(stats, static_cast<int>(flags));
-        if (bits) atomicOr(stats + 1, static_cast<int>(bits));
-        atomicMax(stats + 2, static_cast<int>(m));
-    }
+__device__ __forceinline__ bool negative_half2(uint32_t w) {
+    return ((w & 0x8000u) && (w & 0x7fffu)) || ((w >> 31) && (w & 0x7fff0000u));
 }
+__device__ __forceinline__ float2 half2_floats(uint32_t w) {
+    return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+// The largest magnitude as a float, and the flags it decides.
 __device__ __forceinline__ float half_max(uint32_t mx2, uint32_t& flags) {
     const uint32_t m = max(mx2 & 0xffffu, mx2 >> 16);
+    if (m >= 0x5c00u) flags |= kValueNotFixed;  // 256 and above
     if (m >= 0x7c00u) flags |= kValueNotFinite;
     return m >= 0x7c00u ? 0.0f : __half2float(__ushort_as_half(static_cast<unsigned short>(m)));
+}
+// A block's findings (256 threads). They all meet at three addresses: reduced
+// within the block first, and added only where they change what is there (the
+// words only grow, so a stale read costs one atomic).
+__device__ __forceinline__ void survey_flush(uint32_t flags, uint32_t bits, float mx, int* stats) {
+    __shared__ uint32_t s_part[3][8];
+    flags = __reduce_or_sync(0xffffffffu, flags);
+    bits = __reduce_or_sync(0xffffffffu, bits);
+    uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));  // mx >= 0: bits order like values
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+        s_part[0][warp] = flags;
+        s_part[1][warp] = bits;
+        s_part[2][warp] = m;
+    }
+    __syncthreads();
+    if (warp > 0) return;
+    flags = __reduce_or_sync(0xffffffffu, lane < 8 ? s_part[0][lane] : 0u);
+    bits = __reduce_or_sync(0xffffffffu, lane < 8 ? s_part[1][lane] : 0u);
+    m = __reduce_max_sync(0xffffffffu, lane < 8 ? s_part[2][lane] : 0u);
+    if (lane == 0) {
+        if (flags & ~static_cast<uint32_t>(__ldcg(stats))) atomicOr(stats, static_cast<int>(flags));
+        if (bits & ~static_cast<uint32_t>(__ldcg(stats + 1))) atomicOr(stats + 1, static_cast<int>(bits));
+        if (m > static_cast<uint32_t>(__ldcg(stats + 2))) atomicMax(stats + 2, static_cast<int>(m));
+    }
 }
 
 // One pass over the query and the base rows (n_q and n_r groups of 16 bytes):
@@ -80,7 +92,7 @@ template <bool HALF, bool SURVEY>
 __global__ void __launch_bounds__(256)
     convert_kernel(const uint4* __restrict__ q, size_t n_q, const uint4* __restrict__ r, size_t n_r, float mul,
                    uint8_t* __restrict__ q_out, uint8_t* __restrict__ r_out, int* __restrict__ stats) {
-    uint32_t flags = 0, bits = 0, mx2 = 0;
+    uint32_t flags = 0, bits = 0, mx2 = 0, words = 0;
     float mx = 0.0f;
     const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x, n = n_q + n_r;
     for (size_t i0 = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i0 < n; i0 += 4 * stride) {
@@ -99,30 +111,39 @@ __global__ void __launch_bounds__(256)
             uint8_t* out = in_q ? q_out : r_out;
             if constexpr (HALF) {
                 if constexpr (SURVEY) {
-                    survey_half2(v[k].x, flags, bits, mx2);
-                    survey_half2(v[k].y, flags, bits, mx2);
-                    survey_half2(v[k].z, flags, bits, mx2);
-                    survey_half2(v[k].w, flags, bits, mx2);
+                    const uint32_t w[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
+                    words = 0;
+                    #pragma unroll
+                    for (int e = 0; e < 4; ++e) survey_half2(w[e], half2_floats(w[e]), bits, mx2, words);
+                    if ((words & 0x80008000u) &&
+                        (negative_half2(w[0]) || negative_half2(w[1]) || negative_half2(w[2]) || negative_half2(w[3])))
+                        flags |= kValueNotFixed;
                 }
-                if (out) reinterpret_cast<uint2*>(out)[at] = pack8(v[k], mul);
+                if (out) {
+                    const float2 a = half2_floats(v[k].x), b = half2_floats(v[k].y), c = half2_floats(v[k].z),
+                                 d = half2_floats(v[k].w);
+                    reinterpret_cast<uint2*>(out)[at] = make_uint2(pack4(make_float4(a.x, a.y, b.x, b.y), mul),
+                                                                   pack4(make_float4(c.x, c.y, d.x, d.y), mul));
+                }
             } else {
                 const float4 f = *reinterpret_cast<const float4*>(&v[k]);
+                uint32_t packed;
                 if constexpr (SURVEY) {
-                    survey_one(f.x, flags, bits, mx);
-                    survey_one(f.y, flags, bits, mx);
-                    survey_one(f.z, flags, bits, mx);
-                    survey_one(f.w, flags, bits, mx);
+                    packed = survey_one(f.x, flags, bits, mx) >> 24;
+                    packed |= (survey_one(f.y, flags, bits, mx) >> 24) << 8;
+                    packed |= (survey_one(f.z, flags, bits, mx) >> 24) << 16;
+                    packed |= (survey_one(f.w, flags, bits, mx) >> 24) << 24;
+                } else {
+                    packed = pack4(f, mul);
                 }
-                if (out) reinterpret_cast<uint32_t*>(out)[at] = pack4(f, mul);
+                if (out) reinterpret_cast<uint32_t*>(out)[at] = packed;
             }
         }
     }
     if constexpr (SURVEY) {
-        if constexpr (HALF) {
-            mx = half_max(mx2, flags);
-            // An integer multiple of 1 up to 255: no bit below 2^24 and in range.
-            if ((bits & 0xffffffu) || (flags & kValueNotFixed)) flags |= kValueNotU8;
-        }
+        if constexpr (HALF) mx = half_max(mx2, flags);
+        // Integers in [0, 255]: in range and no bit below 2^24.
+        if ((bits & 0xffffffu) || (flags & kValueNotFixed)) flags |= kValueNotU8;
         survey_flush(flags, bits, mx, stats);
     }
 }
@@ -151,8 +172,8 @@ cudaError_t launch_convert(const void* q, size_t q_rows, const void* r, size_t r
 // integer below 2^23 times 2^-2s, exact at any scale, so the norms need not
 // wait for s. Blocks [0, base_tiles) write records (norms, 8-row minima), the
 // others query norms and clear the shared bounds. HBM-bound: 256 bytes per row.
-// FP16 2,561 x 500,003: survey 77 + norms 25 us in two passes before, the whole
-// call 407 -> 356 us.
+// FP16 2,561 x 500,003: survey 77 + norms 25 us in two passes before, 30 us now
+// (65 with per-element integer shifts and three atomics per warp).
 __global__ void __launch_bounds__(256)
     survey_norms_f16_kernel(const __half* __restrict__ r, int r_n, int base_tiles, int metric, int32_t* __restrict__ rec,
                             const __half* __restrict__ q, int q_n, int q_pad, int32_t* __restrict__ qnorm,
@@ -171,7 +192,7 @@ __global__ void __launch_bounds__(256)
         v[part][1] = row < n ? p[1] : make_uint4(0u, 0u, 0u, 0u);
     }
     __shared__ float nrm[kBN];
-    uint32_t flags = 0, bits = 0, mx2 = 0;
+    uint32_t flags = 0, bits = 0, mx2 = 0, words = 0;
     #pragma unroll
     for (int part = 0; part < 4; ++part) {
         float s = 0.0f;
@@ -180,8 +201,8 @@ __global__ void __launch_bounds__(256)
             const uint32_t w[4] = {v[part][h].x, v[part][h].y, v[part][h].z, v[part][h].w};
             #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                survey_half2(w[k], flags, bits, mx2);
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+                const float2 f = half2_floats(w[k]);
+                survey_half2(w[k], f, bits, mx2, words);
                 s = fmaf(f.x, f.x, s);
                 s = fmaf(f.y, f.y, s);
             }
@@ -208,6 +229,15 @@ __global__ void __launch_bounds__(256)
             for (int i = 1; i < 8; ++i) m = fminf(m, nrm[8 * threadIdx.x + i]);
             o[kBN + threadIdx.x] = __float_as_int(m);
         }
+    }
+    if (words & 0x80008000u) {
+        #pragma unroll
+        for (int part = 0; part < 4; ++part)
+            #pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (negative_half2(v[part][h].x) || negative_half2(v[part][h].y) || negative_half2(v[part][h].z) ||
+                    negative_half2(v[part][h].w))
+                    flags |= kValueNotFixed;
     }
     const float mx = half_max(mx2, flags);
     survey_flush(flags, bits, mx, stats);

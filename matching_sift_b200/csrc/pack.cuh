@@ -21,8 +21,8 @@ enum ValueFlags : uint32_t {
 int value_shift(uint32_t bits);
 
 // The survey of q_rows + r_rows rows of 128 floats or halves (16-byte aligned)
-// and, where out pointers are given, their u8 form (clamped; exact when
-// kValueNotU8 is not set).
+// and, where out pointers are given, their u8 form (meaningful when kValueNotU8
+// is not set).
 cudaError_t launch_survey(const void* q, size_t q_rows, const void* r, size_t r_rows, bool half, uint8_t* q_out,
                           uint8_t* r_out, int* stats, int num_sms, cudaStream_t stream);
 // Values times mul (a power of two; products known to be integers in [0, 255]) as u8.
