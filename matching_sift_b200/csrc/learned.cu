@@ -12,15 +12,24 @@
 // Warps: 0 = weight and input-tile TMA, TMEM allocation, MMA issue (one
 //            thread); the u8 input tiles stream through a 2-stage ring,
 //            loaded two tiles ahead;
-//        1..8 = conversion and epilogue, two warps per TMEM lane quarter:
-//            thread = tile row (TMEM lane), warp half h converts K block h of
+//        1..16 = conversion and epilogue, four warps per TMEM lane quarter:
+//            thread = tile row (TMEM lane), warp group g converts 32 columns of
 //            the input row and applies layer 1's epilogue to hidden columns
-//            [128 h, 128 h + 128); half 0 also forms the codes.
-// Per tile i (epilogue threads):
-//   convert x(i) -> x_s      [x_ready]     MMA1: TMEM[0,256) = x W1^T
-//   epi1: h = bf16(relu(acc / 64 + b1)) -> h_s   [h_ready]   MMA2: TMEM[256,288) = h W2^T
-//   convert x(i+1) (x_s is free once MMA1(i) completed) while MMA2(i) runs
-//   epi2: z = acc + b2 -> code bits (and z)
+//            [64 g, 64 g + 64); group i % 4 forms the codes of tile i.
+// Two tiles are in flight, so that the epilogue warps never wait for the tensor
+// cores; TMEM holds layer 1's accumulators of both, buffer i % 2 of 256 columns,
+// and layer 2's 32 columns reuse the first ones of their tile's buffer once they
+// are read. Per tile i (epilogue threads), while MMA1(i) has just completed:
+//   convert x(i+1) -> x_s (free: MMA1(i) is done)
+//   take layer 2's accumulators of tile i - 1
+//   [x_ready]  MMA1(i+1): TMEM[256 ((i+1) % 2)] = x W1^T
+//   epi1(i): h = bf16(relu(acc / 64 + b1)) -> h_s (free: MMA2(i-1) is done)
+//   [h_ready]  MMA2(i): TMEM[256 (i % 2)], 32 columns = h W2^T
+//   epi2(i-1): z = acc + b2 -> code bits (and z)
+// Bound by shared memory (about 340 KB of operand reads and activation writes a
+// tile, 2,650 cycles of 128 bytes, against 2,000 of MMAs) and by the chain MMA1 ->
+// convert -> MMA1 over the one x_s buffer. 1M rows, 16 bits: 154 us with 8
+// epilogue warps, MMA1 in line with them and a branch per output bit, 105 us now.
 // Every wait is bounded (2 s) and reports through `err`.
 #include <climits>
 #include <cuda_bf16.h>
@@ -31,7 +40,7 @@
 namespace sift {
 namespace {
 
-constexpr int kLEpiWarps = 8;  // two per TMEM lane quarter
+constexpr int kLEpiWarps = 16;  // four per TMEM lane quarter
 constexpr int kLThreads = 32 * (1 + kLEpiWarps);
 constexpr int kXKBlock = 128 * 128;                     // bytes of one K block of a 128-row BF16 tile
 constexpr int kW1Bytes = kMlpHidden * kMlpIn * 2;       // 64 KB
@@ -42,13 +51,13 @@ constexpr uint32_t kLTmemCols = 512;
 constexpr int kXStages = 2;                             // u8 input tile ring
 constexpr int kXTileBytes = 128 * kMlpIn;               // 16 KB
 
-struct __align__(8) MlpCtl {
+struct __align__(16) MlpCtl {
     uint64_t w_full, x_ready, h_ready, m1, m2, drain;
     uint64_t xfull[kXStages];
     uint32_t tmem_base;
     int abort_flag, no_abort;
-    float b1[kMlpHidden];
-    float b2[kMlpOutRows];
+    alignas(16) float b1[kMlpHidden];
+    alignas(16) float b2[kMlpOutRows];
 };
 
 constexpr size_t kLSmemBytes = 1024 + kW1Bytes + kW2Bytes + kXBytes + kHBytes + kXStages * kXTileBytes + sizeof(MlpCtl);
@@ -65,18 +74,24 @@ __device__ __forceinline__ uint32_t bf16x2(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// Half h of row r of a u8 tile in shared memory (TMA, 128-byte swizzle; rows
-// past the end of the input are zeros) -> BF16 K block h of x_s.
-__device__ __forceinline__ void convert_row(const uint8_t* u8_tile, int r, uint8_t* x_s, int h) {
+// Byte b of w as a float: 2^23 + byte built in the mantissa, minus 2^23 (exact).
+template <int B>
+__device__ __forceinline__ float byte_float(uint32_t w) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u + B)) - 8388608.0f;
+}
+
+// 16-byte chunks 2 g and 2 g + 1 of row r of a u8 tile in shared memory (TMA,
+// 128-byte swizzle; rows past the end of the input are zeros) -> BF16 in x_s.
+__device__ __forceinline__ void convert_row(const uint8_t* u8_tile, int r, uint8_t* x_s, int g) {
     #pragma unroll
-    for (int c = 4 * h; c < 4 * h + 4; ++c) {
+    for (int c = 2 * g; c < 2 * g + 2; ++c) {
         const uint4 v = *reinterpret_cast<const uint4*>(u8_tile + sw128_off(r, c));
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
         uint32_t o[8];
         #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            o[2 * q] = bf16x2(static_cast<float>(w[q] & 0xff), static_cast<float>((w[q] >> 8) & 0xff));
-            o[2 * q + 1] = bf16x2(static_cast<float>((w[q] >> 16) & 0xff), static_cast<float>(w[q] >> 24));
+            o[2 * q] = bf16x2(byte_float<0>(w[q]), byte_float<1>(w[q]));
+            o[2 * q + 1] = bf16x2(byte_float<2>(w[q]), byte_float<3>(w[q]));
         }
         // elements 16c .. 16c + 15: K block c / 4, chunks 2 (c % 4) and 2 (c % 4) + 1
         uint8_t* blk = x_s + (c >> 2) * kXKBlock;
@@ -153,14 +168,32 @@ __global__ void __launch_bounds__(kLThreads, 1)
             constexpr uint32_t idesc1 = ptx::idesc_make(1 /*F32*/, 1 /*BF16*/, 1 /*BF16*/, 128, kMlpHidden);
             constexpr uint32_t idesc2 = ptx::idesc_make(1 /*F32*/, 1 /*BF16*/, 1 /*BF16*/, 128, kMlpOutRows);
             const bool ok = ptx::mbar_wait(bar_w, 0, abort_flag, err, kErrWaitMmaFull);
-            for (int i = 0; i < my_tiles && ok; ++i) {
-                if (!ptx::mbar_wait(bar_x, i & 1, abort_flag, err, kErrWaitMmaFull)) break;
+            auto layer2 = [&](int i) -> bool {
+                if (!ptx::mbar_wait(bar_h, i & 1, abort_flag, err, kErrWaitMmaTmem)) return false;
+                ptx::tc_fence_after();
+                #pragma unroll
+                for (int kb = 0; kb < 4; ++kb) {
+                    #pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        ptx::mma_f16(tmem + (i & 1) * kMlpHidden, ptx::sdesc_sw128(h_a + kb * kXKBlock + kk * 32),
+                                     ptx::sdesc_sw128(w2_a + kb * (kMlpOutRows * 128) + kk * 32), idesc2,
+                                     (kb | kk) ? 1u : 0u);
+                }
+                ptx::tc_commit(bar_m2);
+                return true;
+            };
+            bool run = ok;
+            for (int i = 0; i < my_tiles && run; ++i) {
+                if (!ptx::mbar_wait(bar_x, i & 1, abort_flag, err, kErrWaitMmaFull)) {
+                    run = false;
+                    break;
+                }
                 ptx::tc_fence_after();
                 #pragma unroll
                 for (int kb = 0; kb < 2; ++kb) {
                     #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
-                        ptx::mma_f16(tmem, ptx::sdesc_sw128(x_a + kb * kXKBlock + kk * 32),
+                        ptx::mma_f16(tmem + (i & 1) * kMlpHidden, ptx::sdesc_sw128(x_a + kb * kXKBlock + kk * 32),
                                      ptx::sdesc_sw128(w1_a + kb * (kMlpHidden * 128) + kk * 32), idesc1,
                                      (kb | kk) ? 1u : 0u);
                 }
@@ -172,18 +205,9 @@ __global__ void __launch_bounds__(kLThreads, 1)
                     ptx::tma_load_2d(xr_a + st * kXTileBytes, &xmap, 0, (bx + issued * gx) * 128, bar_xf + 8 * st);
                     ++issued;
                 }
-                if (!ptx::mbar_wait(bar_h, i & 1, abort_flag, err, kErrWaitMmaTmem)) break;
-                ptx::tc_fence_after();
-                #pragma unroll
-                for (int kb = 0; kb < 4; ++kb) {
-                    #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        ptx::mma_f16(tmem + kMlpHidden, ptx::sdesc_sw128(h_a + kb * kXKBlock + kk * 32),
-                                     ptx::sdesc_sw128(w2_a + kb * (kMlpOutRows * 128) + kk * 32), idesc2,
-                                     (kb | kk) ? 1u : 0u);
-                }
-                ptx::tc_commit(bar_m2);
+                if (i > 0) run = layer2(i - 1);
             }
+            if (run) layer2(my_tiles - 1);
             if (!ok) ptx::mbar_wait(bar_w, 0, never, err, kErrWaitDrain);  // weights landed before exit
             // Input tiles in flight land before exit (the last kXStages issued).
             for (int t = (issued > kXStages ? issued - kXStages : 0); t < issued; ++t)
@@ -194,72 +218,100 @@ __global__ void __launch_bounds__(kLThreads, 1)
         __syncwarp();
     } else {
         const int quarter = warp & 3;
-        const int half = (warp - 1) >> 2;   // which K block / hidden half this warp handles
+        const int grp = (warp - 1) >> 2;    // input columns [32 grp, + 32), hidden columns [64 grp, + 64)
         const int r = quarter * 32 + lane;  // tile row = TMEM lane
         const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-        bool conv_ok = true;
-        if (my_tiles > 0) {
-            conv_ok = ptx::mbar_wait(bar_xf, 0, abort_flag, err, kErrWaitEpilogue);
-            if (conv_ok) convert_row(xr_s, r, x_s, half);
+        auto wait_all = [&](uint32_t bar, uint32_t parity) -> bool {
+            const bool w = __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag, err, kErrWaitEpilogue));
+            ptx::tc_fence_after();
+            return w;
+        };
+        auto convert = [&](int i) -> bool {
+            const int st = i % kXStages;
+            const bool w = __all_sync(0xffffffffu, ptx::mbar_wait(bar_xf + 8 * st, (i / kXStages) & 1, abort_flag, err,
+                                                                  kErrWaitEpilogue));
+            if (w) convert_row(xr_s + st * kXTileBytes, r, x_s, grp);
+            return w;
+        };
+        // Layer 2 of tile i: every warp waits for it (h_s and the TMEM buffer are
+        // reused next); group i % 4 takes the accumulators, and forms the codes
+        // once the next MMAs have been started.
+        uint32_t v2[32];
+        auto take2 = [&](int i) -> bool {
+            if (!wait_all(bar_m2, i & 1)) return false;
+            if ((i & 3) == grp) {
+                ptx::tmem_ld32(tmem + lane_base + (i & 1) * kMlpHidden, v2);
+                ptx::tmem_ld_wait(v2);
+            }
+            return true;
+        };
+        auto codes2 = [&](int i) {
+            if ((i & 3) != grp) return;
+            const int g = (bx + i * gx) * 128 + r;
+            uint32_t code = 0;
+            float z[32];
+            #pragma unroll
+            for (int j = 0; j < kMlpMaxBits; j += 4) {  // outputs past k are 0 + 0
+                const float4 b = *reinterpret_cast<const float4*>(&ctl->b2[j]);
+                z[j] = __uint_as_float(v2[j]) + b.x;
+                z[j + 1] = __uint_as_float(v2[j + 1]) + b.y;
+                z[j + 2] = __uint_as_float(v2[j + 2]) + b.z;
+                z[j + 3] = __uint_as_float(v2[j + 3]) + b.w;
+            }
+            #pragma unroll
+            for (int j = 0; j < kMlpMaxBits; ++j) code |= z[j] > 0.0f ? 1u << j : 0u;
+            if (g < n) {
+                codes[g] = code & (0xffffffffu >> (32 - k));
+                if (zout) {
+                    #pragma unroll
+                    for (int j = 0; j < kMlpMaxBits; ++j)
+                        if (j < k) zout[static_cast<size_t>(g) * k + j] = z[j];
+                }
+            }
+        };
+        bool ok = my_tiles > 0 && convert(0);
+        if (ok) {
             ptx::fence_proxy_async();
             ptx::mbar_arrive(bar_x);
         }
-        for (int i = 0; i < my_tiles && __all_sync(0xffffffffu, conv_ok); ++i) {
-            const int g0 = (bx + i * gx) * 128;
-            bool waited = ptx::mbar_wait(bar_m1, i & 1, abort_flag, err, kErrWaitEpilogue);
-            if (!__all_sync(0xffffffffu, waited)) break;
-            ptx::tc_fence_after();
-            #pragma unroll 1
-            for (int m = 4 * half; m < 4 * half + 4; ++m) {
+        for (int i = 0; i < my_tiles && ok; ++i) {
+            ok = wait_all(bar_m1, i & 1);
+            if (ok && i + 1 < my_tiles) ok = convert(i + 1);
+            if (ok && i > 0) ok = take2(i - 1);
+            if (!ok) break;
+            ptx::tc_fence_before();
+            ptx::fence_proxy_async();
+            if (i + 1 < my_tiles) ptx::mbar_arrive(bar_x);
+            const uint32_t acc = tmem + lane_base + (i & 1) * kMlpHidden + 64 * grp;
+            uint8_t* blk = h_s + grp * kXKBlock;
+            #pragma unroll
+            for (int m = 0; m < 2; ++m) {
                 uint32_t v[32];
-                ptx::tmem_ld32(tmem + lane_base + m * 32, v);
+                ptx::tmem_ld32(acc + 32 * m, v);
                 ptx::tmem_ld_wait(v);
-                uint8_t* blk = h_s + (m >> 1) * kXKBlock;
                 #pragma unroll
                 for (int c8 = 0; c8 < 4; ++c8) {
                     uint32_t o[4];
                     #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int j = m * 32 + c8 * 8 + 2 * e;
-                        const float a = fmaxf(fmaf(__uint_as_float(v[c8 * 8 + 2 * e]), kMlpInScale, ctl->b1[j]), 0.0f);
-                        const float b =
-                            fmaxf(fmaf(__uint_as_float(v[c8 * 8 + 2 * e + 1]), kMlpInScale, ctl->b1[j + 1]), 0.0f);
-                        o[e] = bf16x2(a, b);
+                    for (int e = 0; e < 2; ++e) {
+                        const float4 bj = *reinterpret_cast<const float4*>(&ctl->b1[64 * grp + 32 * m + 8 * c8 + 4 * e]);
+                        const uint32_t* a = v + 8 * c8 + 4 * e;
+                        o[2 * e] = bf16x2(fmaxf(fmaf(__uint_as_float(a[0]), kMlpInScale, bj.x), 0.0f),
+                                          fmaxf(fmaf(__uint_as_float(a[1]), kMlpInScale, bj.y), 0.0f));
+                        o[2 * e + 1] = bf16x2(fmaxf(fmaf(__uint_as_float(a[2]), kMlpInScale, bj.z), 0.0f),
+                                              fmaxf(fmaf(__uint_as_float(a[3]), kMlpInScale, bj.w), 0.0f));
                     }
-                    *reinterpret_cast<uint4*>(blk + sw128_off(r, 4 * (m & 1) + c8)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    *reinterpret_cast<uint4*>(blk + sw128_off(r, 4 * m + c8)) = make_uint4(o[0], o[1], o[2], o[3]);
                 }
             }
             ptx::tc_fence_before();
             ptx::fence_proxy_async();
             ptx::mbar_arrive(bar_h);
-            if (i + 1 < my_tiles) {
-                const int st = (i + 1) % kXStages;
-                conv_ok = ptx::mbar_wait(bar_xf + 8 * st, ((i + 1) / kXStages) & 1, abort_flag, err, kErrWaitEpilogue);
-                if (conv_ok) convert_row(xr_s + st * kXTileBytes, r, x_s, half);
-                ptx::fence_proxy_async();
-                ptx::mbar_arrive(bar_x);
-            }
-            if (half) continue;  // layer 2's 32 columns: half 0
-            waited = ptx::mbar_wait(bar_m2, i & 1, abort_flag, err, kErrWaitEpilogue);
-            if (!__all_sync(0xffffffffu, waited)) break;
-            ptx::tc_fence_after();
-            uint32_t v[32];
-            ptx::tmem_ld32(tmem + lane_base + kMlpHidden, v);
-            ptx::tmem_ld_wait(v);
+            if (i > 0) codes2(i - 1);
+        }
+        if (ok && my_tiles > 0 && take2(my_tiles - 1)) {
             ptx::tc_fence_before();
-            const int g = g0 + r;
-            if (g < n) {
-                uint32_t code = 0;
-                #pragma unroll
-                for (int j = 0; j < kMlpMaxBits; ++j) {
-                    if (j < k) {
-                        const float z = __uint_as_float(v[j]) + ctl->b2[j];
-                        code |= (z > 0.0f ? 1u : 0u) << j;
-                        if (zout) zout[static_cast<size_t>(g) * k + j] = z;
-                    }
-                }
-                codes[g] = code;
-            }
+            codes2(my_tiles - 1);
         }
     }
     ptx::tc_fence_before();
