@@ -18,18 +18,20 @@
 //                    four more blocks form the pairs' loss terms
 //   mlp_reduce_kernel  the shares of all chunks, the loss, and in training the
 //                    Adam update with the BF16 copies of the next step
-// The step is bound by FP32 issue (0.43 GFMA at a batch of 2,048 pairs, 11 us
-// on 148 SMs) and by the latency of three short launches. Before: eight
-// launches, with the weight gradients in 8 and 32 blocks that walked all rows
-// (dW2 566 us, dW1 515 us) and W1 transposed through 2-byte shared stores in
-// every forward block (115 us). One step at 2,048 pairs, 16 bits (whole
-// mlp_loss_grad call): 865 -> 103 us, at 4,096 pairs 1,671 -> 168 us; 300 training
-// steps of 2,048 pairs with their labels 266 -> 25 ms. The gradients' error
-// against FP64 fell with the shorter sums (2,048 pairs: 1.0e-6 -> 1.4e-7 of the norm).
+// The step is bound by FP32 issue (0.43 GFMA at a batch of 2,048 pairs, 14 us on
+// 148 SMs at the 1.2 cycles that a warp's FMA takes; paired FMAs (f32x2) take
+// 2.4), by the bandwidth from shared memory to registers and by the latency of
+// three short launches. Before: eight launches, with the weight gradients in 8
+// and 32 blocks that walked all rows (dW2 566 us, dW1 515 us) and W1 transposed
+// through 2-byte shared stores in every forward block (115 us). One step at 2,048
+// pairs, 16 bits (whole mlp_loss_grad call): 865 -> 78 us (of which the forward 16,
+// the backward 22). The gradients' error against FP64 fell with the shorter sums
+// (2,048 pairs: 1.0e-6 -> 1.7e-7 of the norm).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cuda_bf16.h>
+#include <type_traits>
 #include "learned.cuh"
 
 namespace sift {
@@ -39,8 +41,11 @@ namespace {
 // 48 rows per block (128 blocks for 3 x 2,048 rows: one wave). W1 arrives
 // transposed ([in][hidden], 64 KB) so that it is copied as it is; warp w owns
 // rows 6 w .. 6 w + 5 and lane l hidden units 8 l .. 8 l + 7, so one 16-byte
-// load of weights and three broadcast loads of inputs feed 48 FMAs. Sums run
-// over the inputs (hidden units) in order.
+// load of weights and three broadcast loads of inputs feed 48 FMAs (19,000 cycles
+// of the block's 31,000; a warp's FMAs alone would take 14,700). 16 warps of 6 rows
+// and 4 units each took 20,900: as many FMAs for more loaded bytes. The weights
+// arrive by asynchronous copies under the conversion of the inputs. Sums run over
+// the inputs (hidden units) in order.
 constexpr int kFwdRows = 48;
 constexpr int kFwdThreads = 256;
 constexpr int kFwdWarpRows = kFwdRows / (kFwdThreads / 32);
@@ -49,34 +54,78 @@ constexpr int kFwdW2Pitch = kMlpOutRows + 1;
 constexpr size_t kFwdSmem = kMlpIn * kMlpHidden * 2 + kMlpHidden * kFwdW2Pitch * 4 + kFwdRows * kMlpIn * 4 +
                             kFwdRows * kFwdHPitch * 4;
 
+// Layer 2 of NR rows of a warp (h: the first of them), one output per lane.
+template <int NR>
+__device__ __forceinline__ void fwd_layer2(const float* __restrict__ h, const float* __restrict__ w2m, float (&acc)[NR]) {
+    #pragma unroll
+    for (int r = 0; r < NR; ++r) acc[r] = 0.0f;
+    #pragma unroll 4
+    for (int j = 0; j < kMlpHidden; j += 4) {
+        float w[4];
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) w[u] = w2m[(j + u) * kFwdW2Pitch];
+        #pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const float4 hv = *reinterpret_cast<const float4*>(h + r * kFwdHPitch + j);
+            acc[r] = fmaf(hv.x, w[0], acc[r]);
+            acc[r] = fmaf(hv.y, w[1], acc[r]);
+            acc[r] = fmaf(hv.z, w[2], acc[r]);
+            acc[r] = fmaf(hv.w, w[3], acc[r]);
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kFwdThreads, 1)
     mlp_fwd_kernel(const uint8_t* __restrict__ x, int R, const __nv_bfloat16* __restrict__ w1t,
                    const float* __restrict__ b1, const __nv_bfloat16* __restrict__ w2b, const float* __restrict__ b2,
                    int k, float* __restrict__ h_out, float* __restrict__ t_out, float* __restrict__ colpart) {
     extern __shared__ __align__(16) uint8_t smem[];
     uint8_t* w1s = smem;                                                            // [128][256] bf16
-    float* w2s = reinterpret_cast<float*>(smem + kMlpIn * kMlpHidden * 2);          // [256][33]
-    float* xs = w2s + kMlpHidden * kFwdW2Pitch;                                     // [128][48]
+    float* xs = reinterpret_cast<float*>(smem + kMlpIn * kMlpHidden * 2);           // [128][48]
     float* hs = xs + kFwdRows * kMlpIn;                                             // [48][260]
+    float* w2s = hs + kFwdRows * kFwdHPitch;                                        // [256][33]
     __shared__ float s_col[kFwdThreads / 32][32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = blockIdx.x * kFwdRows;
-    #pragma unroll 8
     for (int e = tid; e < kMlpIn * kMlpHidden / 8; e += kFwdThreads)
-        reinterpret_cast<uint4*>(w1s)[e] = reinterpret_cast<const uint4*>(w1t)[e];
-    for (int e = tid; e < kFwdRows * 8; e += kFwdThreads) {
-        const int r = e % kFwdRows, c = e / kFwdRows;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (row0 + r < R) v = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row0 + r) * kMlpIn)[c];
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(w1s + 16 * e))),
+                     "l"(w1t + 8 * e)
+                     : "memory");
+    uint4 xv[(kFwdRows * 8 + kFwdThreads - 1) / kFwdThreads], wv[kMlpOutRows * kMlpHidden / 8 / kFwdThreads];
+    #pragma unroll
+    for (int u = 0; u < static_cast<int>(sizeof(xv) / 16); ++u) {
+        const int e = tid + u * kFwdThreads, r = e % kFwdRows, c = e / kFwdRows;
+        xv[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (c < 8 && row0 + r < R) xv[u] = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row0 + r) * kMlpIn)[c];
+    }
+    #pragma unroll
+    for (int u = 0; u < static_cast<int>(sizeof(wv) / 16); ++u) {
+        const int e = tid + u * kFwdThreads, m = e % kMlpOutRows, c = e / kMlpOutRows;
+        wv[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (m < k) wv[u] = reinterpret_cast<const uint4*>(w2b + m * kMlpHidden)[c];
+    }
+    const float4 bj[2] = {reinterpret_cast<const float4*>(b1)[2 * lane], reinterpret_cast<const float4*>(b1)[2 * lane + 1]};
+    #pragma unroll
+    for (int u = 0; u < static_cast<int>(sizeof(xv) / 16); ++u) {
+        const int e = tid + u * kFwdThreads, r = e % kFwdRows, c = e / kFwdRows;
+        if (c >= 8) break;
+        const uint32_t w[4] = {xv[u].x, xv[u].y, xv[u].z, xv[u].w};
         #pragma unroll
         for (int i = 0; i < 16; ++i)
             xs[(16 * c + i) * kFwdRows + r] = static_cast<float>((w[i >> 2] >> (8 * (i & 3))) & 0xffu) * kMlpInScale;
     }
-    for (int e = tid; e < kMlpOutRows * kMlpHidden; e += kFwdThreads) {
-        const int m = e / kMlpHidden, j = e % kMlpHidden;
-        w2s[j * kFwdW2Pitch + m] = m < k ? __bfloat162float(w2b[e]) : 0.0f;
+    #pragma unroll
+    for (int u = 0; u < static_cast<int>(sizeof(wv) / 16); ++u) {
+        const int e = tid + u * kFwdThreads, m = e % kMlpOutRows, c = e / kMlpOutRows;
+        const uint32_t w[4] = {wv[u].x, wv[u].y, wv[u].z, wv[u].w};
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            w2s[(8 * c + 2 * i) * kFwdW2Pitch + m] = __uint_as_float(w[i] << 16);
+            w2s[(8 * c + 2 * i + 1) * kFwdW2Pitch + m] = __uint_as_float(w[i] & 0xffff0000u);
+        }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     {
         float acc[kFwdWarpRows][8];
@@ -86,7 +135,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             for (int c = 0; c < 8; ++c) acc[r][c] = 0.0f;
         const uint4* wp = reinterpret_cast<const uint4*>(w1s) + lane;
         const float* xp = xs + warp * kFwdWarpRows;
-        #pragma unroll 4
+        #pragma unroll 8
         for (int i = 0; i < kMlpIn; ++i) {
             const uint4 v = wp[i * (kMlpHidden / 8)];
             const uint32_t w2[4] = {v.x, v.y, v.z, v.w};
@@ -98,26 +147,24 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             }
             #pragma unroll
             for (int r = 0; r < kFwdWarpRows; r += 2) {
-                const float2 xv = *reinterpret_cast<const float2*>(xp + i * kFwdRows + r);
+                const float2 xv2 = *reinterpret_cast<const float2*>(xp + i * kFwdRows + r);
                 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
-                    acc[r][c] = fmaf(xv.x, w[c], acc[r][c]);
-                    acc[r + 1][c] = fmaf(xv.y, w[c], acc[r + 1][c]);
+                    acc[r][c] = fmaf(xv2.x, w[c], acc[r][c]);
+                    acc[r + 1][c] = fmaf(xv2.y, w[c], acc[r + 1][c]);
                 }
             }
         }
-        float bj[8];
-        #pragma unroll
-        for (int c = 0; c < 8; ++c) bj[c] = b1[8 * lane + c];
         #pragma unroll
         for (int r = 0; r < kFwdWarpRows; ++r) {
             const int lr = warp * kFwdWarpRows + r;
-            float hv[8];
-            #pragma unroll
-            for (int c = 0; c < 8; ++c) hv[c] = __bfloat162float(__float2bfloat16_rn(fmaxf(acc[r][c] + bj[c], 0.0f)));
             #pragma unroll
             for (int g = 0; g < 2; ++g) {
-                const float4 o = make_float4(hv[4 * g], hv[4 * g + 1], hv[4 * g + 2], hv[4 * g + 3]);
+                const float* z = acc[r] + 4 * g;
+                const float4 o = make_float4(__bfloat162float(__float2bfloat16_rn(fmaxf(z[0] + bj[g].x, 0.0f))),
+                                             __bfloat162float(__float2bfloat16_rn(fmaxf(z[1] + bj[g].y, 0.0f))),
+                                             __bfloat162float(__float2bfloat16_rn(fmaxf(z[2] + bj[g].z, 0.0f))),
+                                             __bfloat162float(__float2bfloat16_rn(fmaxf(z[3] + bj[g].w, 0.0f))));
                 *reinterpret_cast<float4*>(hs + lr * kFwdHPitch + 8 * lane + 4 * g) = o;
                 if (row0 + lr < R)
                     *reinterpret_cast<float4*>(h_out + static_cast<size_t>(row0 + lr) * kMlpHidden + 8 * lane + 4 * g) =
@@ -126,33 +173,33 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         }
     }
     __syncwarp();  // layer 2 reads the warp's own rows
-    float acc[kFwdWarpRows];
-    #pragma unroll
-    for (int r = 0; r < kFwdWarpRows; ++r) acc[r] = 0.0f;
-    #pragma unroll 2
-    for (int j = 0; j < kMlpHidden; j += 4) {
-        float w[4];
-        #pragma unroll
-        for (int u = 0; u < 4; ++u) w[u] = w2s[(j + u) * kFwdW2Pitch + lane];
-        #pragma unroll
-        for (int r = 0; r < kFwdWarpRows; ++r) {
-            const float4 hv = *reinterpret_cast<const float4*>(hs + (warp * kFwdWarpRows + r) * kFwdHPitch + j);
-            acc[r] = fmaf(hv.x, w[0], acc[r]);
-            acc[r] = fmaf(hv.y, w[1], acc[r]);
-            acc[r] = fmaf(hv.z, w[2], acc[r]);
-            acc[r] = fmaf(hv.w, w[3], acc[r]);
-        }
-    }
-    const float bm = lane < k ? b2[lane] : 0.0f;
     float col = 0.0f;
-    #pragma unroll
-    for (int r = 0; r < kFwdWarpRows; ++r) {
-        const int row = row0 + warp * kFwdWarpRows + r;
-        if (row < R) {
-            const float t = lane < k ? tanhf(acc[r] + bm) : 0.0f;
-            t_out[static_cast<size_t>(row) * kMlpOutRows + lane] = t;
+    auto finish = [&](int lr, int m, float z) {  // t of row lr, output m
+        if (row0 + lr < R) {
+            const float t = m < k ? tanhf(z + (m < k ? b2[m] : 0.0f)) : 0.0f;
+            t_out[static_cast<size_t>(row0 + lr) * kMlpOutRows + m] = t;
             col += t;
         }
+    };
+    if (k <= kMlpOutRows / 2) {
+        // Half the lanes would have no output: each half of a warp takes half its rows.
+        constexpr int NR = kFwdWarpRows / 2;
+        const int m = lane & 15, lr = warp * kFwdWarpRows + (lane >> 4) * NR;
+        float acc[NR];
+        fwd_layer2<NR>(hs + lr * kFwdHPitch, w2s + m, acc);
+        #pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            finish(lr + r, m, acc[r]);
+            if (row0 + lr + r < R) t_out[static_cast<size_t>(row0 + lr + r) * kMlpOutRows + 16 + m] = 0.0f;
+        }
+        col += __shfl_xor_sync(0xffffffffu, col, 16);
+        if (lane >= 16) col = 0.0f;
+    } else {
+        const int lr = warp * kFwdWarpRows;
+        float acc[kFwdWarpRows];
+        fwd_layer2<kFwdWarpRows>(hs + lr * kFwdHPitch, w2s + lane, acc);
+        #pragma unroll
+        for (int r = 0; r < kFwdWarpRows; ++r) finish(lr + r, lane, acc[r]);
     }
     s_col[warp][lane] = col;
     __syncthreads();
@@ -169,8 +216,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
 // C = gridDim.y, 32 pairs (96 rows: queries, neighbours, random rows) at a time:
 // dz of the 96 rows, then per 32 rows the hidden gradient
 // da1[row][j] = (sum_m dz[row][m] W2[m][j]) (h[row][j] > 0) and the rank-32
-// updates dW1 += da1^T (x / 64) (4 x 8 outputs per thread, 64 x 128 per block),
-// dW2 += dz^T h, db1, db2. The next 32 rows' x and h load meanwhile. The four
+// updates dW1 += da1^T (x / 64) (4 x 8 outputs per thread, 64 x 128 per half of the
+// block) and dW2 += dz^T h in one loop: each half of the block's 16 warps takes
+// every second row, and the halves' sums meet at the end. db1 and db2 are summed
+// where da1 and dz are formed. The next 32 rows' x and h load meanwhile. 8 warps
+// that took all rows and ran dW2 as a loop of its own needed 68,500 cycles, this
+// 43,300 (38.5 -> 22 us); 8 x 8 outputs per thread over four row groups 53,200. The four
 // blocks of a chunk recompute its dz (a few FMAs per row against the 8,192 of
 // its share of dW1). The chunk's sums go to part[c][kMlpParamCount].
 // Blocks (a, C) are the loss role, which only reads t and runs beside the
@@ -179,12 +230,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
 // p + 32, ... per strided sum) that does not depend on the chunks.
 constexpr int kBwdCols = 64;
 constexpr int kBwdPairs = 32;
-constexpr int kBwdThreads = 256;
+constexpr int kBwdThreads = 512;
 constexpr int kBwdColBlocks = kMlpHidden / kBwdCols;
 constexpr int kBwdMaxChunks = 36;  // + the loss role, x 4 column blocks = one block per SM
-constexpr int kBwdPitch = kBwdCols + 4, kBwdXPitch = kMlpIn + 4;
-constexpr size_t kBwdSmem =
-    (3 * kBwdPairs * 33 + 32 * kBwdPitch * 2 + 32 * kBwdXPitch + kMlpOutRows * kBwdCols + 32 + 8 * 32) * 4;
+constexpr int kBwdPitch = kBwdCols + 4, kBwdXPitch = kMlpIn + 4, kBwdDzPitch = kMlpOutRows + 4;
+constexpr size_t kBwdSmem = (3 * kBwdPairs * kBwdDzPitch + 32 * kBwdPitch * 2 + 32 * kBwdXPitch +
+                             kMlpOutRows * kBwdCols + 32 + (kBwdThreads / 32) * 32) * 4;
+// The sums at the end of a block reuse the buffers of its loop.
+static_assert((kBwdCols * kMlpIn + kMlpOutRows * kBwdCols + 32 * kBwdCols + (kBwdThreads / 32) * 32) * 4 <= kBwdSmem,
+              "buffers of the final sums");
 
 __device__ __forceinline__ void loss_role(const float* __restrict__ t, int B, int k, int a, float* __restrict__ colp,
                                           float* __restrict__ terms) {
@@ -235,20 +289,40 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     float* as = hs + 32 * kBwdPitch;                   // [32][68]
     float* xs = as + 32 * kBwdPitch;                   // [32][132]
     float* w2s = xs + 32 * kBwdXPitch;                 // [32][64]
-    float* dzs = w2s + kMlpOutRows * kBwdCols;         // [96][33]
-    float* cs = dzs + 3 * kBwdPairs * 33;              // [32]
-    float* red = cs + 32;                              // [8][32]
+    float* dzs = w2s + kMlpOutRows * kBwdCols;         // [96][36]
+    float* cs = dzs + 3 * kBwdPairs * kBwdDzPitch;     // [32]
+    float* red = cs + 32;                              // [16][32]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int col0 = blockIdx.x * kBwdCols;
     const int i_begin = static_cast<int>(static_cast<long long>(B) * c / C);
     const int i_end = static_cast<int>(static_cast<long long>(B) * (c + 1) / C);
     const float rows = 3.0f * B;
+    constexpr int kWarps = kBwdThreads / 32;
+
+    // Row r4 of a part and its 4 hidden units (8 inputs) from 4 q4 (8 q4): what
+    // this thread loads, and the hidden gradient that it forms.
+    const int r4 = tid >> 4, q4 = tid & 15;
+    uint2 nx;
+    float4 nh;
+    auto fetch = [&](int p, int i0, int np) {
+        if (r4 < np) {
+            const size_t row = static_cast<size_t>(p) * B + i0 + r4;
+            nx = reinterpret_cast<const uint2*>(x + row * kMlpIn)[q4];
+            nh = *reinterpret_cast<const float4*>(h + row * kMlpHidden + col0 + 4 * q4);
+        } else {
+            nx = make_uint2(0u, 0u);
+            nh = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    if (i_begin < i_end) fetch(0, i_begin, min(kBwdPairs, i_end - i_begin));
 
     {
         float s = 0.0f;
-        for (int b = warp; b < n_colpart; b += kBwdThreads / 32) s += colpart[static_cast<size_t>(b) * 32 + lane];
+        #pragma unroll 8
+        for (int b = warp; b < n_colpart; b += kWarps) s += colpart[static_cast<size_t>(b) * 32 + lane];
         red[warp * 32 + lane] = s;
     }
+    #pragma unroll
     for (int e = tid; e < kMlpOutRows * kBwdCols; e += kBwdThreads) {
         const int m = e / kBwdCols, j = e % kBwdCols;
         w2s[e] = m < k ? __bfloat162float(w2b[m * kMlpHidden + col0 + j]) : 0.0f;
@@ -257,158 +331,186 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
     if (warp == 0) {
         float s = 0.0f;
         #pragma unroll
-        for (int w = 0; w < kBwdThreads / 32; ++w) s += red[w * 32 + lane];
+        for (int w = 0; w < kWarps; ++w) s += red[w * 32 + lane];
         cs[lane] = s;
     }
     __syncthreads();
 
-    // Outputs of this thread: dW1 rows 4 ty .. + 3 (hidden units), columns
-    // 4 tx .. + 3 and 64 + 4 tx .. + 3; dW2 row m2, columns 8 j2 .. + 7.
-    const int ty = tid >> 4, tx = tid & 15;
-    const int m2 = tid >> 3, j2 = tid & 7;
-    float acc[4][8], acc2[8], b1s[4] = {0.0f, 0.0f, 0.0f, 0.0f}, b2s = 0.0f;
+    // Outputs of this thread, over the rows r with r % 2 == half: dW1 rows 4 ty .. + 3
+    // (hidden units), columns 4 tx .. + 3 and 64 + 4 tx .. + 3; dW2 rows ty (and
+    // 16 + ty), columns 4 tx .. + 3.
+    const int half = tid >> 8, ty = (tid >> 4) & 15, tx = tid & 15;
+    float acc[4][8], acc2[2][4], b1s[4] = {0.0f, 0.0f, 0.0f, 0.0f}, b2s = 0.0f;
     #pragma unroll
     for (int e = 0; e < 8; ++e) {
-        acc2[e] = 0.0f;
+        acc2[e >> 2][e & 3] = 0.0f;
         #pragma unroll
         for (int q = 0; q < 4; ++q) acc[q][e] = 0.0f;
     }
 
-    // x and h of 32 rows [part p of pairs i0 ..): 16 bytes of x and 32 of h per thread.
-    uint4 nx;
-    float4 nh[2];
-    auto fetch = [&](int p, int i0, int np) {
-        const int r = tid >> 3, q = tid & 7;
-        if (r < np) {
-            const size_t row = static_cast<size_t>(p) * B + i0 + r;
-            nx = reinterpret_cast<const uint4*>(x + row * kMlpIn)[q];
-            nh[0] = *reinterpret_cast<const float4*>(h + row * kMlpHidden + col0 + 8 * q);
-            nh[1] = *reinterpret_cast<const float4*>(h + row * kMlpHidden + col0 + 8 * q + 4);
-        } else {
-            nx = make_uint4(0u, 0u, 0u, 0u);
-            nh[0] = nh[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-    };
-
-    if (i_begin < i_end) fetch(0, i_begin, min(kBwdPairs, i_end - i_begin));
     for (int i0 = i_begin; i0 < i_end; i0 += kBwdPairs) {
         const int np = min(kBwdPairs, i_end - i0);
         // dz of the 3 np rows: a warp per pair, a lane per output.
-        for (int pi = warp; pi < kBwdPairs; pi += kBwdThreads / 32) {
+        constexpr int kPer = kBwdPairs / kWarps;
+        float tv[kPer][3];
+        #pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const int pi = warp + u * kWarps;
+            const size_t i = static_cast<size_t>(i0) + pi;
+            #pragma unroll
+            for (int p = 0; p < 3; ++p)
+                tv[u][p] = pi < np ? t[(static_cast<size_t>(p) * B + i) * kMlpOutRows + lane] : 0.0f;
+        }
+        #pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const int pi = warp + u * kWarps;
+            const float tq = tv[u][0], tp = tv[u][1], tn = tv[u][2];
+            float sqn = tq * tn;  // zero for lanes >= k
+            #pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sqn += __shfl_xor_sync(0xffffffffu, sqn, o);
+            sqn /= k;
+            const float cp = -1.0f / (k * static_cast<float>(B));
+            const float cn = lw.neg * 2.0f * sqn / (k * static_cast<float>(B));
             float dq = 0.0f, dp = 0.0f, dn = 0.0f;
-            if (pi < np) {
-                const size_t i = static_cast<size_t>(i0) + pi;
-                const float tq = t[i * kMlpOutRows + lane], tp = t[(B + i) * kMlpOutRows + lane],
-                            tn = t[(2 * static_cast<size_t>(B) + i) * kMlpOutRows + lane];
-                float sqn = tq * tn;  // zero for lanes >= k
-                #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) sqn += __shfl_xor_sync(0xffffffffu, sqn, o);
-                sqn /= k;
-                const float cp = -1.0f / (k * static_cast<float>(B));
-                const float cn = lw.neg * 2.0f * sqn / (k * static_cast<float>(B));
-                if (lane < k) {
-                    const float bal = lw.balance * 2.0f * (cs[lane] / rows) / rows;
-                    dq = (cp * tp + cn * tn + bal) * (1.0f - tq * tq);
-                    dp = (cp * tq + bal) * (1.0f - tp * tp);
-                    dn = (cn * tq + bal) * (1.0f - tn * tn);
-                }
+            if (pi < np && lane < k) {
+                const float bal = lw.balance * 2.0f * (cs[lane] / rows) / rows;
+                dq = (cp * tp + cn * tn + bal) * (1.0f - tq * tq);
+                dp = (cp * tq + bal) * (1.0f - tp * tp);
+                dn = (cn * tq + bal) * (1.0f - tn * tn);
             }
-            dzs[pi * 33 + lane] = dq;
-            dzs[(kBwdPairs + pi) * 33 + lane] = dp;
-            dzs[(2 * kBwdPairs + pi) * 33 + lane] = dn;
+            dzs[pi * kBwdDzPitch + lane] = dq;
+            dzs[(kBwdPairs + pi) * kBwdDzPitch + lane] = dp;
+            dzs[(2 * kBwdPairs + pi) * kBwdDzPitch + lane] = dn;
+            b2s += dq + dp + dn;
         }
         for (int p = 0; p < 3; ++p) {
             {
-                const int r = tid >> 3, q = tid & 7;
-                const uint32_t w[4] = {nx.x, nx.y, nx.z, nx.w};
+                const uint32_t w[2] = {nx.x, nx.y};
                 #pragma unroll
-                for (int g = 0; g < 4; ++g)
-                    *reinterpret_cast<float4*>(xs + r * kBwdXPitch + 16 * q + 4 * g) =
+                for (int g = 0; g < 2; ++g)
+                    *reinterpret_cast<float4*>(xs + r4 * kBwdXPitch + 8 * q4 + 4 * g) =
                         make_float4(static_cast<float>(w[g] & 0xffu) * kMlpInScale,
                                     static_cast<float>((w[g] >> 8) & 0xffu) * kMlpInScale,
                                     static_cast<float>((w[g] >> 16) & 0xffu) * kMlpInScale,
                                     static_cast<float>(w[g] >> 24) * kMlpInScale);
-                *reinterpret_cast<float4*>(hs + r * kBwdPitch + 8 * q) = nh[0];
-                *reinterpret_cast<float4*>(hs + r * kBwdPitch + 8 * q + 4) = nh[1];
+                *reinterpret_cast<float4*>(hs + r4 * kBwdPitch + 4 * q4) = nh;
             }
+            const float4 hr = nh;
             if (p < 2)
                 fetch(p + 1, i0, np);
             else if (i0 + kBwdPairs < i_end)
                 fetch(0, i0 + kBwdPairs, min(kBwdPairs, i_end - i0 - kBwdPairs));
             __syncthreads();  // dzs, xs, hs
-            const float* dz = dzs + p * kBwdPairs * 33;
+            const float* dz = dzs + p * kBwdPairs * kBwdDzPitch;
             {
-                const int r = tid >> 3, q = tid & 7;
-                float s[8];
-                #pragma unroll
-                for (int e = 0; e < 8; ++e) s[e] = 0.0f;
-                for (int m = 0; m < k; ++m) {
-                    const float d = dz[r * 33 + m];
-                    const float4 wa = *reinterpret_cast<const float4*>(w2s + m * kBwdCols + 8 * q);
-                    const float4 wb = *reinterpret_cast<const float4*>(w2s + m * kBwdCols + 8 * q + 4);
-                    s[0] = fmaf(d, wa.x, s[0]);
-                    s[1] = fmaf(d, wa.y, s[1]);
-                    s[2] = fmaf(d, wa.z, s[2]);
-                    s[3] = fmaf(d, wa.w, s[3]);
-                    s[4] = fmaf(d, wb.x, s[4]);
-                    s[5] = fmaf(d, wb.y, s[5]);
-                    s[6] = fmaf(d, wb.z, s[6]);
-                    s[7] = fmaf(d, wb.w, s[7]);
+                // dz and W2 are zero for outputs past k.
+                float g[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                #pragma unroll 4
+                for (int m = 0; m < k; m += 4) {
+                    const float4 d = *reinterpret_cast<const float4*>(dz + r4 * kBwdDzPitch + m);
+                    const float dv[4] = {d.x, d.y, d.z, d.w};
+                    #pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float4 w = *reinterpret_cast<const float4*>(w2s + (m + u) * kBwdCols + 4 * q4);
+                        g[0] = fmaf(dv[u], w.x, g[0]);
+                        g[1] = fmaf(dv[u], w.y, g[1]);
+                        g[2] = fmaf(dv[u], w.z, g[2]);
+                        g[3] = fmaf(dv[u], w.w, g[3]);
+                    }
                 }
-                const float* hr = hs + r * kBwdPitch + 8 * q;
-                #pragma unroll
-                for (int e = 0; e < 8; ++e) as[r * kBwdPitch + 8 * q + e] = hr[e] > 0.0f ? s[e] : 0.0f;
+                const float4 a = make_float4(hr.x > 0.0f ? g[0] : 0.0f, hr.y > 0.0f ? g[1] : 0.0f,
+                                             hr.z > 0.0f ? g[2] : 0.0f, hr.w > 0.0f ? g[3] : 0.0f);
+                *reinterpret_cast<float4*>(as + r4 * kBwdPitch + 4 * q4) = a;
+                b1s[0] += a.x;
+                b1s[1] += a.y;
+                b1s[2] += a.z;
+                b1s[3] += a.w;
             }
             __syncthreads();  // as
-            #pragma unroll 4
-            for (int r = 0; r < 32; ++r) {
-                const float4 a = *reinterpret_cast<const float4*>(as + r * kBwdPitch + 4 * ty);
-                const float4 u = *reinterpret_cast<const float4*>(xs + r * kBwdXPitch + 4 * tx);
-                const float4 v = *reinterpret_cast<const float4*>(xs + r * kBwdXPitch + 64 + 4 * tx);
-                const float av[4] = {a.x, a.y, a.z, a.w};
-                const float bv[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-                #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    #pragma unroll
-                    for (int e = 0; e < 8; ++e) acc[q][e] = fmaf(av[q], bv[e], acc[q][e]);
-                    b1s[q] += av[q];
-                }
-            }
-            if (m2 < k) {
+            auto updates = [&](auto two_tag) {
+                constexpr bool TWO = decltype(two_tag)::value;  // more than 16 outputs
                 #pragma unroll 4
-                for (int r = 0; r < 32; ++r) {
-                    const float d = dz[r * 33 + m2];
-                    const float4 u = *reinterpret_cast<const float4*>(hs + r * kBwdPitch + 8 * j2);
-                    const float4 v = *reinterpret_cast<const float4*>(hs + r * kBwdPitch + 8 * j2 + 4);
-                    acc2[0] = fmaf(d, u.x, acc2[0]);
-                    acc2[1] = fmaf(d, u.y, acc2[1]);
-                    acc2[2] = fmaf(d, u.z, acc2[2]);
-                    acc2[3] = fmaf(d, u.w, acc2[3]);
-                    acc2[4] = fmaf(d, v.x, acc2[4]);
-                    acc2[5] = fmaf(d, v.y, acc2[5]);
-                    acc2[6] = fmaf(d, v.z, acc2[6]);
-                    acc2[7] = fmaf(d, v.w, acc2[7]);
-                    b2s += d;
+                for (int r = half; r < np; r += 2) {
+                    const float4 a = *reinterpret_cast<const float4*>(as + r * kBwdPitch + 4 * ty);
+                    const float4 u = *reinterpret_cast<const float4*>(xs + r * kBwdXPitch + 4 * tx);
+                    const float4 v = *reinterpret_cast<const float4*>(xs + r * kBwdXPitch + 64 + 4 * tx);
+                    const float4 hv = *reinterpret_cast<const float4*>(hs + r * kBwdPitch + 4 * tx);
+                    const float d = dz[r * kBwdDzPitch + ty];
+                    const float av[4] = {a.x, a.y, a.z, a.w};
+                    const float bv[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+                    const float cv[4] = {hv.x, hv.y, hv.z, hv.w};
+                    #pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        #pragma unroll
+                        for (int e = 0; e < 8; ++e) acc[q][e] = fmaf(av[q], bv[e], acc[q][e]);
+                    }
+                    #pragma unroll
+                    for (int e = 0; e < 4; ++e) acc2[0][e] = fmaf(d, cv[e], acc2[0][e]);
+                    if constexpr (TWO) {
+                        const float d1 = dz[r * kBwdDzPitch + 16 + ty];
+                        #pragma unroll
+                        for (int e = 0; e < 4; ++e) acc2[1][e] = fmaf(d1, cv[e], acc2[1][e]);
+                    }
                 }
-            }
+            };
+            if (k > 16)
+                updates(std::true_type{});
+            else
+                updates(std::false_type{});
             __syncthreads();  // xs, hs, as and (after the last part) dzs are rewritten
         }
     }
 
-    float* o = part + static_cast<size_t>(c) * kMlpParamCount;
-    float* o1 = o + static_cast<size_t>(col0) * kMlpIn;
-    #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        float* row = o1 + (4 * ty + q) * kMlpIn + 4 * tx;
-        *reinterpret_cast<float4*>(row) = make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
-        *reinterpret_cast<float4*>(row + 64) = make_float4(acc[q][4], acc[q][5], acc[q][6], acc[q][7]);
-        if (tx == 0) o[kMlpHidden * kMlpIn + col0 + 4 * ty + q] = b1s[q];
+    // The two halves' sums, then the rows' shares of db1 and the warps' of db2, in order.
+    float* f1 = reinterpret_cast<float*>(smem);  // [64][128]
+    float* f2 = f1 + kBwdCols * kMlpIn;          // [32][64]
+    float* fb1 = f2 + kMlpOutRows * kBwdCols;    // [32][64]
+    float* fb2 = fb1 + 32 * kBwdCols;            // [16][32]
+    if (half == 1) {
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            float* row = f1 + (4 * ty + q) * kMlpIn + 4 * tx;
+            *reinterpret_cast<float4*>(row) = make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
+            *reinterpret_cast<float4*>(row + 64) = make_float4(acc[q][4], acc[q][5], acc[q][6], acc[q][7]);
+        }
+        #pragma unroll
+        for (int g = 0; g < 2; ++g)
+            *reinterpret_cast<float4*>(f2 + (16 * g + ty) * kBwdCols + 4 * tx) =
+                make_float4(acc2[g][0], acc2[g][1], acc2[g][2], acc2[g][3]);
     }
+    *reinterpret_cast<float4*>(fb1 + r4 * kBwdCols + 4 * q4) = make_float4(b1s[0], b1s[1], b1s[2], b1s[3]);
+    fb2[warp * 32 + lane] = b2s;
+    __syncthreads();
+    float* o = part + static_cast<size_t>(c) * kMlpParamCount;
     float* o2 = o + kMlpHidden * kMlpIn + kMlpHidden;
-    float* row2 = o2 + m2 * kMlpHidden + col0 + 8 * j2;
-    *reinterpret_cast<float4*>(row2) = make_float4(acc2[0], acc2[1], acc2[2], acc2[3]);
-    *reinterpret_cast<float4*>(row2 + 4) = make_float4(acc2[4], acc2[5], acc2[6], acc2[7]);
-    if (blockIdx.x == 0 && j2 == 0) o2[kMlpOutRows * kMlpHidden + m2] = b2s;
+    if (half == 0) {
+        auto sum4 = [](const float* mine, const float* other) {
+            const float4 b = *reinterpret_cast<const float4*>(other);
+            return make_float4(mine[0] + b.x, mine[1] + b.y, mine[2] + b.z, mine[3] + b.w);
+        };
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float* row = f1 + (4 * ty + q) * kMlpIn + 4 * tx;
+            float* out = o + static_cast<size_t>(col0 + 4 * ty + q) * kMlpIn + 4 * tx;
+            *reinterpret_cast<float4*>(out) = sum4(acc[q], row);
+            *reinterpret_cast<float4*>(out + 64) = sum4(acc[q] + 4, row + 64);
+        }
+        #pragma unroll
+        for (int g = 0; g < 2; ++g)
+            *reinterpret_cast<float4*>(o2 + (16 * g + ty) * kMlpHidden + col0 + 4 * tx) =
+                sum4(acc2[g], f2 + (16 * g + ty) * kBwdCols + 4 * tx);
+    } else if (tid < 256 + kBwdCols) {
+        const int j = tid - 256;
+        float s = 0.0f;
+        #pragma unroll
+        for (int r = 0; r < 32; ++r) s += fb1[r * kBwdCols + j];
+        o[kMlpHidden * kMlpIn + col0 + j] = s;
+    } else if (blockIdx.x == 0 && warp == kWarps - 1) {
+        float s = 0.0f;
+        #pragma unroll
+        for (int w = 0; w < kWarps; ++w) s += fb2[w * 32 + lane];
+        o2[kMlpOutRows * kMlpHidden + lane] = s;
+    }
 }
 
 // ------------------------------------------------- reduction and Adam step
