@@ -95,9 +95,9 @@ int ensure_ready(DeviceCtx*& out, int& dev) {
             if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return SIFT_ERR_CUDA;
             if (prop.major != 10) return SIFT_ERR_UNSUPPORTED;  // sm_100a code only
             c.num_sms = prop.multiProcessorCount;
-            if (cudaMalloc(&c.d_status, 4 * sizeof(int)) != cudaSuccess) return SIFT_ERR_ALLOC;
-            if (cudaMemset(c.d_status, 0, 4 * sizeof(int)) != cudaSuccess) return SIFT_ERR_CUDA;
-            if (cudaMallocHost(&c.h_status, 4 * sizeof(int)) != cudaSuccess) return SIFT_ERR_ALLOC;
+            if (cudaMalloc(&c.d_status, kStatusInts * sizeof(int)) != cudaSuccess) return SIFT_ERR_ALLOC;
+            if (cudaMemset(c.d_status, 0, kStatusInts * sizeof(int)) != cudaSuccess) return SIFT_ERR_CUDA;
+            if (cudaMallocHost(&c.h_status, kStatusInts * sizeof(int)) != cudaSuccess) return SIFT_ERR_ALLOC;
             if (cudaStreamCreateWithFlags(&c.copy_stream, cudaStreamNonBlocking) != cudaSuccess) return SIFT_ERR_CUDA;
             for (auto& e : c.chunk_ev)
                 if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return SIFT_ERR_CUDA;
@@ -194,10 +194,10 @@ int map_cuda(cudaError_t e) {
 }
 
 
-// Reads and clears the device status words: one copy on `st` and one
+// Reads the first `ints` device status words (and clears the error code): one copy on `st` and one
 // synchronisation, which also waits for all the work enqueued on `st` before.
-int collect_device_status(DeviceCtx& c, cudaStream_t st) {
-    SIFT_CUDA(cudaMemcpyAsync(c.h_status, c.d_status, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+int collect_device_status(DeviceCtx& c, cudaStream_t st, int ints) {
+    SIFT_CUDA(cudaMemcpyAsync(c.h_status, c.d_status, ints * sizeof(int), cudaMemcpyDeviceToHost, st));
     SIFT_CUDA(cudaStreamSynchronize(st));
     const int code = c.h_status[0];
     if (code != 0) {

@@ -17,13 +17,14 @@ constexpr int kMaxDevices = 64;
 // Largest power-of-two scale 2^-s of descriptor values the exact kernels take.
 constexpr int kMaxShift = 24;
 
+constexpr int kStatusInts = 8;
 struct DeviceCtx {
     std::mutex mu;            // serialises the calls that use the arena
     bool ready = false;
     int num_sms = 0;
     char* arena = nullptr;    // scratch, grown on demand, reused across calls
     size_t arena_bytes = 0;
-    int* d_status = nullptr;  // [0] device error code, [1] pack flag / value stats [1..3]
+    int* d_status = nullptr;  // [0] device error code, [1..3] value stats, [4..7] loss of a training step (floats)
     int* h_status = nullptr;  // pinned mirror of d_status
     cudaStream_t copy_stream = nullptr;  // host->device chunk copies that overlap the search
     cudaEvent_t chunk_ev[17] = {};       // per-chunk "landed" events + one "arena free" event
@@ -92,7 +93,7 @@ int encode_bf16_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t ro
                    uint32_t box_rows);
 int map_cuda(cudaError_t e);
 // Reads and clears the device status words. Caller has synchronised `st`.
-int collect_device_status(DeviceCtx& c, cudaStream_t st);
+int collect_device_status(DeviceCtx& c, cudaStream_t st, int ints = 2);
 // Benchmark timing of one kernel launch on `st` (CUDA events recorded on the
 // launching stream when profiling is enabled; collected by tag).
 enum ProfTag : int { kProfSearch = 0, kProfHash = 1, kProfScan = 2, kProfTags = 3 };

@@ -158,7 +158,6 @@ int mlp_loss_grad(const uint8_t* x, int B, int k, const float* params, float neg
     const size_t o_w1t = L.take(kMlpHidden * kMlpIn * 2);
     const size_t o_w2b = L.take(kMlpOutRows * kMlpHidden * 2);
     const size_t o_tb = L.take(mlp_train_bytes(B));
-    const size_t o_loss = L.take(16);
     SIFT_TRY(detail::ensure_arena(c, L.off));
     char* A = c.arena;
     cudaStream_t st = nullptr;
@@ -166,13 +165,19 @@ int mlp_loss_grad(const uint8_t* x, int B, int k, const float* params, float neg
     const MlpParams g = mlp_params_at(grads);
     auto* w1t = reinterpret_cast<__nv_bfloat16*>(A + o_w1t);
     auto* w2b = reinterpret_cast<__nv_bfloat16*>(A + o_w2b);
-    float* loss = reinterpret_cast<float*>(A + o_loss);
+    // The loss lands next to the status word: one pinned copy brings both (a copy
+    // to the caller's pageable memory would wait for the kernels on its own).
+    float* loss = reinterpret_cast<float*>(c.d_status + 4);
     SIFT_CUDA(launch_mlp_export(p, k, nullptr, w1t, w2b, nullptr, nullptr, st));
     SIFT_CUDA(launch_mlp_loss_grad(x, B, k, p, w1t, w2b, MlpLossWeights{neg_w, bal_w}, mlp_train_bufs_at(A + o_tb, B),
                                    g, loss, st));
-    SIFT_CUDA(cudaMemcpyAsync(loss_host, loss, 4 * sizeof(float), cudaMemcpyDeviceToHost, st));
     detail::g_launches += 4;
-    return detail::collect_device_status(c, st);
+    const bool loss_dev = detail::is_device_accessible(loss_host);
+    if (loss_dev) SIFT_CUDA(cudaMemcpyAsync(loss_host, loss, 4 * sizeof(float), cudaMemcpyDeviceToDevice, st));
+    const int rc = detail::collect_device_status(c, st, detail::kStatusInts);
+    if (loss_dev) return rc;
+    if (rc == SIFT_OK || rc == SIFT_ERR_DEVICE_TIMEOUT) std::memcpy(loss_host, c.h_status + 4, 4 * sizeof(float));
+    return rc;
 }
 
 int mlp_train(const uint8_t* base, uint32_t r_n, const uint8_t* tq, uint32_t t_n, int k, int steps, int batch,

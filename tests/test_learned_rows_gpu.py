@@ -1,10 +1,12 @@
 """Gradients of one training step where the row halves of the backward, the row
 pairs of a forward warp and the two output ranges (up to 16, above) end, against
-FP64.
+FP64; and the place of the loss.
 
 Tolerance as for the other edges of the step: FP32 sums give relative errors near
 1e-6, a hidden value that rounds to the other BF16 neighbour changes by 2^-8 of
 itself and at most a few of a row's 256 do, so 2e-3 of a block's norm bounds both."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -38,3 +40,18 @@ def test_gradients_at_row_halves(cuda_device, B, k):
         assert np.linalg.norm(g[a:b] - want[a:b]) <= 2e-3 * np.linalg.norm(want[a:b])
     w2 = g[cuts[2]:cuts[3]].reshape(lh.OUT_ROWS, lh.HID)
     assert not w2[k:].any() and not g[cuts[3] + k:].any()  # outputs past k have no gradient
+
+
+def test_loss_lands_in_any_memory(cuda_device):
+    import torch
+
+    x = torch.from_numpy(_rows(4, 1)).to(cuda_device)
+    p = torch.from_numpy(lh.init_params(8, seed=1)).to(cuda_device)
+    g = torch.empty_like(p)
+    loss = torch.zeros(4, device=cuda_device)
+    fn = ms.lib().sift_mlp_loss_grad
+    pinned, pageable = torch.zeros(4).pin_memory(), torch.zeros(4)
+    for out in (loss, pinned, pageable):
+        assert fn(x.data_ptr(), 4, 8, p.data_ptr(), 0.7, 0.9, g.data_ptr(),
+                  ctypes.cast(out.data_ptr(), fn.argtypes[-1])) == ms.SIFT_OK
+    assert pageable[0] > 0 and torch.equal(pinned, pageable) and torch.equal(loss.cpu(), pageable)
