@@ -42,6 +42,7 @@
 #include <algorithm>
 #include <cuda_fp16.h>
 #include "exact2nn.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "epilogue.cuh"
 
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(256) row_norms_kernel(const uint8_t* __restric
                                                         int metric, int32_t* __restrict__ norm,
                                                         int32_t* __restrict__ rec,
                                                         int32_t* __restrict__ thresh) {
+    launch_next();
     // 32 rows per block, 8 threads per row, 16 elements per thread.
     const int row = blockIdx.x * 32 + (threadIdx.x >> 3);
     const int sub = threadIdx.x & 7;
@@ -212,6 +214,7 @@ __global__ void __launch_bounds__(256) row_norms_float_kernel(const __half* __re
                                                               int metric, int32_t* __restrict__ norm,
                                                               int32_t* __restrict__ rec,
                                                               int32_t* __restrict__ thresh) {
+    launch_next();
     const int row = blockIdx.x * 32 + (threadIdx.x >> 3);
     const int sub = threadIdx.x & 7;
     float s = 0.0f;
@@ -266,6 +269,7 @@ __global__ void __launch_bounds__(256)
     batch_prep_kernel(const uint8_t* __restrict__ base, const WorkItem* __restrict__ items, int n_items,
                       const WorkItem single, int tiles, int32_t* __restrict__ rec, const uint8_t* __restrict__ q, int q_n, int q_pad,
                       int32_t* __restrict__ qnorm, int32_t* __restrict__ thresh) {
+    launch_next();
     const int sub = threadIdx.x & 7, lrow = threadIdx.x >> 3;
     const bool is_base = static_cast<int>(blockIdx.x) < tiles;
     const uint8_t* x = q;
@@ -576,7 +580,7 @@ struct MergeOut {
 // ordered images of float keys (float_key) and qn is a float bit pattern (the
 // general float path); else integers.
 template <bool FLOATKEY>
-__device__ __forceinline__ void merge_finish(const MergeTop2& t, int q, int n_b, const int32_t* __restrict__ qnorm,
+__device__ __forceinline__ void merge_finish(const MergeTop2& t, int q, int n_b, const int32_t* qnorm,
                                              int metric, float thr, float dscale, const MergeOut& out) {
     // out.qmul (FP16 rows holding integers): query norms are floats, the integers divided by it.
     bool v1, v2;
@@ -658,7 +662,7 @@ __device__ __forceinline__ MergeTop2 merge_lists_of_rows(const MergeTop2& mine) 
 }
 
 // Lists sub, sub + step, ... < n of a row (list s at p + s * stride).
-__device__ __forceinline__ void merge_lists(MergeTop2& t, const int4* __restrict__ p, size_t stride, int sub, int n,
+__device__ __forceinline__ void merge_lists(MergeTop2& t, const int4* p, size_t stride, int sub, int n,
                                             int step) {
     int s = sub;
     for (; s + 3 * step < n; s += 4 * step) {
@@ -673,9 +677,10 @@ __device__ __forceinline__ void merge_lists(MergeTop2& t, const int4* __restrict
 
 template <bool FLOATKEY, int LANES>
 __global__ void __launch_bounds__(kMergeThreads<LANES>)
-    merge2nn_kernel(const int4* __restrict__ partial, const ExactPlan plan, const WorkItem* __restrict__ items,
-                    int n_items, const WorkItem single, int group_rows, int total_q, const int32_t* __restrict__ qnorm,
+    merge2nn_kernel(const int4* partial, const ExactPlan plan, const WorkItem* items,
+                    int n_items, const WorkItem single, int group_rows, int total_q, const int32_t* qnorm,
                     int metric, float thr, float dscale, const MergeOut out) {
+    wait_previous();
     const int row0 = blockIdx.x * (kMergeThreads<LANES> / LANES);
     int q = row0 + (LANES == 1 ? threadIdx.x : threadIdx.x % kMergeRows);
     const long long W = plan.units, G = plan.grid;
@@ -829,15 +834,13 @@ cudaError_t launch_merge(const int4* partial, const ExactPlan& plan, const WorkI
     const int lists = plan.max_splits * plan.parts;
     const int blocks = (total_q + kMergeRows - 1) / kMergeRows;
     if (lists <= 4)
-        merge2nn_kernel<FLOATKEY, 1><<<(total_q + 255) / 256, kMergeThreads<1>, 0, stream>>>(
+        return launch_after(merge2nn_kernel<FLOATKEY, 1>, (total_q + 255) / 256, kMergeThreads<1>, 0, stream,
             partial, plan, items, n_items, single, group_rows, total_q, qnorm, metric, threshold, dist_scale, out);
-    else if (lists <= 32)
-        merge2nn_kernel<FLOATKEY, 8><<<blocks, kMergeThreads<8>, 0, stream>>>(
+    if (lists <= 32)
+        return launch_after(merge2nn_kernel<FLOATKEY, 8>, blocks, kMergeThreads<8>, 0, stream,
             partial, plan, items, n_items, single, group_rows, total_q, qnorm, metric, threshold, dist_scale, out);
-    else
-        merge2nn_kernel<FLOATKEY, 32><<<blocks, kMergeThreads<32>, 0, stream>>>(
+    return launch_after(merge2nn_kernel<FLOATKEY, 32>, blocks, kMergeThreads<32>, 0, stream,
             partial, plan, items, n_items, single, group_rows, total_q, qnorm, metric, threshold, dist_scale, out);
-    return cudaGetLastError();
 }
 
 WorkItem merge_item(const ExactPlan& plan) {

@@ -86,6 +86,7 @@
 #include <climits>
 #include <type_traits>
 #include "exact2nn.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "epilogue.cuh"
 
@@ -312,6 +313,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
     volatile int* abort_flag = &ctl->abort_flag;
     volatile int* never = &ctl->no_abort;
 
+    wait_previous();
     Cursor cur;
     if (n_units > 0) cur.init(items, n_items, single, w_begin);
 
@@ -729,9 +731,8 @@ cudaError_t launch_batch_variant(const CUtensorMap& qmap, const CUtensorMap& bma
     cudaError_t e = set_smem_once(exact2nn_u8_pair_batch_kernel<QPT, QB>, Cfg::kSmemBytes, attr_set);
     if (e != cudaSuccess) return e;
     if (bp.plan.grid <= 0) return cudaSuccess;
-    exact2nn_u8_pair_batch_kernel<QPT, QB><<<2 * bp.plan.grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(
+    return launch_after(exact2nn_u8_pair_batch_kernel<QPT, QB>, 2 * bp.plan.grid, Cfg::kThreads, Cfg::kSmemBytes, stream,
         qmap, bmap, brec, bp.plan, bp.items, bp.n_items, single_item(bp.plan), partial, thresh, err);
-    return cudaGetLastError();
 }
 
 }  // namespace
@@ -745,9 +746,8 @@ cudaError_t launch_exact2nn_u8_pair(const CUtensorMap& qmap, const CUtensorMap& 
     cudaError_t e = set_smem_once(exact2nn_u8_pair_kernel, CfgU8::kSmemBytes, attr_set);
     if (e != cudaSuccess) return e;
     if (plan.grid <= 0) return cudaSuccess;
-    exact2nn_u8_pair_kernel<<<2 * plan.grid, CfgU8::kThreads, CfgU8::kSmemBytes, stream>>>(
+    return launch_after(exact2nn_u8_pair_kernel, 2 * plan.grid, CfgU8::kThreads, CfgU8::kSmemBytes, stream,
         qmap, bmap_half, brec, plan, single_item(plan), partial, thresh, err);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_exact2nn_u8fold_pair(const CUtensorMap& qmap, const CUtensorMap& bmap_half,
@@ -757,9 +757,8 @@ cudaError_t launch_exact2nn_u8fold_pair(const CUtensorMap& qmap, const CUtensorM
     cudaError_t e = set_smem_once(exact2nn_u8fold_pair_kernel, CfgFold::kSmemBytes, attr_set);
     if (e != cudaSuccess) return e;
     if (plan.grid <= 0) return cudaSuccess;
-    exact2nn_u8fold_pair_kernel<<<2 * plan.grid, CfgFold::kThreads, CfgFold::kSmemBytes, stream>>>(
+    return launch_after(exact2nn_u8fold_pair_kernel, 2 * plan.grid, CfgFold::kThreads, CfgFold::kSmemBytes, stream,
         qmap, bmap_half, fmap, brec, plan, single_item(plan), partial, thresh, err);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_exact2nn_u8fold_pair_item(const CUtensorMap& qmap, const CUtensorMap& bmap_half,
@@ -770,9 +769,8 @@ cudaError_t launch_exact2nn_u8fold_pair_item(const CUtensorMap& qmap, const CUte
     cudaError_t e = set_smem_once(exact2nn_u8fold_pair_kernel, CfgFold::kSmemBytes, attr_set);
     if (e != cudaSuccess) return e;
     if (plan.grid <= 0) return cudaSuccess;
-    exact2nn_u8fold_pair_kernel<<<2 * plan.grid, CfgFold::kThreads, CfgFold::kSmemBytes, stream>>>(
+    return launch_after(exact2nn_u8fold_pair_kernel, 2 * plan.grid, CfgFold::kThreads, CfgFold::kSmemBytes, stream,
         qmap, bmap_half, fmap, brec, plan, item, partial, thresh, err);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_exact2nn_u8_pair_item(const CUtensorMap& qmap, const CUtensorMap& bmap_half, const int32_t* brec,
@@ -782,9 +780,8 @@ cudaError_t launch_exact2nn_u8_pair_item(const CUtensorMap& qmap, const CUtensor
     cudaError_t e = set_smem_once(exact2nn_u8_pair_kernel, CfgU8::kSmemBytes, attr_set);
     if (e != cudaSuccess) return e;
     if (plan.grid <= 0) return cudaSuccess;
-    exact2nn_u8_pair_kernel<<<2 * plan.grid, CfgU8::kThreads, CfgU8::kSmemBytes, stream>>>(
+    return launch_after(exact2nn_u8_pair_kernel, 2 * plan.grid, CfgU8::kThreads, CfgU8::kSmemBytes, stream,
         qmap, bmap_half, brec, plan, item, partial, thresh, err);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_exact2nn_f16_pair(const CUtensorMap& qmap, const CUtensorMap& bmap_half, const int32_t* brec,
@@ -794,9 +791,8 @@ cudaError_t launch_exact2nn_f16_pair(const CUtensorMap& qmap, const CUtensorMap&
     cudaError_t e = set_smem_once(exact2nn_f16_pair_kernel, CfgF16::kSmemBytes, attr_set);
     if (e != cudaSuccess) return e;
     if (plan.grid <= 0) return cudaSuccess;
-    exact2nn_f16_pair_kernel<<<2 * plan.grid, CfgF16::kThreads, CfgF16::kSmemBytes, stream>>>(
+    return launch_after(exact2nn_f16_pair_kernel, 2 * plan.grid, CfgF16::kThreads, CfgF16::kSmemBytes, stream,
         qmap, bmap_half, brec, plan, single_item(plan), partial, thresh, err, dscale);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_exact2nn_float_pair(const CUtensorMap& qmap, const CUtensorMap& bmap_half, const int32_t* brec,
@@ -806,9 +802,8 @@ cudaError_t launch_exact2nn_float_pair(const CUtensorMap& qmap, const CUtensorMa
     cudaError_t e = set_smem_once(exact2nn_float_pair_kernel, CfgFloat::kSmemBytes, attr_set);
     if (e != cudaSuccess) return e;
     if (plan.grid <= 0) return cudaSuccess;
-    exact2nn_float_pair_kernel<<<2 * plan.grid, CfgFloat::kThreads, CfgFloat::kSmemBytes, stream>>>(
+    return launch_after(exact2nn_float_pair_kernel, 2 * plan.grid, CfgFloat::kThreads, CfgFloat::kSmemBytes, stream,
         qmap, bmap_half, brec, plan, single_item(plan), partial, thresh, err, has_lo ? 1 : 0);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_exact2nn_u8_pair_batch(const CUtensorMap& qmap, const CUtensorMap& bmap_half, const int32_t* brec,

@@ -21,7 +21,8 @@
 // The step is bound by FP32 issue (0.43 GFMA at a batch of 2,048 pairs, 14 us on
 // 148 SMs at the 1.2 cycles that a warp's FMA takes; paired FMAs (f32x2) take
 // 2.4), by the bandwidth from shared memory to registers and by the latency of
-// three short launches. Before: eight launches, with the weight gradients in 8
+// three short launches, each of which starts while the one before still runs
+// (launch.cuh). Before: eight launches, with the weight gradients in 8
 // and 32 blocks that walked all rows (dW2 566 us, dW1 515 us) and W1 transposed
 // through 2-byte shared stores in every forward block (115 us). One step at 2,048
 // pairs, 16 bits (whole mlp_loss_grad call): 865 -> 76 us (of which the forward 16,
@@ -32,21 +33,11 @@
 #include <cstdint>
 #include <cuda_bf16.h>
 #include <type_traits>
+#include "launch.cuh"
 #include "learned.cuh"
 
 namespace sift {
 namespace {
-
-// The kernels of a step are launched while the one before still runs (launch_after),
-// so that their blocks stand ready when it ends: 80.5 -> 77.8 us per step. Nothing is
-// read or written before this wait, after which the kernel before, and with it all
-// earlier work of the stream, is complete; the next one may launch only then.
-// Their inputs are plain pointers (no const __restrict__), whose loads the compiler
-// may not take for constant and move above the wait.
-__device__ __forceinline__ void wait_previous() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 
 // ---------------------------------------------------------------- forward
 // 48 rows per block (128 blocks for 3 x 2,048 rows: one wave). W1 arrives
@@ -694,22 +685,6 @@ MlpTrainBufs mlp_train_bufs_at(char* base, int B) {
 }
 
 namespace {
-
-// A launch that need not wait for the kernel before it to end (wait_previous does).
-template <typename... P, typename... A>
-cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
 
 cudaError_t launch_fwd_bwd(const uint8_t* x, int B, int k, const MlpParams& p, const __nv_bfloat16* w1t,
                            const __nv_bfloat16* w2b, const MlpLossWeights& lw, const MlpTrainBufs& tb,

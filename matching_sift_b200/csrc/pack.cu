@@ -8,6 +8,7 @@
 #include <climits>
 #include <cuda_fp16.h>
 #include "exact2nn.cuh"
+#include "launch.cuh"
 #include "pack.cuh"
 
 namespace sift {
@@ -256,6 +257,7 @@ __global__ void __launch_bounds__(256)
                            int32_t* __restrict__ rec, const float* __restrict__ q, int q_n, int q_pad,
                            __half* __restrict__ q_out, int32_t* __restrict__ qnorm, int32_t* __restrict__ thresh,
                            float mul) {
+    launch_next();
     const int base_blocks = r_pad / 32;
     const bool is_base = static_cast<int>(blockIdx.x) < base_blocks;
     const int b = static_cast<int>(blockIdx.x) - (is_base ? 0 : base_blocks);
