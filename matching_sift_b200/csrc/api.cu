@@ -473,7 +473,7 @@ int exact_match_chunked(const MatchArgs& a, DeviceCtx& c, cudaStream_t st, bool 
         if (fold)
             SIFT_CUDA(launch_fold_records_u8(rows, plans[ch].r_n, plans[ch].r_pad, a.metric, rec,
                                              fold_digits + static_cast<size_t>(off / kBN) * 2 * kFoldHalfBytes / 4,
-                                             st));
+                                             nullptr, 0, 0, nullptr, nullptr, st));
         else
             SIFT_CUDA(launch_row_norms_u8(rows, plans[ch].r_n, plans[ch].r_pad, a.metric, nullptr, rec, nullptr, st));
         WorkItem it{};
@@ -625,7 +625,8 @@ int exact_match_float(const MatchArgs& a, DeviceCtx& c, cudaStream_t st, const V
 // folded norms: 517 x 733 (1 unit per worker) 11.1 | 15.9 us, 1,000 x 10,000 (2)
 // 16.9 | 25.3, 4,000 x 20,000 (17) 31.7 | 43.8, 3,000 x 60,000 (38) 51.3 | 58.7,
 // 10,000 x 30,000 (64) 74.9 | 81.6, 2,000 x 200,000 (85) 94.3 | 84.2,
-// 10,000 x 100,000 (211) 204 | 168.
+// 10,000 x 100,000 (211) 204 | 168. (Both have lost 1-4 us since, to overlapped
+// launches and to the query norms in the folded records' launch.)
 constexpr int kPackedUnits = 64;
 bool packed_search(const ExactPlan& plan, int metric) {
     return metric == SIFT_METRIC_L2 && plan.grid > 0 && plan.units <= static_cast<long long>(kPackedUnits) * plan.grid;
@@ -714,12 +715,12 @@ int exact_match(const MatchArgs& a) {
     if (use_packed) {
         SIFT_CUDA(launch_batch_prep(rd, qd, q_n, packed_plan, brec, qnorm, thresh, st));
         ++g_launches;
+    } else if (use_fold) {
+        SIFT_CUDA(launch_fold_records_u8(rd, r_n, plan.r_pad, a.metric, brec, reinterpret_cast<uint32_t*>(A + o_fold),
+                                         qd, q_n, plan.q_pad, qnorm, thresh, st));
+        ++g_launches;
     } else if (!use_f16) {
-        if (use_fold)
-            SIFT_CUDA(launch_fold_records_u8(rd, r_n, plan.r_pad, a.metric, brec,
-                                             reinterpret_cast<uint32_t*>(A + o_fold), st));
-        else
-            SIFT_CUDA(launch_row_norms_u8(rd, r_n, plan.r_pad, a.metric, nullptr, brec, nullptr, st));
+        SIFT_CUDA(launch_row_norms_u8(rd, r_n, plan.r_pad, a.metric, nullptr, brec, nullptr, st));
         SIFT_CUDA(launch_row_norms_u8(qd, q_n, plan.q_pad, kMetricL2, qnorm, nullptr, thresh, st));
         g_launches += (plan.r_pad > 0 ? 1 : 0) + 1;
     }

@@ -130,20 +130,25 @@ __global__ void __launch_bounds__(256) row_norms_kernel(const uint8_t* __restric
 //
 // One block per base tile: 8 threads per row, the 4 rows of a thread's
 // 32-row parts loaded up front (64 bytes in flight per thread), then per row
-// the norm, the folded half-norm c, its digits and the residual.
-__global__ void __launch_bounds__(256) fold_records_kernel(const uint8_t* __restrict__ x, int n, int n_pad,
-                                                           int metric, int32_t* __restrict__ rec,
-                                                           uint32_t* __restrict__ fold) {
-    const int t = blockIdx.x;
+// the norm, the folded half-norm c, its digits and the residual. Blocks past the
+// base tiles take 128 query rows each: norms and cleared bounds (a launch of
+// their own cost 2.5 us of every search).
+__global__ void __launch_bounds__(256)
+    fold_records_kernel(const uint8_t* __restrict__ x, int n, int n_pad, int metric, int32_t* __restrict__ rec,
+                        uint32_t* __restrict__ fold, const uint8_t* __restrict__ q, int q_n, int q_pad,
+                        int32_t* __restrict__ qnorm, int32_t* __restrict__ thresh) {
+    launch_next();
+    const int tiles = n_pad / kBN;
+    const bool is_base = static_cast<int>(blockIdx.x) < tiles;
+    const int t = is_base ? blockIdx.x : blockIdx.x - tiles;
     const int sub = threadIdx.x & 7;
     const int lrow = threadIdx.x >> 3;
     uint4 w[4];
     #pragma unroll
     for (int part = 0; part < 4; ++part) {
         const int row = t * kBN + part * 32 + lrow;
-        w[part] = row < n ? load16_u8(x, row, sub) : make_uint4(0u, 0u, 0u, 0u);
+        w[part] = row < (is_base ? n : q_n) ? load16_u8(is_base ? x : q, row, sub) : make_uint4(0u, 0u, 0u, 0u);
     }
-    __shared__ int32_t res[kBN];
     int32_t* r = rec + static_cast<size_t>(t) * kRecInts;
     #pragma unroll
     for (int part = 0; part < 4; ++part) {
@@ -156,6 +161,14 @@ __global__ void __launch_bounds__(256) fold_records_kernel(const uint8_t* __rest
         s += __shfl_xor_sync(0xffffffffu, s, 1);
         s += __shfl_xor_sync(0xffffffffu, s, 2);
         s += __shfl_xor_sync(0xffffffffu, s, 4);
+        if (!is_base) {
+            const int row = t * kBN + wr;
+            if (sub == 0 && row < q_pad) {
+                qnorm[row] = static_cast<int32_t>(s);
+                thresh[row] = thresh[q_pad + row] = INT_MAX;
+            }
+            continue;
+        }
         const int32_t norm = live ? (metric == kMetricL2 ? static_cast<int32_t>(s) : 0) : kKeyPad;
         const int32_t c = live ? min((norm + 1) >> 1, kFoldMax) : 0;
         const int32_t resid = norm - 2 * c;
@@ -171,23 +184,7 @@ __global__ void __launch_bounds__(256) fold_records_kernel(const uint8_t* __rest
         const size_t off = (static_cast<size_t>(t) * 2 + (wr >> 6)) * kFoldHalfBytes + ((wr & 63) >> 3) * 256 +
                            (sub >> 2) * 128 + (wr & 7) * 16 + 4 * (sub & 3);
         fold[off / 4] = word;
-        if (sub == 0) {
-            res[wr] = resid;
-            r[wr] = resid;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 16) {
-        int m = res[8 * threadIdx.x];
-        #pragma unroll
-        for (int i = 1; i < 8; ++i) m = min(m, res[8 * threadIdx.x + i]);
-        r[128 + threadIdx.x] = m;
-    } else if (threadIdx.x < 24) {
-        const int hh = threadIdx.x - 16;
-        int m = res[16 * hh];
-        #pragma unroll
-        for (int i = 1; i < 16; ++i) m = min(m, res[16 * hh + i]);
-        r[144 + hh] = m;
+        if (sub == 0) r[wr] = resid;
     }
 }
 
@@ -790,9 +787,11 @@ cudaError_t launch_row_norms_u8(const uint8_t* x, int n, int n_pad, int metric, 
 }
 
 cudaError_t launch_fold_records_u8(const uint8_t* x, int n, int n_pad, int metric, int32_t* rec, uint32_t* fold,
+                                   const uint8_t* q, int q_n, int q_pad, int32_t* qnorm, int32_t* thresh,
                                    cudaStream_t stream) {
-    if (n_pad <= 0) return cudaSuccess;
-    fold_records_kernel<<<n_pad / kBN, 256, 0, stream>>>(x, n, n_pad, metric, rec, fold);
+    const int blocks = n_pad / kBN + (q_pad + kBN - 1) / kBN;
+    if (blocks <= 0) return cudaSuccess;
+    fold_records_kernel<<<blocks, 256, 0, stream>>>(x, n, n_pad, metric, rec, fold, q, q_n, q_pad, qnorm, thresh);
     return cudaGetLastError();
 }
 

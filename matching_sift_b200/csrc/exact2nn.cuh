@@ -144,9 +144,11 @@ cudaError_t launch_merge2nn_float(const int4* partial, const ExactPlan& plan, in
 cudaError_t launch_row_norms_u8(const uint8_t* x, int n, int n_pad, int metric, int32_t* norm, int32_t* rec,
                                 int32_t* thresh, cudaStream_t stream);
 // Records of the fold variant: residuals |b|^2 - 2 c (c = the folded
-// half-norm) in place of the norms, their 8- and 16-row minima, and the
-// folding digits of every row, n_pad / kBN tiles x 2 x kFoldHalfBytes bytes.
+// half-norm) in place of the norms, no minima, and the folding digits of every
+// row, n_pad / kBN tiles x 2 x kFoldHalfBytes bytes; with the squared norms of q_n
+// query rows and the cleared bounds thresh[2 q_pad] (q_pad = 0: none).
 cudaError_t launch_fold_records_u8(const uint8_t* x, int n, int n_pad, int metric, int32_t* rec, uint32_t* fold,
+                                   const uint8_t* q, int q_n, int q_pad, int32_t* qnorm, int32_t* thresh,
                                    cudaStream_t stream);
 // The fused GEMM + top-2 kernel. partial: [max_splits][parts][q_pad] int4
 // {key1, idx1, key2, idx2} with key = norm(b) - 2 q.b. brec: base records
