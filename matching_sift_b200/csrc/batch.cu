@@ -76,7 +76,7 @@ int build(const sift_pair* pairs, int n_pairs, uint32_t r_rows, int qpt, int wor
     b.items.resize(n_pairs);
     b.units = make_batch_items(n_pairs, na.data(), nb.data(), off.data(), b.group_rows, b.items.data(),
                                &b.total_tiles, &b.total_q);
-    b.plan = make_batch_plan(b.items.data(), n_pairs, b.units, b.total_q, workers, 2);
+    b.plan = make_batch_plan(b.items.data(), n_pairs, b.group_rows, b.units, b.total_q, workers, 2);
     return SIFT_OK;
 }
 

@@ -108,7 +108,6 @@ enum AccKind : int {
 // a vote on its largest w. 512 pairs of 500-8,000 rows: always testing 1,251 us,
 // never 1,168, from tile 8 / 16 / 28 on 1,139 / 1,117 / 1,117; 64 pairs of
 // 7,000-8,000 rows: 863, 962, 848 / 843 / 855.
-constexpr int kPackedDenseTiles = 16;
 constexpr int kPackedMaxKey = 1 << 23;
 constexpr int kPackedNone = INT_MIN;  // w of a padding row: below every floor
 

@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(kMergeThreads<LANES>)
     wait_previous();
     const int row0 = blockIdx.x * (kMergeThreads<LANES> / LANES);
     int q = row0 + (LANES == 1 ? threadIdx.x : threadIdx.x % kMergeRows);
-    const long long W = plan.units, G = plan.grid;
+    const long long W = plan.weight > 0 ? plan.weight : plan.units, G = plan.grid;
     auto item_of = [&](int row) {
         return items ? items[find_item(n_items, row, [&](int k) { return static_cast<long long>(items[k].a_off); })]
                      : single;
@@ -693,9 +693,14 @@ __global__ void __launch_bounds__(kMergeThreads<LANES>)
         n_b = it.n_b;
         // No base rows: no CTA scanned this query and every neighbour is absent.
         if (W > 0 && it.tiles > 0) {
-            const long long first = it.u_begin + static_cast<long long>((q - it.a_off) / group_rows) * it.tiles;
+            const int g = (q - it.a_off) / group_rows;
+            long long first = it.u_begin + static_cast<long long>(g) * it.tiles, last = first + it.tiles - 1;
+            if (plan.weight > 0) {
+                first = unit_weight_begin(it, group_rows, g, 0);
+                last = unit_weight_begin(it, group_rows, g, it.tiles - 1);
+            }
             const int c0 = plan_cta_of(first, W, G);
-            const int c1 = plan_cta_of(first + it.tiles - 1, W, G);
+            const int c1 = plan_cta_of(last, W, G);
             merge_lists(t, partial + q, plan.q_pad, LANES == 1 ? 0 : threadIdx.x / kMergeRows,
                         (c1 - c0 + 1) * plan.parts, LANES);
         }
@@ -885,7 +890,7 @@ cudaError_t launch_batch_prep(const uint8_t* base, const uint8_t* q, int q_n, co
 
 long long make_batch_items(int n_items, const int* n_a, const int* n_b, const int* b_off, int group_rows,
                            WorkItem* items, int* total_tiles, int* total_queries) {
-    long long u = 0;
+    long long u = 0, w = 0;
     int a = 0, rec = 0;
     for (int p = 0; p < n_items; ++p) {
         WorkItem& it = items[p];
@@ -897,7 +902,9 @@ long long make_batch_items(int n_items, const int* n_a, const int* n_b, const in
         it.groups = (n_a[p] + group_rows - 1) / group_rows;
         it.tiles = (n_b[p] + kBN - 1) / kBN;
         it.u_begin = u;
+        it.w_begin = w;
         it.rec_off = rec;
+        if (it.groups > 0) w = unit_weight_begin(it, group_rows, it.groups - 1, it.tiles);
         u += static_cast<long long>(it.groups) * it.tiles;
         rec += it.tiles;
         a += n_a[p];
@@ -907,8 +914,9 @@ long long make_batch_items(int n_items, const int* n_a, const int* n_b, const in
     return u;
 }
 
-ExactPlan make_batch_plan(const WorkItem* items, int n_items, long long units, int total_queries, int num_workers,
-                          int parts) {
+constexpr int kMinWeightedUnits = 8;  // per worker: they weigh at least 32, a dense unit 6
+ExactPlan make_batch_plan(const WorkItem* items, int n_items, int group_rows, long long units, int total_queries,
+                          int num_workers, int parts) {
     ExactPlan p{};
     p.parts = parts;
     p.q_n = total_queries;
@@ -918,13 +926,24 @@ ExactPlan make_batch_plan(const WorkItem* items, int n_items, long long units, i
     p.units = units;
     p.grid = static_cast<int>(std::min<long long>(num_workers, units));
     int ms = 1;
+    // A share of at least one dense unit's weight holds a unit: no worker of a
+    // group's range is without one, so every list that the merge reads is written.
+    if (units >= kMinWeightedUnits * static_cast<long long>(p.grid) && n_items > 0) {
+        const WorkItem& it = items[n_items - 1];
+        p.weight = it.groups > 0 ? unit_weight_begin(it, group_rows, it.groups - 1, it.tiles) : it.w_begin;
+    }
+    const long long W = p.weight > 0 ? p.weight : units;
     if (p.grid > 0) {
         for (int k = 0; k < n_items; ++k) {
             const WorkItem& it = items[k];
             for (int g = 0; g < it.groups && it.tiles > 0; ++g) {
-                const long long first = it.u_begin + static_cast<long long>(g) * it.tiles;
-                const int c0 = plan_cta_of(first, units, p.grid);
-                const int c1 = plan_cta_of(first + it.tiles - 1, units, p.grid);
+                long long first = it.u_begin + static_cast<long long>(g) * it.tiles, last = first + it.tiles - 1;
+                if (p.weight > 0) {
+                    first = unit_weight_begin(it, group_rows, g, 0);
+                    last = unit_weight_begin(it, group_rows, g, it.tiles - 1);
+                }
+                const int c0 = plan_cta_of(first, W, p.grid);
+                const int c1 = plan_cta_of(last, W, p.grid);
                 ms = std::max(ms, c1 - c0 + 1);
             }
         }

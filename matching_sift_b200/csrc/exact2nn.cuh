@@ -50,6 +50,7 @@ struct ExactPlan {
     int grid;                       // persistent CTAs (CTA pairs for the pair kernel)
     int max_splits;                 // max CTAs covering one query group
     int parts;                      // partial top-2 lists per (split, query): column slices
+    long long weight;               // > 0: batches, whose units are shared out by weight (WorkItem)
 };
 
 __host__ __device__ inline long long plan_w0(long long c, long long W, long long G) { return (c * W) / G; }
@@ -73,8 +74,46 @@ struct WorkItem {
     int groups, tiles;
     int rec_off;
     int idx_base;
+    long long w_begin;  // weight of the units before the problem's
 };
-static_assert(sizeof(WorkItem) == 40, "WorkItem layout");
+static_assert(sizeof(WorkItem) == 48, "WorkItem layout");
+
+// Weights of a batch's units, in sixths of a dense one. The first
+// kPackedDenseTiles tiles of a base set run the packed network untested and cost
+// 1.115 us per unit, later ones 0.947, and 0.18 less where a group's second query
+// tile has no rows (least squares over the workers of 512 pairs of 500-8,000
+// rows; the same within 3% over 128 pairs). With equal shares of units the 74
+// workers took 870-991 us (mean 927, standard deviation 25.5); weighted as here
+// what is left to chance is 8.5: 512 pairs 1,084 -> 1,050 us, mutual matching of 128
+// pairs 546 -> 520. Worker c owns the units whose weight position
+// lies in [plan_w0(c), plan_w0(c + 1)), plan_cta_of of that position inverts it.
+constexpr int kPackedDenseTiles = 16;
+constexpr int kDenseWeight = 6, kLateWeight = 5;
+__host__ __device__ inline long long tiles_weight(int tiles, int light) {
+    const int dense = tiles < kPackedDenseTiles ? tiles : kPackedDenseTiles;
+    return static_cast<long long>(dense) * (kDenseWeight - light) +
+           static_cast<long long>(tiles - dense) * (kLateWeight - light);
+}
+// 1 when query group g's second tile per CTA has no rows.
+__host__ __device__ inline int group_light(const WorkItem& it, int group_rows, int g) {
+    return group_rows > 2 * kBM && it.n_a - g * group_rows <= 2 * kBM ? 1 : 0;
+}
+// Weight position of unit (g, j) of a problem.
+__host__ __device__ inline long long unit_weight_begin(const WorkItem& it, int group_rows, int g, int j) {
+    return it.w_begin + g * tiles_weight(it.tiles, 0) + tiles_weight(j, group_light(it, group_rows, g));
+}
+// The first unit at or past weight position x of the problem that holds x; j may be
+// it.tiles (the next group's first unit).
+__host__ __device__ inline void unit_at_weight(const WorkItem& it, int group_rows, long long x, int& g, int& j) {
+    long long r = x - it.w_begin;
+    const long long full = tiles_weight(it.tiles, 0);
+    g = static_cast<int>(r / full < it.groups - 1 ? r / full : it.groups - 1);
+    r -= g * full;
+    const int light = group_light(it, group_rows, g);
+    const long long dense = tiles_weight(it.tiles < kPackedDenseTiles ? it.tiles : kPackedDenseTiles, light);
+    j = static_cast<int>(r <= dense ? (r + kDenseWeight - light - 1) / (kDenseWeight - light)
+                                    : kPackedDenseTiles + (r - dense + kLateWeight - light - 1) / (kLateWeight - light));
+}
 
 // Batch plan: items[] in device memory, plan.units = sum of all units,
 // plan.q_pad = query capacity (>= total query rows, multiple of kBM),
@@ -94,8 +133,8 @@ long long make_batch_items(int n_items, const int* n_a, const int* n_b, const in
                            WorkItem* items, int* total_tiles, int* total_queries);
 // The plan of a batch: units, grid, q_pad (query capacity) and max_splits over
 // every query group of every problem.
-ExactPlan make_batch_plan(const WorkItem* items, int n_items, long long units, int total_queries, int num_workers,
-                          int parts);
+ExactPlan make_batch_plan(const WorkItem* items, int n_items, int group_rows, long long units, int total_queries,
+                          int num_workers, int parts);
 
 // num_workers: persistent CTAs (or CTA pairs); parts: partial top-2 lists
 // each worker writes per query (one per disjoint column slice it scans).

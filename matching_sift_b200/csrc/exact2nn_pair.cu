@@ -160,6 +160,29 @@ struct PairCfg {
 };
 
 // Walks a CTA pair's contiguous unit range over the work items.
+// The last of n items (n >= 1) that `at_most` holds for, over a list where it holds
+// for the first items only (the first one at least): 32 probes per step, all lanes
+// of the warp. Empty items share the next one's begin, so the last one owns it.
+template <typename F>
+__device__ __forceinline__ int warp_last_at_most(int n, F at_most) {
+    int lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 31) / 32;
+        const int at = lo + static_cast<int>(threadIdx.x & 31) * step;
+        const int k = __popc(__ballot_sync(0xffffffffu, at < hi && (at == lo || at_most(at)))) - 1;
+        hi = min(hi, lo + (k + 1) * step);
+        lo += k * step;
+    }
+    return lo;
+}
+// The number of the first unit at or past weight position x (x below the total).
+__device__ __forceinline__ long long unit_of_weight(const WorkItem* items, int n, int group_rows, long long x) {
+    const WorkItem it = items[warp_last_at_most(n, [&](int k) { return items[k].w_begin <= x; })];
+    int g, j;
+    unit_at_weight(it, group_rows, x, g, j);
+    return it.u_begin + static_cast<long long>(g) * it.tiles + j;
+}
+
 struct Cursor {
     const WorkItem* items;  // device list, or null for the single item `it`
     int n_items;
@@ -171,12 +194,7 @@ struct Cursor {
         n_items = n;
         p = 0;
         if (list) {
-            int lo = 0, hi = n - 1;  // largest p with u_begin <= w (empty items share the next one's u_begin)
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (list[mid].u_begin <= w) lo = mid; else hi = mid - 1;
-            }
-            p = lo;
+            p = warp_last_at_most(n, [&](int k) { return list[k].u_begin <= w; });
             it = list[p];
         } else {
             it = single;
@@ -251,10 +269,11 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
     const uint32_t rank = ptx::cluster_ctarank();
     const bool leader = rank == 0;
     const int pair = static_cast<int>(blockIdx.x >> 1);
-    const long long W = plan.units;
+    const bool weighted = PACKED && plan.weight > 0;
+    const long long W = weighted ? plan.weight : plan.units;
     const long long G = plan.grid;  // pairs
-    const long long w_begin = plan_w0(pair, W, G);
-    const int n_units = static_cast<int>(plan_w0(pair + 1, W, G) - w_begin);
+    long long w_begin = plan_w0(pair, W, G);
+    int n_units = static_cast<int>(plan_w0(pair + 1, W, G) - w_begin);
 
     const uint32_t bar_full = ptx::smem_u32(&ctl->full[0]);
     const uint32_t bar_rfull = ptx::smem_u32(&ctl->rfull[0]);
@@ -315,6 +334,12 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
 
     wait_previous();
     Cursor cur;
+    if (weighted) {
+        const long long u_end =
+            pair + 1 < G ? unit_of_weight(items, n_items, 2 * QPT * kBM, w_begin + n_units) : plan.units;
+        w_begin = unit_of_weight(items, n_items, 2 * QPT * kBM, w_begin);
+        n_units = static_cast<int>(u_end - w_begin);
+    }
     if (n_units > 0) cur.init(items, n_items, single, w_begin);
 
     if (warp == 0) {
@@ -500,7 +525,9 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                 const int q_local = ((cur.g * QPT + t) * 2 + static_cast<int>(rank)) * kBM + quarter * 32 + lane;
                 valid = q_local < cur.it.n_a;
                 active = __any_sync(0xffffffffu, valid);
-                split = pair - plan_cta_of(cur.group_first_unit(), W, G);
+                split = pair - plan_cta_of(weighted ? unit_weight_begin(cur.it, 2 * QPT * kBM, cur.g, 0)
+                                                    : cur.group_first_unit(),
+                                           W, G);
                 q = cur.it.a_off + q_local;
                 next_thr = valid ? __ldcg(thresh + q) : INT_MAX;
                 next_best = !PACKED && valid ? __ldcg(best_key + q) : INT_MAX;
