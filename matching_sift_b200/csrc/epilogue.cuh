@@ -108,6 +108,13 @@ enum AccKind : int {
 // a vote on its largest w. 512 pairs of 500-8,000 rows: always testing 1,251 us,
 // never 1,168, from tile 8 / 16 / 28 on 1,139 / 1,117 / 1,117; 64 pairs of
 // 7,000-8,000 rows: 863, 962, 848 / 843 / 855.
+// The FP16 kernel runs it for the first kPackedFirstUnits units of a worker, whose
+// bounds are loose (they took 2-5 times a later unit's 1,250 cycles): 2,000 x 100,000
+// 94 -> 89 us per call, 2,561 x 500,003 304.6 -> 299.6, 5,000 x 300,000 311 -> 301,
+// 10,000 x 1,000,000 equal within 0.3%; 4, 6, 16 and 32 units: 301.5, 300, 304.5, 322
+// at 2,561 x 500,003. The u8 kernel's steady state lost more to the added code
+// (10,000 x 1,000,000 1,167 -> 1,187-1,214) than its first units gave.
+constexpr int kPackedFirstUnits = 8;
 constexpr int kPackedMaxKey = 1 << 23;
 constexpr int kPackedNone = INT_MIN;  // w of a padding row: below every floor
 
@@ -127,21 +134,37 @@ __device__ __forceinline__ void top2_join(int& hi, int& lo, int h, int l) {
     hi = max(hi, h);
 }
 
-// Rows [0, 16) of the chunk that starts at tile column c0: accumulators v, K at
-// k (16-byte aligned), nv valid rows in the tile; m1 >= m2: the running two
+// w of one accumulator. FLOAT (FP16 rows of u8 values): acc and the record's norm k
+// are floats, integers below 2^23 once multiplied by dscale: adding 2^23 leaves the
+// integer in the low bits of the sum, and the exponents' share of w, (256 - 128) x
+// 0x4B000000, is 2^31 (modulo 2^32). With the norms 0 of plain dot products w is
+// 256 q.b + 127 - col < 2^31.
+template <bool FLOAT>
+__device__ __forceinline__ int packed_w(uint32_t acc, int32_t k, int col, float dscale) {
+    if constexpr (FLOAT) {
+        const uint32_t a = __float_as_uint(fmaf(__uint_as_float(acc), dscale, 8388608.0f));
+        const uint32_t n = __float_as_uint(fmaf(__int_as_float(k), dscale, 8388608.0f));
+        return static_cast<int>((a << 8) - (n << 7) + (0x80000000u + static_cast<uint32_t>(127 - col)));
+    } else {
+        return static_cast<int>((acc << 8) + static_cast<uint32_t>(k));
+    }
+}
+
+// Rows [0, 16) of the chunk that starts at tile column c0: accumulators v, K (FLOAT:
+// norms) at k (16-byte aligned), nv valid rows in the tile; m1 >= m2: the running two
 // largest w. DENSE: the network at once; else only where some lane's largest w
 // passes its second.
-template <bool DENSE>
+template <bool DENSE, bool FLOAT = false>
 __device__ __forceinline__ void packed16(const uint32_t (&v)[16], int c0, int nv, const int32_t* k, int& m1,
-                                         int& m2) {
+                                         int& m2, float dscale = 0.0f) {
     int w[16];
     #pragma unroll
     for (int g = 0; g < 4; ++g) {
         const int4 kv = *reinterpret_cast<const int4*>(k + 4 * g);
-        w[4 * g] = static_cast<int>((v[4 * g] << 8) + static_cast<uint32_t>(kv.x));
-        w[4 * g + 1] = static_cast<int>((v[4 * g + 1] << 8) + static_cast<uint32_t>(kv.y));
-        w[4 * g + 2] = static_cast<int>((v[4 * g + 2] << 8) + static_cast<uint32_t>(kv.z));
-        w[4 * g + 3] = static_cast<int>((v[4 * g + 3] << 8) + static_cast<uint32_t>(kv.w));
+        w[4 * g] = packed_w<FLOAT>(v[4 * g], kv.x, c0 + 4 * g, dscale);
+        w[4 * g + 1] = packed_w<FLOAT>(v[4 * g + 1], kv.y, c0 + 4 * g + 1, dscale);
+        w[4 * g + 2] = packed_w<FLOAT>(v[4 * g + 2], kv.z, c0 + 4 * g + 2, dscale);
+        w[4 * g + 3] = packed_w<FLOAT>(v[4 * g + 3], kv.w, c0 + 4 * g + 3, dscale);
     }
     if (c0 + 16 > nv) {  // the last tile of a base set: rows past it (any values) never count
         #pragma unroll

@@ -553,7 +553,24 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
                     const int32_t* rec = r_smem + s * kRecInts;
                     constexpr int kKind = MODE == kModeFloat ? kAccFloat : (F16 ? kAccF32Int : kAccS32);
                     const int row0 = cur.it.idx_base + j * kBN;
-                    if constexpr (!PACKED) {
+                    if (MODE == kModeF16Int && n < kPackedFirstUnits) {
+                        // The packed network, one chunk at a time in a rolled
+                        // loop (unrolled, its registers spill in the loop below).
+                        const int floor = valid ? packed_floor(st.thr) : INT_MAX;
+                        const int nv = cur.it.n_b - j * kBN;  // valid rows of the tile, if fewer than 128
+                        int m1 = floor, m2 = floor;
+                        #pragma unroll 1
+                        for (int c = 0; c < kBN; c += 16) {
+                            uint32_t v[16];
+                            ptx::tmem_ld16(taddr + c, v);
+                            ptx::tmem_ld_wait(v);
+                            packed16<true, true>(v, c, nv, rec + c, m1, m2, dscale);
+                        }
+                        ptx::tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive_cluster_relaxed(lead_tempty);
+                        packed_merge(m1, m2, floor, row0, st);
+                    } else if constexpr (!PACKED) {
                         // Two passes over the slot's 128 columns (8 chunks of 16).
                         // The first bounds every 8-row subgroup against the
                         // threshold held at its start, with no vote and no branch,
