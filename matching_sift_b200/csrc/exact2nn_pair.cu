@@ -273,7 +273,8 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
     const long long W = weighted ? plan.weight : plan.units;
     const long long G = plan.grid;  // pairs
     long long w_begin = plan_w0(pair, W, G);
-    int n_units = static_cast<int>(plan_w0(pair + 1, W, G) - w_begin);
+    const long long w_end = plan_w0(pair + 1, W, G);
+    int n_units = static_cast<int>(w_end - w_begin);
 
     const uint32_t bar_full = ptx::smem_u32(&ctl->full[0]);
     const uint32_t bar_rfull = ptx::smem_u32(&ctl->rfull[0]);
@@ -336,7 +337,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
     Cursor cur;
     if (weighted) {
         const long long u_end =
-            pair + 1 < G ? unit_of_weight(items, n_items, 2 * QPT * kBM, w_begin + n_units) : plan.units;
+            pair + 1 < G ? unit_of_weight(items, n_items, 2 * QPT * kBM, w_end) : plan.units;
         w_begin = unit_of_weight(items, n_items, 2 * QPT * kBM, w_begin);
         n_units = static_cast<int>(u_end - w_begin);
     }
