@@ -336,6 +336,53 @@ __global__ void __launch_bounds__(kLThreads, 1)
 constexpr int kProbeRows = 32;
 constexpr int kProbeThreads = 256;
 
+// The probes of a query with a NaN margin (weights or sums that are not finite):
+// comparisons with it are all false, so counting gives several bits or subsets the
+// same rank. One thread selects instead, bits by insertion in bit order and then, for
+// each probe, the first subset left that none is lighter than, with the empty one
+// (sum 0) first. Rare and slow (a few thousand steps); out: one code per kProbeRows + 1.
+__device__ __noinline__ void probe_codes_unordered(const float* __restrict__ z, uint32_t code, int k, int flip,
+                                                   int n_probes, uint32_t* out) {
+    int bit[6];
+    float mag[6];
+    int m = 0;
+    for (int j = 0; j < k; ++j) {
+        const float a = fabsf(z[j]);
+        int p;
+        if (m < flip) p = m++;
+        else if (flip > 0 && a < mag[flip - 1]) p = flip - 1;
+        else continue;
+        for (; p > 0 && mag[p - 1] > a; --p) {
+            mag[p] = mag[p - 1];
+            bit[p] = bit[p - 1];
+        }
+        mag[p] = a;
+        bit[p] = j;
+    }
+    uint64_t taken = 0;
+    for (int p = 0; p < n_probes; ++p) {
+        int best = -1;
+        float lightest = 0.0f;
+        for (int s = 0; s < (1 << m); ++s) {
+            if ((taken >> s) & 1u) continue;
+            float sum = 0.0f;
+            for (int b = 0; b < m; ++b)
+                if ((s >> b) & 1) sum += mag[b];
+            if (best < 0 || sum < lightest) {
+                best = s;
+                lightest = sum;
+            }
+        }
+        uint32_t c = code;
+        if (best >= 0) {
+            taken |= 1ull << best;
+            for (int b = 0; b < m; ++b)
+                if ((best >> b) & 1) c ^= 1u << bit[b];
+        }
+        out[p * (kProbeRows + 1)] = c;
+    }
+}
+
 __global__ void __launch_bounds__(kProbeThreads)
     probe_codes_kernel(const uint32_t* __restrict__ codes, const float* __restrict__ z, int n, int k, int flip,
                        int n_probes, uint32_t* __restrict__ out) {
@@ -359,6 +406,11 @@ __global__ void __launch_bounds__(kProbeThreads)
         if (row0 + col >= n) break;
         const uint32_t code = codes[row0 + col];
         const float a = mags[r];
+        if (__any_sync(0xffffffffu, isnan(a))) {
+            if (lane == 0)
+                probe_codes_unordered(z + static_cast<size_t>(row0 + col) * k, code, k, flip, n_probes, &s_out[0][col]);
+            continue;
+        }
         int rank = 0;
         for (int j = 0; j < k; ++j) {
             const float b = __shfl_sync(0xffffffffu, a, j);
