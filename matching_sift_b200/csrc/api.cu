@@ -672,7 +672,7 @@ int exact_match(const MatchArgs& a) {
     SIFT_TRY(plan_inputs(a.q, a.r, use_f16 ? -1 : a.type, q_n, r_n, L, ip));
     const size_t o_brec = L.take(static_cast<size_t>(plan.base_tiles) * kRecInts * 4 + 16);
     const size_t o_qnorm = L.take(static_cast<size_t>(plan.q_pad) * 4);
-    const size_t o_thr = L.take(static_cast<size_t>(plan.q_pad) * 8);
+    const size_t o_thr = L.take(static_cast<size_t>(plan.q_pad) * (use_packed ? 4 : 8));
     const size_t o_part = L.take(static_cast<size_t>(plan.max_splits) * plan.parts * plan.q_pad * sizeof(int4));
     const size_t o_m = (a.matches && !m_dev) ? L.take(static_cast<size_t>(q_n) * 4) : 0;
     const size_t o_s = (a.sorted && !s_dev) ? L.take(static_cast<size_t>(q_n) * 16) : 0;

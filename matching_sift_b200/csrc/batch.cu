@@ -109,7 +109,7 @@ BatchLayout layout_for(const Built* builds, int n) {
     o.o_items = L.take(sizeof(WorkItem) * (b.items.size() + 1));
     o.o_rec = L.take(static_cast<size_t>(b.total_tiles) * kRecInts * 4 + 16);
     o.o_qn = L.take(static_cast<size_t>(b.plan.q_pad) * 4 + 16);
-    o.o_thr = L.take(static_cast<size_t>(b.plan.q_pad) * 8 + 16);
+    o.o_thr = L.take(static_cast<size_t>(b.plan.q_pad) * 4 + 16);
     o.o_part = L.take(part + 16);
     o.bytes = L.off;
     return o;

@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(256)
                 row < n ? 127 - col - 128 * static_cast<int32_t>(s) : 0;
         } else if (row < q_pad) {
             qnorm[row] = static_cast<int32_t>(s);
-            thresh[row] = thresh[q_pad + row] = INT_MAX;
+            thresh[row] = INT_MAX;
         }
     }
 }

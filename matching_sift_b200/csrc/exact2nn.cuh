@@ -205,7 +205,8 @@ cudaError_t launch_exact2nn_u8_pair(const CUtensorMap& qmap, const CUtensorMap& 
 // CTA (2: query groups of 512 rows, 1: groups of 256 rows; the items must be
 // made with the same group size); qbuf: query buffers (1 or 2). Shapes built:
 // (2, 1), (2, 2), (1, 2). bp.items null: the single problem of bp.plan (small
-// searches; squared distances only).
+// searches; squared distances only). thresh: [q_pad], the bounds of the
+// second-best keys alone (launch_batch_prep).
 cudaError_t launch_exact2nn_u8_pair_batch(const CUtensorMap& qmap, const CUtensorMap& bmap_half, const int32_t* brec,
                                           const BatchPlan& bp, int4* partial, int32_t* thresh, int* err, int qpt,
                                           int qbuf, cudaStream_t stream);
@@ -246,7 +247,7 @@ cudaError_t launch_merge2nn_chunks(const int4* partial, const ChunkSet& cs, int 
 
 // Base-tile records of every problem of a batch for the packed epilogue
 // (bp.total_tiles records, the first 128 ints of each) and the norms and cleared
-// bounds of its q_n query rows. bp.items null: the single problem of bp.plan.
+// bounds thresh[q_pad] of its q_n query rows. bp.items null: the single problem of bp.plan.
 cudaError_t launch_batch_prep(const uint8_t* base, const uint8_t* q, int q_n, const BatchPlan& bp, int32_t* rec,
                               int32_t* qnorm, int32_t* thresh, cudaStream_t stream);
 // Merge for a batch: query row q belongs to the problem whose range holds it;
