@@ -1,5 +1,7 @@
 #!/usr/bin/env python
-"""Benchmark of the exact 2-NN matching path (one JSON line on rank 0).
+"""Benchmark of the exact 2-NN matching path (one JSON line on rank 0's stdout;
+the full record with every operating point of every variant goes to stderr, or to
+--detail FILE, as one line of its own).
 
 Workload: 10,000 queries against a 1,000,000 x 128 uint8 base from the seeded
 generator (matching_sift_b200.datagen; stand-in for ANN_SIFT1M), exact
@@ -201,6 +203,32 @@ def cpu_reference_rate(q, r, target_s: float):
     return n2 / dt, f"{n2} queries x {r.shape[0]} base rows ({dt:.1f} s)", threads, kind
 
 
+# ------------------------------------------------------------ result line --
+
+def short_line(line):
+    """The result line without what only the full record holds: notes, and the
+    variants' operating points and workloads (readers of stdout may keep only its
+    last 3,000 characters)."""
+    def pick(d, *keys):
+        return {k: d[k] for k in keys if k in d}
+
+    out = {k: v for k, v in line.items() if k not in ("e2e", "roofline", "variants")}
+    if "e2e" in line:
+        out["e2e"] = pick(line["e2e"], "value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "call",
+                          "h2d_copy_ms", "frac_of_h2d_copy")
+    if "roofline" in line:
+        out["roofline"] = pick(line["roofline"], "bound", "kernel", "achieved", "peak", "unit", "frac", "traffic",
+                               "kernel_ms")
+    for name, v in line.get("variants", {}).items():
+        s = pick(v, "value", "ms_per_step", "ms_per_call")
+        if isinstance(v.get("roofline"), dict):
+            s["frac"] = v["roofline"].get("frac")
+        if isinstance(v.get("operating_point"), dict):
+            s.update(pick(v["operating_point"], "ms_per_call", "recall1"))
+        out.setdefault("variants", {})[name] = s
+    return out
+
+
 # ----------------------------------------------------------------- main ----
 
 def main():
@@ -217,6 +245,7 @@ def main():
     ap.add_argument("--base-file", help="base descriptors (.fvecs/.bvecs, e.g. ANN_SIFT1M sift_base.fvecs; "
                                         "the first 1,000,000 rows) instead of the seeded generator")
     ap.add_argument("--query-file", help="query descriptors (.fvecs/.bvecs; the first --queries rows)")
+    ap.add_argument("--detail", help="write the full record to this file instead of stderr")
     ap.add_argument("--truth-file", help="ground truth (.ivecs) for recall of the exact matches")
     args = ap.parse_args()
     if bool(args.base_file) != bool(args.query_file):
@@ -479,7 +508,12 @@ def main():
             rate, sample, threads, kind = cpu_reference_rate(queries, base, 15.0)
             line["cpu_baseline"] = {"value": round(rate, 2), "unit": "queries/s", "cores": threads, "kind": kind,
                                     "sample": sample}
-        print(json.dumps(line), flush=True)
+        if args.detail:
+            with open(args.detail, "w") as f:
+                print(json.dumps(line), file=f)
+        else:
+            print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(short_line(line)), flush=True)
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()
