@@ -60,3 +60,14 @@ def test_record_without_legs():
     line = {k: v for k, v in _record().items() if k not in ("variants", "roofline", "cpu_baseline")}
     got = bench.short_line(line)
     assert got["value"] == line["value"] and "variants" not in got
+
+
+def test_reference_arm_without_the_reference_says_so(monkeypatch, capsys):
+    import types
+
+    import oracle
+
+    monkeypatch.setattr(oracle, "ref_available", lambda: False)
+    bench.reference_arm(types.SimpleNamespace(steps=1, warmup=0), 1, 0)
+    got = json.loads(capsys.readouterr().out)
+    assert got["impl"] == "reference" and got["unavailable"] and "value" not in got
