@@ -620,13 +620,15 @@ int exact_match_float(const MatchArgs& a, DeviceCtx& c, cudaStream_t st, const V
 }
 
 // Searches in which a worker scans few base tiles per query: their thresholds
-// stay loose, so the packed epilogue of the batches (which also needs one launch
-// less before the search) beats the pruned one. Device time of a call, packed |
-// folded norms: 517 x 733 (1 unit per worker) 11.1 | 15.9 us, 1,000 x 10,000 (2)
-// 16.9 | 25.3, 4,000 x 20,000 (17) 31.7 | 43.8, 3,000 x 60,000 (38) 51.3 | 58.7,
-// 10,000 x 30,000 (64) 74.9 | 81.6, 2,000 x 200,000 (85) 94.3 | 84.2,
-// 10,000 x 100,000 (211) 204 | 168. (Both have lost 1-4 us since, to overlapped
-// launches and to the query norms in the folded records' launch.)
+// stay loose, so the packed epilogue of the batches beats the pruned one. Whole
+// match() calls (units per worker), packed | folded norms: 3 x 7 (1) 25.6 | 32.1 us,
+// 60,000 x 500 (6) 26.8 | 39.0, 512 x 303,000 (32) 48.2 | 53.4, 2,000 x 100,000 (42)
+// 57.6 | 61.5, 60,000 x 5,000 (64) 83.8 | 124, 10,000 x 31,000 (66) 79.1 | 84.1,
+// 4,000 x 76,000 (64) 77.7 | 77.7, 2,000 x 150,000 (63) 75.1 | 73.2,
+// 1,000 x 300,000 (63) 75.6 | 71.7, 10,000 x 40,000 (85) 95.7 | 98.3,
+// 2,000 x 200,000 (85) 94.4 | 84.8, 10,000 x 60,000 (127) 132 | 121. The lines cross
+// between ~50 units (one or two query groups, many partial lists) and ~90 (twenty
+// and more); 64 is within 6.5% of the faster side at all of these.
 constexpr int kPackedUnits = 64;
 bool packed_search(const ExactPlan& plan, int metric) {
     return metric == SIFT_METRIC_L2 && plan.grid > 0 && plan.units <= static_cast<long long>(kPackedUnits) * plan.grid;

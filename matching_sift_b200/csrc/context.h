@@ -92,7 +92,8 @@ int encode_u8_rows(CUtensorMap* m, const void* base, uint64_t rows, uint32_t box
 int encode_bf16_2d(CUtensorMap* m, const void* base, uint64_t inner, uint64_t rows, uint32_t box_inner,
                    uint32_t box_rows);
 int map_cuda(cudaError_t e);
-// Reads and clears the device status words. Caller has synchronised `st`.
+// Copies the first `ints` device status words, synchronises `st` and returns the
+// error that the work enqueued on it so far recorded (clearing it).
 int collect_device_status(DeviceCtx& c, cudaStream_t st, int ints = 2);
 // Benchmark timing of one kernel launch on `st` (CUDA events recorded on the
 // launching stream when profiling is enabled; collected by tag).

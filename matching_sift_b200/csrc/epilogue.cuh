@@ -101,7 +101,7 @@ enum AccKind : int {
 // queries finds something new in more than half of its 16-row chunks, and the
 // scan with 8-row bounds and serial updates took ~4,800 cycles per unit there.
 // Measured: 512 image pairs (plan replay) 2,276 -> 1,118 us, mutual matching of
-// 128 pairs 1,175 -> 566 us (1,051 and 522 with later changes around it).
+// 128 pairs 1,175 -> 566 us.
 // The first kPackedDenseTiles tiles of a base set (2,048 rows, where 60-100% of
 // the chunks hold something new for some of the 32 queries) run the network with
 // no test at all, so that the chunks overlap freely; later tiles skip a chunk by

@@ -44,7 +44,8 @@
 // epilogue 670 + release to issue 300 + issue 520 + commit to visible 300 cycles
 // (u8, norms folded); with both parities walked unit by unit by a single lane the
 // issuer spent ~840 cycles per own unit between its tests, on every slot's path.
-// 10,000 x 1,000,000 u8 1,344 -> 1,184 us per call, FP16 2,561 x 500,003
+// 10,000 x 1,000,000 u8 1,344 -> 1,184 us per call in bursts and 1,321 -> 1,265 in
+// long runs of calls, which the board's power limit slows; FP16 2,561 x 500,003
 // 427 -> 412, general float 2,053 x 131,077 345 -> 335, 512 pairs 1,118 -> 1,092.
 //
 // Barriers and who signals them (L = only the leader's copy is used):
@@ -81,8 +82,10 @@
 //                             float norms), and only the values of passing
 //                             subgroups are converted to the u8 kernel's integer
 //                             keys (times dscale = 2^2s); the rest is shared.
-//   exact2nn_u8_pair_batch_kernel<QPT, QB>  u8 batches with the shapes the
-//                             batch autotuner chooses from.
+//   exact2nn_u8_pair_batch_kernel<QPT, QB>  the packed epilogue: u8 batches
+//                             with the shapes the batch autotuner chooses from,
+//                             and single u8 searches of few units per worker
+//                             (QPT 2, QB 1).
 #include <climits>
 #include <type_traits>
 #include "exact2nn.cuh"
@@ -159,7 +162,6 @@ struct PairCfg {
     static_assert(kSmemBytes <= kPSmemBudget + 1024, "shared memory budget");
 };
 
-// Walks a CTA pair's contiguous unit range over the work items.
 // The last of n items (n >= 1) that `at_most` holds for, over a list where it holds
 // for the first items only (the first one at least): 32 probes per step, all lanes
 // of the warp. Empty items share the next one's begin, so the last one owns it.
@@ -183,6 +185,7 @@ __device__ __forceinline__ long long unit_of_weight(const WorkItem* items, int n
     return it.u_begin + static_cast<long long>(g) * it.tiles + j;
 }
 
+// Walks a CTA pair's contiguous unit range over the work items.
 struct Cursor {
     const WorkItem* items;  // device list, or null for the single item `it`
     int n_items;
@@ -509,7 +512,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& qmap, const CUtenso
         // only its second) bounds the final second: over the 10-76 lists of a
         // query the bound converges to the final second itself instead of to the
         // smallest second of any list. FP16 2,561 x 500,003 412 -> 392 us, general
-        // float 2,053 x 131,077 335 -> 330, u8 10,000 x 1,000,000 1,183 -> 1,168;
+        // float 2,053 x 131,077 335 -> 330, u8 10,000 x 1,000,000 1,183 -> 1,168 in bursts;
         // the 2-4 lists of a batch's query gain less than the second bound costs
         // (512 pairs 1,092 -> 1,118), so batches keep one.
         int32_t* const best_key = thresh + plan.q_pad;

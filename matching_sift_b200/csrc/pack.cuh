@@ -9,7 +9,8 @@ namespace sift {
 // them first):
 //   stats[0]  flags below
 //   stats[1]  OR of v * 2^24 as unsigned integers (meaningless with kValueNotFixed)
-//   stats[2]  bit pattern of the largest finite |value| (as a float)
+//   stats[2]  bit pattern of the largest |value| (as a float; meaningless with
+//             kValueNotFinite)
 // With shift s = value_shift(stats[1]) (the smallest s >= 0 that makes every
 // v * 2^s an integer) the values suit the integer kernels when kValueNotFixed is
 // not set and the largest value times 2^s is at most 255.
@@ -30,7 +31,7 @@ cudaError_t launch_pack_u8(const void* q, size_t q_rows, const void* r, size_t r
                            uint8_t* q_out, uint8_t* r_out, int num_sms, cudaStream_t stream);
 
 // FP16 rows in one pass: the survey, base-tile records of float norms (as
-// launch_row_norms_float, mul = 1; padding rows kFloatKeyPad), query norms
+// launch_row_norms_float; padding rows kFloatKeyPad), query norms
 // (float bit patterns) and cleared bounds thresh[2 q_pad].
 cudaError_t launch_survey_norms_f16(const void* r, int r_n, int base_tiles, int metric, int32_t* rec, const void* q,
                                     int q_n, int q_pad, int32_t* qnorm, int32_t* thresh, int* stats,
