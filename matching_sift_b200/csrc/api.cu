@@ -361,19 +361,22 @@ constexpr int kChunkMinRows = 1 << 16;
 constexpr int kChunks = 8;
 
 // Base tiles per chunk, in base order (returns the number of chunks).
-// The pinned copy moves a 128-byte row in ~2.3 ns (~55 GB/s of PCIe), and
-// the search kernel spends ~0.128 ps per query x row (10,000 x 1,000,000 in
-// ~1.28 ms), so with q_n queries a chunk's search takes beta = q_n x 5.5e-5
-// of its copy time. When beta is small the copy sets the pace and only the
+// The pinned copy moves a 128-byte row in ~2.33 ns (~55 GB/s of PCIe), and
+// the search kernel spends ~0.119 ps per query x row (10,000 x 1,000,000 in
+// 1.17-1.2 ms of short work), so with q_n queries a chunk's search takes
+// beta = q_n x 5.1e-5 of its copy time. When beta is small the copy sets the pace and only the
 // last chunk's search (plus the merge) runs after the last byte lands: the
 // chunks then shrink geometrically toward the end of the base, each one
 // 1 / (1.25 beta) of the size of the chunk after it (between 1.25 and 4
 // times, the 1.25 covering the launches of a chunk), from a last chunk of 128
 // tiles (or 1/64 of the base), so that every chunk's search ends about when
 // the next chunk lands. Otherwise (the search sets the pace) the base goes in
-// kChunks equal chunks.
+// kChunks equal chunks. 1,000,000 base rows, medians of 12 calls in four processes
+// each, 5.5e-5 (an older search's) | 5.1e-5: 15,000 queries, equal | shrinking chunks,
+// 2.65-2.77 | 2.51-2.71 ms; 10,000 2.48-2.67 | 2.51-2.72, 14,000 (the same chunks)
+// 2.50-2.61 | 2.49-2.75, 16,000 (equal in both) 2.66-2.78 | 2.66-2.86.
 int plan_chunk_tiles(int q_n, int tiles, int (&out)[kMaxChunks]) {
-    const double beta = 5.5e-5 * q_n, paced = 1.25 * beta;
+    const double beta = 5.1e-5 * q_n, paced = 1.25 * beta;
     if (paced > 1.0) {
         const int per = (tiles + kChunks - 1) / kChunks;
         int n = 0;
