@@ -714,8 +714,8 @@ __global__ void __launch_bounds__(kMergeThreads<LANES>)
     merge_finish<FLOATKEY>(t, q, n_b, qnorm, metric, thr, dscale, out);
 }
 
-// Merge of a search split over base chunks (indices already global): ~90 lists
-// per query row for 10,000 x 1,000,000 in 9 chunks, read as merge2nn_kernel
+// Merge of a search split over base chunks (indices already global): ~75 lists
+// per query row for 10,000 x 1,000,000 in 8 chunks, read as merge2nn_kernel
 // reads them.
 constexpr int kMergeChunkLanes = 8;
 __global__ void __launch_bounds__(kMergeThreads<kMergeChunkLanes>)
