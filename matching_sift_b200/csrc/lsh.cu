@@ -244,6 +244,11 @@ constexpr int kChunkThreads = 1024;
 constexpr int kChunkPer = 8;
 constexpr int kChunkPoints = kChunkThreads * kChunkPer;
 
+// Chunks of n points (n up to 2^31 - 1: the rounded sum needs 64 bits).
+__host__ __device__ constexpr int bucket_chunks(int n) {
+    return static_cast<int>((static_cast<long long>(n) + kChunkPoints - 1) / kChunkPoints);
+}
+
 size_t bucket_smem_bytes(int nbins, bool scatter) {
     return ((static_cast<size_t>(nbins) * 2 + 15) & ~static_cast<size_t>(15)) + (scatter ? kChunkPoints * 4 : 0);
 }
@@ -267,7 +272,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1)
     }
     const int tid = threadIdx.x;
     for (int i = tid; i < (nbins + 1) / 2; i += kChunkThreads) s_words[i] = 0;
-    const int chunks = (n + kChunkPoints - 1) / kChunkPoints;
+    const int chunks = bucket_chunks(n);
     for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
         __syncthreads();  // counters are zero
         uint32_t code[kChunkPer];
@@ -679,7 +684,7 @@ cudaError_t launch_lsh_buckets(const uint32_t* codes, int n, int L, int shift, i
         e = cudaFuncSetAttribute(lsh_bucket_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem_s));
     if (e != cudaSuccess) return e;
-    const int chunks = (n + kChunkPoints - 1) / kChunkPoints;
+    const int chunks = bucket_chunks(n);
     const dim3 grid(std::min(chunks, num_sms), L);
     lsh_bucket_kernel<false><<<grid, kChunkThreads, smem_c, stream>>>(codes, n, shift, nbins, nullptr, hist, nullptr,
                                                                       nullptr);
