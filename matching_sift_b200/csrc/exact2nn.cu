@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256) row_norms_kernel(const uint8_t* __restric
         nrm[threadIdx.x >> 3] = v;
         if (norm) norm[row] = v;
         if (r) r[part * 32 + (threadIdx.x >> 3)] = v;
-        if (thresh) thresh[row] = thresh[n_pad + row] = INT_MAX;
+        if (thresh) thresh[row] = thresh[static_cast<size_t>(n_pad) + row] = INT_MAX;
     }
     __syncthreads();
     if (threadIdx.x < 4 && r) {
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256)
             const int row = t * kBN + wr;
             if (sub == 0 && row < q_pad) {
                 qnorm[row] = static_cast<int32_t>(s);
-                thresh[row] = thresh[q_pad + row] = INT_MAX;
+                thresh[row] = thresh[static_cast<size_t>(q_pad) + row] = INT_MAX;
             }
             continue;
         }
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256) row_norms_float_kernel(const __half* __re
         nrm[threadIdx.x >> 3] = v;
         if (norm) norm[row] = __float_as_int(v);
         if (r) r[part * 32 + (threadIdx.x >> 3)] = __float_as_int(v);
-        if (thresh) thresh[row] = thresh[n_pad + row] = INT_MAX;
+        if (thresh) thresh[row] = thresh[static_cast<size_t>(n_pad) + row] = INT_MAX;
     }
     __syncthreads();
     if (threadIdx.x < 4 && r) {

@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(256)
             nrm[col] = row < n ? (metric == kMetricL2 ? s : 0.0f) : kFloatKeyPad;
         } else if (row < q_pad) {
             qnorm[row] = __float_as_int(s);
-            thresh[row] = thresh[q_pad + row] = INT_MAX;
+            thresh[row] = thresh[static_cast<size_t>(q_pad) + row] = INT_MAX;
         }
     }
     __syncthreads();
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256)
         }
     } else if (sub == 0 && row < q_pad) {
         qnorm[row] = __float_as_int(row < n ? s : kFloatKeyPad);
-        thresh[row] = thresh[q_pad + row] = INT_MAX;
+        thresh[row] = thresh[static_cast<size_t>(q_pad) + row] = INT_MAX;
     }
 }
 
